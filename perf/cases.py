@@ -1,0 +1,388 @@
+"""What this framework is timed on: one dict per case, inputs made from a seed, one pass through the public
+entry points, and the work a pass cannot do without.
+
+Kinds of case, by what a user's program calls:
+
+* ``gate``    one chunk of a learned-gate layer on a paged cache: ``GateSelectorState.append`` and
+              ``score_select``, then ``ops.attn_compact`` (the step ``bench.py`` times);
+* ``layer``   the same through the drop-in attention module, ``LlamaSeerAttentionChunkedDense.forward``, with
+              its projections (``tokens == 1``: a decode step);
+* ``keep``    the reference's operator on ready gate scores, ``chunked_prefill_column_dense_attention_forward``;
+* ``flash``   the training-free operator, ``flashprefill_compactattn_prefill_full_kv``, with a kept mean-K cache;
+* ``dense``   dense causal attention over a paged cache, ``ops.attn_compact`` without a block table: decode
+              steps (``tokens == 1``), first chunks (``tokens == kv_len``) and chunks on an unaligned past;
+* ``append``  ``PagedKVCache.append_rope`` with the mean-K cache: RoPE, paged append and pooling of a chunk;
+* ``gather``  the cache-fill route: ``ops.union_table`` of a keep mask, ``ops.paged_metadata``, ``ops.gather_kv``.
+
+``kv_len`` counts the chunk (``tokens``).  Head counts are those of the repository's configurations (32/8 and
+28/4) and of their tensor-parallel ranks.
+"""
+from __future__ import annotations
+
+import math
+
+import torch
+
+from compactattention_b200 import ops
+from compactattention_b200.chunk_driver import GateSelectorState, SelectionRule
+from compactattention_b200.modules import (
+    chunked_prefill_column_dense_attention_forward,
+    flashprefill_compactattn_prefill_full_kv,
+)
+from compactattention_b200.paged_cache import PagedKVCache
+from compactattention_b200.prefill_sparse.attn_gate import ATTNGATE_CLASSES
+from compactattention_b200.prefill_sparse.llama.modeling_llama_compactattn import (
+    CompactAttnCache,
+    CompactAttnLlamaConfig,
+    LlamaSeerAttentionChunkedDense,
+)
+
+D = 128
+SPREAD = 6.0  # of the gate logits of the "keep" cases, in natural-log units
+ALPHA = 0.06  # the training-free selector's default
+DTYPES = {"bf16": torch.bfloat16, "f16": torch.float16}
+
+
+def listed():
+    return [
+        # one token of one sequence with a short context: the smallest call, all latency
+        _case("dense", "decode_1x4001", tokens=1, kv_len=4001),
+        # a decode batch: bound by the bytes of its caches
+        _case("dense", "decode_8x32k", batch=8, tokens=1, kv_len=32768),
+        # the first chunk of a long prompt runs dense
+        _case("dense", "first_chunk_8192_f16", tokens=8192, kv_len=8192, dtype="f16"),
+        # a short chunk early in a prompt, through the reference's operator
+        _case("keep", "keep_256_of_8k", tokens=256, kv_len=8192, density=0.2),
+        # the last chunk of two prompts: no multiple of the block, so a partly filled block ends it
+        _case("keep", "keep_2x1000_of_64k_f16", batch=2, tokens=1000, kv_len=64 * 1000 + 1000, hq=28, hkv=4, dtype="f16", density=0.1),
+        # the headline: 1024 tokens at the end of 128K, 20 % of the blocks per row
+        _case("gate", "gate_1024_of_128k", tokens=1024, kv_len=131072, density=0.2),
+        # one of eight tensor-parallel ranks of the same layer
+        _case("gate", "gate_1024_of_128k_tp8_rank", tokens=1024, kv_len=131072, hq=4, hkv=1, density=0.2),
+        # the largest chunk of the shape sweep, 28/4 heads
+        _case("gate", "gate_8192_of_128k_28x4", tokens=8192, kv_len=131072, hq=28, hkv=4, density=0.2),
+        # the training-free selector at its default block size
+        _case("flash", "flash_1024_of_32k_f16", tokens=1024, kv_len=32768, dtype="f16", block=128, density=0.25),
+        # storing a chunk, every layer and chunk
+        _case("append", "append_2048", tokens=2048, kv_len=16384),
+        # the compact cache of the headline's shape, for an attention that wants one
+        _case("gather", "gather_1024_of_128k", tokens=1024, kv_len=131072, density=0.2),
+        # a whole attention layer of the 2048-token-chunk prefill, a quarter into a 128K prompt
+        _case("layer", "layer_2048_of_32k", tokens=2048, kv_len=32768, density=0.2),
+    ]
+
+
+def _case(kind, name=None, *, batch=1, tokens, kv_len, hq=32, hkv=8, dtype="bf16", block=64, density=1.0):
+    c = {"kind": kind, "batch": batch, "tokens": tokens, "kv_len": kv_len, "hq": hq, "hkv": hkv, "dtype": dtype, "block": block,
+         "density": density}
+    if name is not None:
+        c["name"] = name
+    return c
+
+
+def _log_int(rng, lo, hi):
+    return int(round(math.exp(rng.uniform(math.log(lo), math.log(hi)))))
+
+
+def _cost(case):
+    w = work(case)
+    return max(w["bytes"], w["flops"] / 50)
+
+
+def draw(rng):
+    most = max(_cost(c) for c in listed())
+    while True:
+        kind = rng.choice(("gate", "gate", "keep", "flash", "dense", "dense", "append", "gather", "layer"))
+        hq, hkv = rng.choice(((32, 8), (32, 8), (28, 4), (16, 4), (8, 2), (4, 1)))
+        dtype = rng.choice(("bf16", "bf16", "f16"))
+        density = round(rng.uniform(0.05, 0.5), 3)
+        block, batch = 64, 1
+        past = _log_int(rng, 8192, 130048)
+        tokens = _log_int(rng, 256, 8192)
+        if rng.random() < 0.5:
+            tokens = max(256, tokens // 256 * 256)  # half of the chunks are full ones
+        if kind == "dense":
+            if rng.random() < 0.6:  # decode
+                tokens, past, batch = 1, _log_int(rng, 1024, 131071), rng.choice((1, 1, 2, 4, 8, 16))
+            else:  # a first chunk or a chunk on whatever came before
+                past = 0 if rng.random() < 0.5 else _log_int(rng, 256, 32768)
+        elif kind == "append":
+            past = _log_int(rng, 256, 32768) // 64 * 64
+            batch = rng.choice((1, 1, 2))
+            tokens = _log_int(rng, 64, 8192)
+        elif kind == "gather":
+            tokens = max(256, tokens // 64 * 64)
+        elif kind == "layer":
+            hq, hkv, dtype = 32, 8, "bf16"
+            past = _log_int(rng, 2048, 65536)
+            if rng.random() < 0.25:
+                tokens = 1
+        elif kind == "keep":
+            batch = rng.choice((1, 1, 2))
+        elif kind == "flash":
+            block = rng.choice((64, 128, 128))
+            density = max(density, 0.1)
+        if kind != "dense":
+            past = past // block * block
+        if kind in ("gather",) and (past + tokens) % 64:
+            continue
+        c = _case(kind, batch=batch, tokens=tokens, kv_len=past + tokens, hq=hq, hkv=hkv, dtype=dtype, block=block,
+                  density=1.0 if kind in ("dense", "append") else density)
+        if batch * c["kv_len"] * hkv <= 3 * (1 << 20) and _cost(c) <= most:
+            return c
+
+
+# ---------------------------------------------------------------- inputs ----------------------------------------
+def _randn(g, shape, dtype, scale=1.0):
+    return (torch.randn(shape, generator=g, device="cuda", dtype=torch.float32) * scale).to(dtype)
+
+
+def _rope(positions, dtype):
+    inv = 1.0 / (500000.0 ** (torch.arange(0, D, 2, dtype=torch.float32, device="cuda") / D))
+    ang = positions.to(torch.float32).view(-1, 1) * inv.view(1, -1)
+    ang = torch.cat([ang, ang], dim=-1).unsqueeze(0)
+    return ang.cos().to(dtype), ang.sin().to(dtype)
+
+
+def _paged(g, k, v):
+    """A paged cache holding ``k``/``v [B, K, Hkv, D]`` on randomly permuted 64-token pages."""
+    b, n, h, _ = k.shape
+    pages = -(-n // 64)
+    perm = torch.randperm(b * pages, generator=g, device="cuda").to(torch.int32).view(b, pages)
+    cache = PagedKVCache(b, pages * 64, h, D, torch.device("cuda"), k.dtype, page_table=perm)
+    for i in range(b):
+        for src, dst in ((k[i], cache.k_pages), (v[i], cache.v_pages)):
+            full = torch.zeros((pages * 64, h, D), dtype=src.dtype, device="cuda")
+            full[:n] = src
+            dst[perm[i].long()] = full.view(pages, 64, h, D)
+    cache.length = n
+    return cache
+
+
+def _agreeing_gate(g, hq, hkv, dtype):
+    """Random gate weights, and per head the input directions that these weights map onto one slowly rotating
+    channel direction: ``x [Hkv, D]`` for keys, ``y [Hq, D]`` for queries.  Keys that carry ``x`` in proportion to
+    their block's importance and queries that lean along ``y`` make the heads of a group and the Q-blocks of a
+    chunk agree on the important blocks, which is what selecting a union of blocks rests on; rows of unrelated
+    random data would between them select every block."""
+    wq, wk = _randn(g, (hq, D, D), dtype, 0.02), _randn(g, (hkv, D, D), dtype, 0.02)
+    slow = torch.cat([torch.arange(45, 64), torch.arange(109, 128)]).cuda()
+    inv_k, inv_q = torch.linalg.inv(wk.double()), torch.linalg.inv(wq.double())
+    rows_k, rows_q = inv_k[:, slow], inv_q.view(hkv, hq // hkv, D, D)[:, :, slow]
+    m = rows_k @ rows_k.transpose(1, 2) + (rows_q @ rows_q.transpose(2, 3)).sum(1)
+    d = torch.zeros((hkv, 1, D), dtype=torch.float64, device="cuda")
+    d[:, 0, slow] = torch.linalg.eigh(m).eigenvectors[:, :, 0]
+    x = (d @ inv_k)[:, 0].float()
+    y = (d.repeat_interleave(hq // hkv, dim=0) @ inv_q)[:, 0].float()
+    return wq, wk, x, y
+
+
+def _importance(g, case, power):
+    """``[B, Kb, Hkv]`` in [0, 1]: how much each key block matters to a KV head's queries."""
+    blocks = -(-case["kv_len"] // case["block"])
+    return torch.rand((case["batch"], blocks, case["hkv"]), generator=g, device="cuda") ** power
+
+
+def _per_token(case, a):
+    return a.repeat_interleave(case["block"], dim=1)[:, : case["kv_len"], :, None]
+
+
+def prepare(case, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    dtype, b, n, kv_len, hq, hkv = (DTYPES[case["dtype"]], case["batch"], case["tokens"], case["kv_len"], case["hq"], case["hkv"])
+    past, block = kv_len - n, case["block"]
+    st = {"case": case}
+    with torch.no_grad():
+        return _PREPARE[case["kind"]](st, g, dtype, b, n, kv_len, hq, hkv, past, block)
+
+
+def _prepare_gate(st, g, dtype, b, n, kv_len, hq, hkv, past, block):
+    case = st["case"]
+    wq, wk, x, y = _agreeing_gate(g, hq, hkv, dtype)
+    k = (_randn(g, (b, kv_len, hkv, D), torch.float32) + _per_token(case, _importance(g, case, 3)) * x).to(dtype)
+    v = _randn(g, (b, kv_len, hkv, D), dtype)
+    st["q"] = (_randn(g, (b, n, hq, D), torch.float32) + 1.5 * y).to(dtype)
+    st["k"] = k[:, past:].contiguous()
+    gate = ATTNGATE_CLASSES["Qavg_Kavg"](block, D, D, hkv, hq, force_double=True).cuda().to(dtype)
+    gate.mask_linear_q.weight.copy_(wq)
+    gate.mask_linear_k.weight.copy_(wk)
+    blocks, past_blocks = -(-kv_len // block), past // block
+    rope = _rope(torch.arange(blocks, device="cuda") * block, torch.float32)
+    st["gate"] = GateSelectorState(gate, b, torch.device("cuda"), cache_dtype=dtype)
+    st["gate"].cache.reserve(blocks)
+    gate.append_key_blocks(st["gate"].cache, k[:, :past], tuple(t[:, :past_blocks] for t in rope))
+    st["rope"] = tuple(t[:, past_blocks:].contiguous() for t in rope)
+    st["cache"] = _paged(g, k, v)
+    st["past_blocks"] = past_blocks
+    st["rule"] = SelectionRule(rule="topk", softmax=False, topk_ratio=(int(round(case["density"] * 1000)), 1000), sink=1, local=2)
+    st["out"] = torch.empty_like(st["q"])
+    return st
+
+
+def _prepare_layer(st, g, dtype, b, n, kv_len, hq, hkv, past, block):
+    case, hidden = st["case"], hq * D
+    wq, wk, x, y = _agreeing_gate(g, hq, hkv, dtype)
+    cfg = CompactAttnLlamaConfig(hidden_size=hidden, num_attention_heads=hq, num_key_value_heads=hkv, head_dim=D,
+                                 seerattn_gate_type="Qavg_Kavg", seerattn_gate_force_double=True, seerattn_gate_block_size=block,
+                                 seerattn_sparsity_method="topk", seerattn_topk_ratio=(int(round(case["density"] * 1000)), 1000),
+                                 max_position_embeddings=kv_len, attention_bias=True)
+    module = LlamaSeerAttentionChunkedDense(cfg, 0).cuda().to(dtype).eval()
+    for lin in (module.q_proj, module.k_proj, module.v_proj, module.o_proj):
+        lin.weight.copy_(_randn(g, lin.weight.shape, torch.float32, 0.02))
+        if lin.bias is not None:
+            lin.bias.zero_()
+    module.q_proj.bias.copy_((1.5 * y).reshape(-1))  # the queries' lean
+    module.attn_gate.mask_linear_q.weight.copy_(wq)
+    module.attn_gate.mask_linear_k.weight.copy_(wk)
+    blocks, past_blocks = -(-kv_len // block), past // block
+    k = (_randn(g, (b, past, hkv, D), torch.float32) + _per_token(dict(case, kv_len=past), _importance(g, case, 3)) * x).to(dtype)
+    v = _randn(g, (b, past, hkv, D), dtype)
+    rope = _rope(torch.arange(blocks, device="cuda") * block, torch.float32)
+    pkv = CompactAttnCache(b, blocks * block, torch.device("cuda"), dtype,
+                           page_table=torch.randperm(b * blocks, generator=g, device="cuda").to(torch.int32).view(b, blocks))
+    layer = pkv.layer(0, hkv, D)
+    layer.kv.append(k, v, position=0)
+    layer.gate = GateSelectorState(module.attn_gate, b, torch.device("cuda"), cache_dtype=dtype)
+    layer.gate.cache.reserve(blocks)
+    module.attn_gate.append_key_blocks(layer.gate.cache, k, tuple(t[:, :past_blocks] for t in rope))
+    st.update(module=module, pkv=pkv, layer=layer, past=past, past_blocks=past_blocks)
+    st["block_rope"] = tuple(t[:, past_blocks:].contiguous() for t in rope)
+    st["token_rope"] = _rope(torch.arange(past, kv_len, device="cuda"), dtype)
+    st["hidden"] = _randn(g, (b, n, hidden), dtype)
+    return st
+
+
+def _prepare_keep(st, g, dtype, b, n, kv_len, hq, hkv, past, block):
+    case = st["case"]
+    blocks, q_blocks = -(-kv_len // block), -(-n // block)
+    st["q"], st["k"], st["v"] = (_randn(g, (b, m, h, D), dtype) for m, h in ((n, hq), (kv_len, hkv), (kv_len, hkv)))
+    a = _importance(g, case, 1).permute(0, 2, 1).repeat_interleave(hq // hkv, dim=1)
+    logits = SPREAD * a[:, :, None, :] + 0.1 * torch.randn((b, hq, q_blocks, blocks), generator=g, device="cuda")
+    st["mask"] = torch.ones((q_blocks, blocks), dtype=torch.bool, device="cuda").tril(blocks - q_blocks).view(1, 1, q_blocks, blocks)
+    st["score"] = logits.masked_fill(~st["mask"], float("-inf")).softmax(dim=-1)
+    # a block of importance a gets about exp(SPREAD a) / (blocks * mean of exp(SPREAD a)) of a row's mass
+    st["threshold"] = math.exp(SPREAD * (1.0 - case["density"])) / (blocks * (math.exp(SPREAD) - 1.0) / SPREAD)
+    return st
+
+
+def _prepare_flash(st, g, dtype, b, n, kv_len, hq, hkv, past, block):
+    case = st["case"]
+    lean = torch.nn.functional.normalize(torch.randn((hkv, D), generator=g, device="cuda"), dim=-1)
+    # The row-max rule keeps a block whose score is within log2(1 / ALPHA) of the best one: the importance of the
+    # blocks spreads the scores (log2 units, as q . k / sqrt(D) * log2 e) so that about `density` of them are.
+    lift = math.sqrt(math.log2(1.0 / ALPHA) / case["density"] * math.sqrt(D) * math.log(2.0))
+    k = (_randn(g, (b, kv_len, hkv, D), torch.float32) + lift * _per_token(case, _importance(g, case, 1)) * lean).to(dtype)
+    st["q"] = (_randn(g, (b, n, hq, D), torch.float32) + lift * lean.repeat_interleave(hq // hkv, dim=0)).to(dtype)
+    st["mean_k"] = ops.pool_blocks(k, block, ("avg",), out_dtype=dtype)
+    st["cache"] = _paged(g, k, _randn(g, (b, kv_len, hkv, D), dtype))
+    return st
+
+
+def _prepare_dense(st, g, dtype, b, n, kv_len, hq, hkv, past, block):
+    st["q"] = _randn(g, (b, n, hq, D), dtype)
+    st["cache"] = _paged(g, _randn(g, (b, kv_len, hkv, D), dtype), _randn(g, (b, kv_len, hkv, D), dtype))
+    return st
+
+
+def _prepare_append(st, g, dtype, b, n, kv_len, hq, hkv, past, block):
+    st["q"], st["k"], st["v"] = (_randn(g, (b, n, h, D), dtype) for h in (hq, hkv, hkv))
+    st["cos"], st["sin"] = _rope(torch.arange(past, kv_len, device="cuda"), dtype)
+    st["cache"] = _paged(g, _randn(g, (b, kv_len, hkv, D), dtype), _randn(g, (b, kv_len, hkv, D), dtype))
+    st["mean_k"] = torch.zeros((b, -(-kv_len // block), hkv, D), dtype=dtype, device="cuda")
+    st["past"] = past
+    return st
+
+
+def _prepare_gather(st, g, dtype, b, n, kv_len, hq, hkv, past, block):
+    blocks, past_blocks = kv_len // block, past // block
+    st["cache"] = _paged(g, _randn(g, (b, kv_len, hkv, D), dtype), _randn(g, (b, kv_len, hkv, D), dtype))
+    st["keep"] = torch.rand((b, hkv, blocks), generator=g, device="cuda") < st["case"]["density"]
+    st["past_blocks"] = past_blocks
+    # room for the rows' pages: the mean number of kept blocks and five deviations more
+    kept = min(past_blocks, math.ceil(past_blocks * st["case"]["density"] + 5 * math.sqrt(past_blocks)))
+    pages = b * hkv * -(-(kept * block + n) // 256)
+    st["k_dst"], st["v_dst"] = (torch.zeros((pages * 256, D), dtype=dtype, device="cuda") for _ in range(2))
+    return st
+
+
+_PREPARE = {"gate": _prepare_gate, "layer": _prepare_layer, "keep": _prepare_keep, "flash": _prepare_flash, "dense": _prepare_dense,
+            "append": _prepare_append, "gather": _prepare_gather}
+
+
+# ---------------------------------------------------------------- one pass ---------------------------------------
+def run(st):
+    c = st["case"]
+    kind, n, kv_len, hq, hkv, block = c["kind"], c["tokens"], c["kv_len"], c["hq"], c["hkv"], c["block"]
+    if kind == "gate":
+        sel = st["gate"]
+        sel.cache.length = st["past_blocks"]  # the chunk's blocks go after the past ones, pass after pass
+        sel.append(st["q"], st["k"], st["rope"], st["rope"])
+        table = sel.score_select(st["rule"], hkv, block)
+        return ops.attn_compact(st["q"], st["cache"].view(), kv_len, hkv, table.block_idx, table.counts, block_size=block, out=st["out"])
+    if kind == "layer":
+        layer = st["layer"]
+        layer.kv.length, layer.gate.cache.length = st["past"], st["past_blocks"]
+        with torch.no_grad():
+            return st["module"](st["hidden"], st["token_rope"], None, past_key_value=st["pkv"], block_position_embeddings=st["block_rope"])[0]
+    if kind == "keep":
+        return chunked_prefill_column_dense_attention_forward(
+            st["q"], st["k"], st["v"], None, n, softmax_scale=D ** -0.5, attn_gate_score=st["score"], block_attention_mask=st["mask"],
+            threshold=st["threshold"], block_size=block, num_key_value_groups=hq // hkv)[0]
+    if kind == "flash":
+        view = st["cache"].view()
+        return flashprefill_compactattn_prefill_full_kv(
+            st["q"], view, view, None, softmax_scale=D ** -0.5, num_key_value_groups=hq // hkv, block_size=block, attention_sink=2,
+            window_size=4, alpha=ALPHA, last_n_block=0, min_budget=0, pack_impl="indexed_dense", indexed_impl="b200_native",
+            cache_fill_backend="auto", mean_k_cache=st["mean_k"], kv_len=kv_len)[0]
+    if kind == "dense":
+        return ops.attn_compact(st["q"], st["cache"].view(), kv_len, hkv, None, None, block_size=block)
+    if kind == "append":
+        q, _ = st["cache"].append_rope(st["q"], st["k"], st["v"], st["cos"], st["sin"], position=st["past"], mean_k=st["mean_k"],
+                                       block_size=block)
+        return {"q": q, "k": st["cache"].k_pages, "v": st["cache"].v_pages, "mean_k": st["mean_k"]}
+    view = st["cache"].view()
+    table = ops.union_table(mask=st["keep"], num_kv_heads=hkv, kv_blocks=kv_len // block, past_blocks=st["past_blocks"], block_size=block)
+    offsets, _ = ops.paged_metadata(table.pages_per_row)
+    ops.gather_kv(view, hkv, c["batch"], n, kv_len, table.block_idx, table.counts, st["k_dst"], st["v_dst"], block_size=block,
+                  page_offsets=offsets)
+    return {"k": st["k_dst"], "v": st["v_dst"], "counts": table.counts, "offsets": offsets}
+
+
+def work(case):
+    b, n, kv_len, hq, hkv, block = (case[k] for k in ("batch", "tokens", "kv_len", "hq", "hkv", "block"))
+    past, kind = kv_len - n, case["kind"]
+    chosen = past * (case["density"] if kind != "layer" or n > 1 else 1.0)  # past tokens read by a KV head
+    qo = 2 * 2 * b * n * hq * D  # queries in, outputs (or rotated queries) out
+    kv_bytes = 2 * 2 * b * hkv * D * (chosen + n)
+    blocks, q_blocks = -(-kv_len // block), -(-n // block)
+    if kind == "append":
+        return {"bytes": qo + 2 * 2 * 2 * b * n * hkv * D, "flops": 0}
+    if kind == "gather":
+        return {"bytes": 2 * kv_bytes, "flops": 0}
+    flops = 4 * D * b * hq * (n * chosen + n * (n + 1) / 2)
+    nbytes = qo + kv_bytes
+    if kind == "keep":
+        nbytes += 4 * b * hq * q_blocks * blocks  # the scores
+    elif kind == "flash":
+        nbytes += 2 * b * blocks * hkv * D  # the mean keys
+        flops += 2 * D * b * hq * n * blocks
+    elif kind in ("gate", "layer") and n > 1:
+        nbytes += 2 * b * blocks * hkv * D  # the key blocks
+        flops += 2 * D * b * hq * q_blocks * blocks
+    if kind == "layer":
+        hidden = hq * D
+        flops += 2 * b * n * hidden * D * (2 * hq + 2 * hkv)
+        nbytes += 2 * hidden * D * (2 * hq + 2 * hkv) + 2 * 2 * b * n * hidden
+    return {"bytes": nbytes, "flops": flops}
+
+
+def tolerance(case):
+    """Measured against the same path in 64 bits (scores, selection and attention; 16-bit rounding of what the
+    entry points store): attention outputs are off by 2.3e-3 (bf16; 2.9e-3 through the layer's projections) and
+    2.9e-4 (f16), their largest entry by 2.7e-2 and 5.8e-3.  The rotated queries, the cache and the pooled keys
+    came out the same; a mean summed in another order may now and then round the other way."""
+    if case["kind"] == "gather":
+        return "exact"
+    if case["kind"] == "append":
+        return {"rel": 1e-4, "max": 1e-2}
+    return {"rel": 1e-2, "max": 0.1} if case["dtype"] == "bf16" else {"rel": 1.2e-3, "max": 0.025}
