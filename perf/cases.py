@@ -386,3 +386,146 @@ def tolerance(case):
     if case["kind"] == "append":
         return {"rel": 1e-4, "max": 1e-2}
     return {"rel": 1e-2, "max": 0.1} if case["dtype"] == "bf16" else {"rel": 1.2e-3, "max": 0.025}
+
+
+# ---------------------------------------------------------------- the same in 64 bits ------------------------------
+def exact(case, seed):
+    """What ``run`` returns, in plain torch and 64 bits on the same inputs; what the entry points store in 16 bits
+    on the way (projections, rotated keys, key blocks, the attention output before a projection) is rounded there
+    as they round it.  None for bytes that are only moved."""
+    if case["kind"] == "gather":
+        return None
+    with torch.no_grad():
+        return _EXACT[case["kind"]](case, prepare(case, seed))
+
+
+def _rotate64(x, cos, sin):
+    """``x [B, L, H, D]`` with tables ``[1, L, D]``."""
+    x, half = x.double(), x.shape[-1] // 2
+    return x * cos.double().unsqueeze(2) + torch.cat([-x[..., half:], x[..., :half]], dim=-1) * sin.double().unsqueeze(2)
+
+
+def _stored(cache, pages, kv_len):
+    return pages[cache.page_table.long()].flatten(1, 2)[:, :kv_len]
+
+
+def _attention64(case, q, k, v, keep=None):
+    """``keep [B, Hkv, blocks]``: the past key blocks that a KV head attends (None: all); the chunk is causal."""
+    b, n, hq, _ = q.shape
+    hkv, kv_len, block = case["hkv"], case["kv_len"], case["block"]
+    past, group = kv_len - n, hq // hkv
+    out = torch.empty(q.shape, dtype=torch.float64, device=q.device)
+    for i in range(b):
+        for h in range(hkv):
+            token = torch.arange(kv_len, device=q.device)
+            if keep is not None:
+                token = token[keep[i, h].repeat_interleave(block)[:kv_len] | (token >= past)]
+            kk, vv = k[i, token, h].double(), v[i, token, h].double()
+            step = max(1, (1 << 26) // (group * token.numel()))
+            for t in range(0, n, step):
+                rows = q[i, t : t + step, h * group : (h + 1) * group].double()
+                hidden = token.view(1, -1) > past + torch.arange(t, t + rows.shape[0], device=q.device).view(-1, 1)
+                s = (rows.flatten(0, 1) @ kk.T * D ** -0.5).view(rows.shape[0], group, -1).masked_fill_(hidden.unsqueeze(1), -math.inf)
+                out[i, t : t + step, h * group : (h + 1) * group] = s.softmax(dim=-1) @ vv
+    return out
+
+
+def _pool64(x, block):
+    whole = x.shape[1] // block * block
+    parts = [x[:, :whole].double().unflatten(1, (-1, block)).mean(2)]
+    if whole < x.shape[1]:
+        parts.append(x[:, whole:].double().mean(1, keepdim=True))
+    return torch.cat(parts, dim=1)
+
+
+def _blocks_of(case, device):
+    """Key block ids ``[Kb]`` and how far each lies behind a row's own block ``[Qb, Kb]``."""
+    q_blocks, blocks = -(-case["tokens"] // case["block"]), -(-case["kv_len"] // case["block"])
+    key = torch.arange(blocks, device=device)
+    return key, (blocks - q_blocks + torch.arange(q_blocks, device=device)).view(-1, 1) - key
+
+
+def _gate_keep64(case, wq, wk, q, k, rope, past_blocks_cached, dtype):
+    """Top-k of the gate's logits per row, the first block and the last two; the union over a KV head's rows."""
+    q_blocks = _rotate64(torch.einsum("bnhi,hio->bnho", _pool64(q, case["block"]), wq.double()), *rope)
+    k_blocks = _rotate64(torch.einsum("bnhi,hio->bnho", _pool64(k, case["block"]), wk.double()), *rope).to(dtype)
+    k_blocks = torch.cat([past_blocks_cached, k_blocks], dim=1).double()
+    key, behind = _blocks_of(case, q.device)
+    k_blocks = k_blocks.repeat_interleave(q_blocks.shape[2] // k_blocks.shape[2], dim=2)
+    score = torch.einsum("bihd,bjhd->bhij", q_blocks, k_blocks).masked_fill(behind < 0, -math.inf)
+    num, den = int(round(case["density"] * 1000)), 1000
+    visible = (behind >= 0).sum(1)
+    size = ((num * visible + den // 2) // den).clamp(min=1).view(-1, 1)
+    rank = score.sort(dim=-1, descending=True, stable=True).indices.argsort(dim=-1)
+    keep = ((rank < size) | (key < 1) | (behind < 2)) & (behind >= 0)
+    return keep.any(2).unflatten(1, (case["hkv"], -1)).any(2)
+
+
+def _exact_gate(case, st):
+    gate = st["gate"].gate
+    keep = _gate_keep64(case, gate.mask_linear_q.weight, gate.mask_linear_k.weight, st["q"], st["k"], st["rope"],
+                        st["gate"].cache.blocks_view()[:, : st["past_blocks"]], st["q"].dtype)
+    return _attention64(case, st["q"], *(_stored(st["cache"], p, case["kv_len"]) for p in (st["cache"].k_pages, st["cache"].v_pages)), keep)
+
+
+def _exact_layer(case, st):
+    module, x, cache, past = st["module"], st["hidden"], st["layer"].kv, st["past"]
+    dtype = x.dtype
+
+    def project(lin, value):
+        y = value.double() @ lin.weight.double().T
+        return y if lin.bias is None else y + lin.bias.double()
+
+    q, k, v = (project(lin, x).to(dtype).unflatten(-1, (-1, D)) for lin in (module.q_proj, module.k_proj, module.v_proj))
+    keep = None
+    if case["tokens"] > 1:
+        keep = _gate_keep64(case, module.attn_gate.mask_linear_q.weight, module.attn_gate.mask_linear_k.weight, q, k, st["block_rope"],
+                            st["layer"].gate.cache.blocks_view()[:, : st["past_blocks"]], dtype)
+    kk = torch.cat([_stored(cache, cache.k_pages, past), _rotate64(k, *st["token_rope"]).to(dtype)], dim=1)
+    vv = torch.cat([_stored(cache, cache.v_pages, past), v], dim=1)
+    attn = _attention64(case, _rotate64(q, *st["token_rope"]).to(dtype), kk, vv, keep).to(dtype)
+    return project(module.o_proj, attn.flatten(2))
+
+
+def _exact_keep(case, st):
+    keep = ((st["score"] > st["threshold"]) & st["mask"]).any(2).unflatten(1, (case["hkv"], -1)).any(2)
+    keep[..., -2:] = True  # the operator's keep_recent_blocks
+    return _attention64(case, st["q"], st["k"], st["v"], keep)
+
+
+def _exact_flash(case, st):
+    q, mean_k, block = st["q"], st["mean_k"].double(), case["block"]
+    b, n, hq, _ = q.shape
+    key, behind = _blocks_of(case, q.device)
+    last = (key + 1) * block - 1
+    score = torch.full((b, hq, behind.shape[0], key.numel()), -math.inf, dtype=torch.float64, device=q.device)
+    for i in range(behind.shape[0]):
+        token = torch.arange(i * block, min((i + 1) * block, n), device=q.device)
+        rows = q[:, token].double().transpose(1, 2)  # [B, Hq, T, D]
+        s = rows @ mean_k.permute(0, 2, 3, 1).repeat_interleave(hq // case["hkv"], dim=1) * (D ** -0.5)
+        s = s.masked_fill((case["kv_len"] - n + token).view(-1, 1) < last, -math.inf)
+        score[:, :, i] = s.logsumexp(dim=2)
+    best = score.masked_fill(behind < 0, -math.inf).amax(dim=-1, keepdim=True)
+    keep = ((score >= best + math.log(ALPHA)) | (key < 2) | (behind < 4)) & (behind >= 0)
+    keep = keep.any(2).unflatten(1, (case["hkv"], -1)).any(2)
+    return _attention64(case, q, *(_stored(st["cache"], p, case["kv_len"]) for p in (st["cache"].k_pages, st["cache"].v_pages)), keep)
+
+
+def _exact_dense(case, st):
+    return _attention64(case, st["q"], *(_stored(st["cache"], p, case["kv_len"]) for p in (st["cache"].k_pages, st["cache"].v_pages)))
+
+
+def _exact_append(case, st):
+    cache, past, block = st["cache"], st["past"], case["block"]
+    token = torch.arange(past, case["kv_len"], device=st["q"].device)
+    page, slot = cache.page_table.long()[:, token // 64], token % 64
+    k = _rotate64(st["k"], st["cos"], st["sin"])
+    k_pages, v_pages, mean_k = cache.k_pages.double(), cache.v_pages.double(), st["mean_k"].double()
+    k_pages[page, slot] = k
+    v_pages[page, slot] = st["v"].double()
+    mean_k[:, past // block :] = _pool64(k.to(st["k"].dtype), block)
+    return {"q": _rotate64(st["q"], st["cos"], st["sin"]), "k": k_pages, "v": v_pages, "mean_k": mean_k}
+
+
+_EXACT = {"gate": _exact_gate, "layer": _exact_layer, "keep": _exact_keep, "flash": _exact_flash, "dense": _exact_dense,
+          "append": _exact_append}
