@@ -25,7 +25,7 @@
 // MMA order S_A0 S_B0 { PV_A(j) S_A(j+1) PV_B(j) S_B(j+1) } so one tile's softmax overlaps the
 // other tile's MMAs.  Every wait is bounded; on expiry the CTA raises CA_STATUS_TIMEOUT, drains
 // what it issued, frees TMEM and returns.
-#include "ca_common.cuh"
+#include "ca_attn_shared.cuh"
 
 #include <mutex>
 
@@ -916,6 +916,31 @@ static int encode_map(CUtensorMap* map, CUtensorMapDataType dt, int rank, const 
   return CA_OK;
 }
 
+int encode_kv_maps(const ca_attn_params* p, CUtensorMap* k_map, CUtensorMap* v_map, int (&slot_of_role)[3]) {
+  const CUtensorMapDataType dt = p->dtype == CA_DTYPE_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
+  // roles: 0 token-in-page, 1 page, 2 head; outer dimensions sorted by ascending stride
+  const cuuint64_t role_dim[3] = {(cuuint64_t)p->kv.page_size, (cuuint64_t)p->kv.num_pages,
+                                  (cuuint64_t)(p->Hkv / (p->kv.head_div > 1 ? p->kv.head_div : 1))};
+  const cuuint64_t role_stride[3] = {(cuuint64_t)p->kv.token_stride * 2, (cuuint64_t)p->kv.page_stride * 2,
+                                     (cuuint64_t)p->kv.head_stride * 2};
+  const cuuint32_t role_box[3] = {64, 1, 1};
+  int order[3] = {0, 1, 2};
+  for (int i = 0; i < 3; ++i)
+    for (int j = i + 1; j < 3; ++j)
+      if (role_stride[order[j]] < role_stride[order[i]]) { int t = order[i]; order[i] = order[j]; order[j] = t; }
+  cuuint64_t dims[4] = {(cuuint64_t)kHeadDim, 0, 0, 0};
+  cuuint64_t strides[3];
+  cuuint32_t box[4] = {64, 0, 0, 0};
+  for (int i = 0; i < 3; ++i) {
+    dims[i + 1] = role_dim[order[i]];
+    strides[i] = role_stride[order[i]];
+    box[i + 1] = role_box[order[i]];
+    slot_of_role[order[i]] = i;
+  }
+  const int rc = encode_map(k_map, dt, 4, p->kv.k, dims, strides, box, "k");
+  return rc != CA_OK ? rc : encode_map(v_map, dt, 4, p->kv.v, dims, strides, box, "v");
+}
+
 static int validate(const ca_attn_params* p) {
   CA_REQUIRE(p != nullptr, "params is null");
   CA_REQUIRE(p->q && p->out && p->kv.k && p->kv.v, "q, out, kv.k and kv.v must be non-null");
@@ -1022,6 +1047,7 @@ int ca_attn_compact(const ca_attn_params* p, ca_stream_t stream_) {
   rc = get_device_info(&dev);
   if (rc != CA_OK) return rc;
   if (dev.cc_major != 10) return fail(CA_ERR_UNSUPPORTED, "this library targets sm_100a; device is sm_%d%d", dev.cc_major, dev.cc_minor);
+  if (decode_applies(p)) return launch_decode(p, dev, stream);
 
   const int G = p->Hq / p->Hkv;
   const int tpt = kTileM / G;
@@ -1030,7 +1056,7 @@ int ca_attn_compact(const ca_attn_params* p, ca_stream_t stream_) {
   const CUtensorMapDataType dt = p->dtype == CA_DTYPE_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
 
   CUtensorMap q_map, k_map, v_map;
-  int slot_tok = 0, slot_page = 1, slot_head = 2;
+  int slots[3];
   {
     // (d, g, hkv, token, batch): the box walks g fastest, then tokens, so tile row = token*G + g
     cuuint64_t dims[5] = {(cuuint64_t)kHeadDim, (cuuint64_t)G, (cuuint64_t)p->Hkv, (cuuint64_t)p->Q, (cuuint64_t)p->B};
@@ -1040,33 +1066,8 @@ int ca_attn_compact(const ca_attn_params* p, ca_stream_t stream_) {
     rc = encode_map(&q_map, dt, 5, p->q, dims, strides, box, "q");
     if (rc != CA_OK) return rc;
   }
-  {
-    // roles: 0 token-in-page, 1 page, 2 head; outer dimensions sorted by ascending stride
-    const cuuint64_t role_dim[3] = {(cuuint64_t)p->kv.page_size, (cuuint64_t)p->kv.num_pages,
-                                    (cuuint64_t)(p->Hkv / (p->kv.head_div > 1 ? p->kv.head_div : 1))};
-    const cuuint64_t role_stride[3] = {(cuuint64_t)p->kv.token_stride * 2, (cuuint64_t)p->kv.page_stride * 2,
-                                       (cuuint64_t)p->kv.head_stride * 2};
-    const cuuint32_t role_box[3] = {64, 1, 1};
-    int order[3] = {0, 1, 2};
-    for (int i = 0; i < 3; ++i)
-      for (int j = i + 1; j < 3; ++j)
-        if (role_stride[order[j]] < role_stride[order[i]]) { int t = order[i]; order[i] = order[j]; order[j] = t; }
-    cuuint64_t dims[4] = {(cuuint64_t)kHeadDim, 0, 0, 0};
-    cuuint64_t strides[3];
-    cuuint32_t box[4] = {64, 0, 0, 0};
-    int slot_of_role[3];
-    for (int i = 0; i < 3; ++i) {
-      dims[i + 1] = role_dim[order[i]];
-      strides[i] = role_stride[order[i]];
-      box[i + 1] = role_box[order[i]];
-      slot_of_role[order[i]] = i;
-    }
-    slot_tok = slot_of_role[0], slot_page = slot_of_role[1], slot_head = slot_of_role[2];
-    rc = encode_map(&k_map, dt, 4, p->kv.k, dims, strides, box, "k");
-    if (rc != CA_OK) return rc;
-    rc = encode_map(&v_map, dt, 4, p->kv.v, dims, strides, box, "v");
-    if (rc != CA_OK) return rc;
-  }
+  rc = encode_kv_maps(p, &k_map, &v_map, slots);
+  if (rc != CA_OK) return rc;
 
   KernelArgs a;
   a.Q = p->Q;
@@ -1100,9 +1101,9 @@ int ca_attn_compact(const ca_attn_params* p, ca_stream_t stream_) {
   a.idesc_pv = ptx::make_idesc_f16(fmt, kTileM, kHeadDim, 0, 1);
   a.wait_limit_ns = 2000000000ull;
   a.kv_head_div = p->kv.head_div > 1 ? p->kv.head_div : 1;
-  a.slot_tok = slot_tok;
-  a.slot_page = slot_page;
-  a.slot_head = slot_head;
+  a.slot_tok = slots[0];
+  a.slot_page = slots[1];
+  a.slot_head = slots[2];
 
   // persistent grid: one CTA per SM, never more CTAs than units when units cannot be cut
   const long long n_units = static_cast<long long>(p->B) * p->Hkv * n_pairs;
