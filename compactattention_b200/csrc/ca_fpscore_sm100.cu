@@ -323,7 +323,7 @@ int launch_fp_score_sm100(const ca_flashprefill_score_params* p, cudaStream_t st
   a.wait_limit_ns = 2000000000ull;
   a.status = nullptr;
   CA_CUDA(cudaFuncSetAttribute(fp_score_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-  launch_kernel(fp_score_kernel, dim3(a.Qb, p->Hkv, p->B), dim3(kThreads), smem, stream, q_map, k_map, a);
+  launch_kernel_as(true, fp_score_kernel, dim3(a.Qb, p->Hkv, p->B), dim3(kThreads), smem, stream, q_map, k_map, a);
   CA_LAUNCH_CHECK("fp_score_kernel");
   return CA_OK;
 }

@@ -174,7 +174,7 @@ int ca_gather_kv(const ca_gather_params* p, ca_stream_t stream_) {
   a.status = p->status;
   // persistent grid: a multiple of the SM count, 8 CTAs of 256 threads per SM
   const int grid = dev.sm_count * 8;
-  launch_kernel(gather_kv_kernel, dim3(grid), dim3(kThreads), 0, static_cast<cudaStream_t>(stream_), a);
+  launch_kernel_as(true, gather_kv_kernel, dim3(grid), dim3(kThreads), 0, static_cast<cudaStream_t>(stream_), a);
   CA_LAUNCH_CHECK("gather_kv_kernel");
   return CA_OK;
 }

@@ -853,7 +853,7 @@ int ca_pool_blocks(const ca_pool_params* p, ca_stream_t stream_) {
   const int nb = ceil_div(p->L, p->block_size);
   const int phases = kPoolThreads / (p->D / 8);
   const size_t smem = static_cast<size_t>(3) * phases * p->D * sizeof(float);
-  launch_kernel(pool_blocks_kernel, dim3(nb, p->B * p->H), dim3(kPoolThreads), smem, static_cast<cudaStream_t>(stream_), a);
+  launch_kernel_as(true, pool_blocks_kernel, dim3(nb, p->B * p->H), dim3(kPoolThreads), smem, static_cast<cudaStream_t>(stream_), a);
   CA_LAUNCH_CHECK("pool_blocks_kernel");
   return CA_OK;
 }

@@ -812,6 +812,9 @@ struct UnionArgs {
   uint8_t* keep_kv;         // optional bool [B,Hkv,Kb]: union with every chunk column on
 };
 
+// Bit t of the result: byte t of x is not zero.
+__device__ __forceinline__ uint32_t mask_bits(uint32_t x) { return (__vsetgtu4(x, 0u) * 0x10204080u) >> 28; }
+
 __global__ void __launch_bounds__(kRowThreads) union_table_kernel(const UnionArgs a) {
   ptx::grid_launch_dependents();
   ptx::grid_dependency_wait();  // nothing in global memory is touched before this
@@ -836,7 +839,15 @@ __global__ void __launch_bounds__(kRowThreads) union_table_kernel(const UnionArg
       const uint8_t* m = a.mask + b * a.m_b + h * a.m_h + i * a.m_q;
       const int j0 = w * 32;
       const int n = a.Kb - j0 < 32 ? a.Kb - j0 : 32;
-      for (int t = 0; t < n; ++t) word |= (m[(j0 + t) * a.m_k] ? 1u : 0u) << t;
+      const uint8_t* m0 = m + j0 * a.m_k;
+      if (a.m_k == 1 && n == 32 && (reinterpret_cast<uintptr_t>(m0) & 15u) == 0) {
+        // 32 entries in two loads: one latency instead of 32 byte loads that the compiler issues a few at a time
+        const uint4 lo = *reinterpret_cast<const uint4*>(m0), hi = *reinterpret_cast<const uint4*>(m0 + 16);
+        word = mask_bits(lo.x) | mask_bits(lo.y) << 4 | mask_bits(lo.z) << 8 | mask_bits(lo.w) << 12 | mask_bits(hi.x) << 16 |
+               mask_bits(hi.y) << 20 | mask_bits(hi.z) << 24 | mask_bits(hi.w) << 28;
+      } else {
+        for (int t = 0; t < n; ++t) word |= (m0[t * a.m_k] ? 1u : 0u) << t;
+      }
     }
     if (word) atomicOr(&words[w], word);
   }
@@ -1011,7 +1022,7 @@ int ca_select_rows(const ca_select_params* p, ca_stream_t stream_) {
   size_t smem = 0;
   int rc = fill_row_args(p, &a, &smem, true);
   if (rc != CA_OK) return rc;
-  launch_kernel(select_rows_kernel, dim3(p->B * p->H * p->Qb), dim3(kRowThreads), smem, static_cast<cudaStream_t>(stream_), a);
+  launch_kernel_as(true, select_rows_kernel, dim3(p->B * p->H * p->Qb), dim3(kRowThreads), smem, static_cast<cudaStream_t>(stream_), a);
   CA_LAUNCH_CHECK("select_rows_kernel");
   return CA_OK;
 }
@@ -1129,7 +1140,7 @@ int ca_union_table(const ca_union_params* p, ca_stream_t stream_) {
   a.block_idx = p->block_idx, a.idx_stride = p->idx_stride, a.counts = p->counts;
   a.cache_seqlens = p->cache_seqlens, a.pages_per_row = p->pages_per_row;
   a.keep_kv = static_cast<uint8_t*>(p->keep_kv);
-  launch_kernel(union_table_kernel, dim3(p->B * p->Hkv), dim3(kRowThreads), 0, static_cast<cudaStream_t>(stream_), a);
+  launch_kernel_as(true, union_table_kernel, dim3(p->B * p->Hkv), dim3(kRowThreads), 0, static_cast<cudaStream_t>(stream_), a);
   CA_LAUNCH_CHECK("union_table_kernel");
   return CA_OK;
 }
@@ -1141,7 +1152,7 @@ int ca_paged_metadata(const int32_t* pages_per_row, int rows, int32_t* page_offs
   CA_REQUIRE(pages_per_row && page_offsets, "pages_per_row and page_offsets must be non-null");
   CA_REQUIRE(rows > 0, "rows must be positive");
   CA_REQUIRE(block_table == nullptr || max_pages > 0, "max_pages must be positive with a block_table");
-  launch_kernel(paged_metadata_kernel, dim3(1), dim3(kRowThreads), 0, static_cast<cudaStream_t>(stream_), pages_per_row, rows, page_offsets,
+  launch_kernel_as(true, paged_metadata_kernel, dim3(1), dim3(kRowThreads), 0, static_cast<cudaStream_t>(stream_), pages_per_row, rows, page_offsets,
                                                                                     block_table, max_pages);
   CA_LAUNCH_CHECK("paged_metadata_kernel");
   return CA_OK;

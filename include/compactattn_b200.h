@@ -47,12 +47,11 @@ int ca_abi_version(void);
 /* Number of kernel launches the library has enqueued in this process (all entry points). */
 int64_t ca_launch_count(void);
 /*
- * Programmatic dependent launch (off by default): when enabled, every kernel is enqueued so that
- * its CTAs may become resident and run their prologue while the previous kernel in the stream
- * drains; each kernel waits (griddepcontrol.wait) before its first global-memory access, so
- * results do not change.  Measured on B200: the selection chain gains 2-3 us per step, the long
- * attention launch gains nothing, so plain launches stay the default.  Returns the previous
- * setting.  No reference counterpart (the reference launches through torch / Triton).
+ * Programmatic dependent launch of the kernels that are enqueued plainly otherwise (off by default; the kernels of
+ * the path - append, pooling, gate, scores, selection, table, gather, attention - are always enqueued so): a
+ * kernel's CTAs may become resident and run their prologue while the previous kernel in the stream drains; each
+ * kernel waits (griddepcontrol.wait) before its first global-memory access, so results do not change.  Returns the
+ * previous setting.  No reference counterpart (the reference launches through torch / Triton).
  */
 int ca_set_programmatic_launch(int enabled);
 
