@@ -46,12 +46,9 @@ constexpr int kMaxRows = 1024;  // (batch x kv heads) rows per launch
 constexpr int kMaxSegs = 64;    // segments planned per batch
 constexpr float kRescaleThreshold = 8.0f;  // log2 units; lazy accumulator rescale
 constexpr int kMinSpanSteps = 8;           // shortest span worth a CTA of its own when units are cut
-#ifndef CA_ATTN_MIN_UNIT_STEPS
-#define CA_ATTN_MIN_UNIT_STEPS 24
-#endif
-// (units of 27-30 KV steps: 44 us cut against 66 us whole, so the threshold must stay below that;
-// units of ~6 steps: 22 us whole against 45 us cut)
-constexpr int kMinUnitStepsToCut = CA_ATTN_MIN_UNIT_STEPS;  // average KV steps per unit below which units stay whole
+// What cutting units costs a CTA (partials, the merge), in KV steps of about 2.2 us.  32 units of 27-30 steps: 44 us
+// cut, 66 us whole; of ~6 steps: 45 us cut, 22 us whole; of ~20 steps the two tie (54 us cut, 41 us whole).
+constexpr int kCutCostSteps = 12;
 // Measured on B200 (sustained 300-launch loop, 128K context, 20 % density): handing P to the MMA warp
 // in two halves 434 us, in one piece 450 us; packed fp32 pairs for the scale and the row sum 421 us.
 // A polynomial exp2 on the FMA pipe for part of the exponentials (2 / 4 / 6 of every 16 pairs) took
@@ -130,7 +127,6 @@ struct KernelArgs {
   int slot_tok, slot_page, slot_head;
   int kv_head_div;     // block-table rows per KV head (1 unless per-query-head / sub-group tables)
   int split;           // 1: spans may cut units (needs the workspace)
-  int max_cut_steps;   // > 0: units longer than this many KV steps on average stay whole
   SegDesc* descs;      // [2 * gridDim.x]
   float* part_ml;      // [2 * gridDim.x][kPartialMLFloats]
   float* part_o;       // [2 * gridDim.x][kPartialOFloats]
@@ -138,6 +134,7 @@ struct KernelArgs {
 
 struct Shared {
   uint64_t q_full[2];
+  uint64_t q_free;
   uint64_t ring_full[kStages];
   uint64_t ring_empty[kStages];
   uint64_t s_full[2];
@@ -149,7 +146,9 @@ struct Shared {
   int abort_flag;
   int n_segs;
   int more;            // another batch of segments follows
-  long long next_x;    // linear KV-step index where the next batch starts
+  int cut;             // spans may end inside a unit
+  int cur_row, cur_pair;        // the unit the next segment comes from ...
+  long long cur_acc, next_x;    // ... its first linear KV step, and the step where the next segment starts
   int row_count[kMaxRows];
   long long row_prefix[kMaxRows + 1];
   Segment segs[kMaxSegs];
@@ -189,32 +188,50 @@ __device__ __forceinline__ int unit_iters(const KernelArgs& a, int count, int pa
   return (count * a.spb + chunk_subs(a, pair) + 1) >> 1;
 }
 
-// Plans up to kMaxSegs segments of this CTA's span starting at linear step x (thread 0 only).
-__device__ void plan_segments(const KernelArgs& a, Shared* sh, long long x, long long span_begin, long long span_end,
-                              int R) {
-  int n = 0;
-  // row containing x: largest r with row_prefix[r] <= x
-  int lo = 0, hi = R;
+// Finds the unit that holds linear KV step x (one warp, all lanes): its row and pair, its first step.
+__device__ void locate_unit(const KernelArgs& a, const Shared* sh, long long x, int R, int lane, int* row, int* pair, long long* acc) {
+  int lo = 0, hi = R;  // largest row with row_prefix[row] <= x
   while (hi - lo > 1) {
     const int mid = (lo + hi) >> 1;
     if (sh->row_prefix[mid] <= x) lo = mid; else hi = mid;
   }
-  int row = lo;
-  long long acc = sh->row_prefix[row];
-  int pair = 0;
+  long long base = sh->row_prefix[lo];
+  const int count = sh->row_count[lo];
+  *row = lo, *pair = 0, *acc = base;
+  for (int p0 = 0; p0 < a.n_pairs; p0 += 32) {
+    const int p = p0 + lane;
+    const int ni = p < a.n_pairs ? unit_iters(a, count, p) : 0;
+    int inc = ni;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int n = __shfl_up_sync(0xffffffffu, inc, d);
+      if (lane >= d) inc += n;
+    }
+    const uint32_t hit = __ballot_sync(0xffffffffu, p < a.n_pairs && base + inc > x);
+    if (hit) {
+      const int l = __ffs(hit) - 1;
+      *pair = p0 + l;
+      *acc = base + __shfl_sync(0xffffffffu, inc - ni, l);
+      return;
+    }
+    base += __shfl_sync(0xffffffffu, inc, 31);
+  }
+}
+
+// Plans up to kMaxSegs further segments of this CTA's span (thread 0 only).
+__device__ void plan_segments(const KernelArgs& a, Shared* sh, long long span_begin, long long span_end, int R) {
+  int n = 0;
+  int row = sh->cur_row, pair = sh->cur_pair;
+  long long acc = sh->cur_acc, x = sh->next_x;
+  const bool cut = sh->cut != 0;
   while (x < span_end && n < kMaxSegs && row < R) {
     const int count = sh->row_count[row];
     const int ni = unit_iters(a, count, pair);
-    if (x >= acc + ni) {  // unit lies before x: walk on
-      acc += ni;
-      if (++pair == a.n_pairs) pair = 0, ++row;
-      continue;
-    }
     Segment s;
     s.row = row, s.pair = pair;
     s.j0 = static_cast<int>(x - acc);
     const long long rem = span_end - acc;
-    s.j1 = rem < ni ? static_cast<int>(rem) : ni;
+    s.j1 = cut && rem < ni ? static_cast<int>(rem) : ni;
     s.n_past_sub = count * a.spb;
     s.n_sub = s.n_past_sub + chunk_subs(a, pair);
     const bool partial = !(s.j0 == 0 && s.j1 == ni);
@@ -227,9 +244,11 @@ __device__ void plan_segments(const KernelArgs& a, Shared* sh, long long x, long
     }
     sh->segs[n++] = s;
     x = acc + s.j1;
+    acc += ni;
+    if (++pair == a.n_pairs) pair = 0, ++row;
   }
   sh->n_segs = n;
-  sh->next_x = x;
+  sh->cur_row = row, sh->cur_pair = pair, sh->cur_acc = acc, sh->next_x = x;
   sh->more = (x < span_end && row < R) ? 1 : 0;
 }
 
@@ -295,6 +314,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     sh->abort_flag = 0;
     ptx::mbar_init(ptx::smem_u32(&sh->q_full[0]), 1);
     ptx::mbar_init(ptx::smem_u32(&sh->q_full[1]), 1);
+    ptx::mbar_init(ptx::smem_u32(&sh->q_free), 1);
     for (int s = 0; s < kStages; ++s) {
       ptx::mbar_init(ptx::smem_u32(&sh->ring_full[s]), 1);
       ptx::mbar_init(ptx::smem_u32(&sh->ring_empty[s]), 1);
@@ -323,8 +343,8 @@ __global__ void __launch_bounds__(kThreads, 1)
   }
   ptx::grid_dependency_wait();  // nothing in global memory is touched before this
 
-  // ---- per-row KV-step totals and their prefix (every CTA; a few thousand integer operations) ----
-  for (int r = tid; r < R; r += kThreads) {
+  // ---- per-row KV-step totals and their prefix (every CTA; a warp per row) ----
+  for (int r = warp; r < R; r += kThreads / 32) {
     int count = a.past_blocks;
     if (a.block_idx != nullptr) {
       count = a.counts[r];
@@ -334,10 +354,13 @@ __global__ void __launch_bounds__(kThreads, 1)
         count = count < 0 ? 0 : cap;
       }
     }
-    sh->row_count[r] = count;
-    long long tot = 0;
-    for (int p = 0; p < a.n_pairs; ++p) tot += unit_iters(a, count, p);
-    sh->row_prefix[r + 1] = tot;  // turned into a prefix below
+    int tot = 0;
+    for (int p = lane; p < a.n_pairs; p += 32) tot += unit_iters(a, count, p);
+    tot = __reduce_add_sync(0xffffffffu, tot);
+    if (lane == 0) {
+      sh->row_count[r] = count;
+      sh->row_prefix[r + 1] = tot;  // turned into a prefix below
+    }
   }
   if (tid == 0 && a.descs) {
     SegDesc none;
@@ -350,43 +373,71 @@ __global__ void __launch_bounds__(kThreads, 1)
   ptx::tc_fence_after();
   const uint32_t tmem = sh->tmem_base;
   long long span_begin = 0, span_end = 0;
-  if (tid == 0) {
-    for (int r = 0; r < R; ++r) sh->row_prefix[r + 1] += sh->row_prefix[r];
+  if (warp == 0) {
+    if (lane == 0) {
+      for (int r = 0; r < R; ++r) sh->row_prefix[r + 1] += sh->row_prefix[r];
+    }
+    // shortest and longest unit: the first pair of the shortest row, the last pair of the longest
+    int c_lo = 0x7fffffff, c_hi = 0;
+    for (int r = lane; r < R; r += 32) c_lo = min(c_lo, sh->row_count[r]), c_hi = max(c_hi, sh->row_count[r]);
+    const int l_min = unit_iters(a, __reduce_min_sync(0xffffffffu, c_lo), 0);
+    const int l_max = unit_iters(a, __reduce_max_sync(0xffffffffu, c_hi), a.n_pairs - 1);
+    __syncwarp();
     const long long total = sh->row_prefix[R];
-    long long nc = gridDim.x;
     const long long c = blockIdx.x;
-    const long long n_units_all = static_cast<long long>(R) * a.n_pairs;
-    // Cutting units pays only when a unit is long: measured on B200, units of ~6 KV steps ran 2x
-    // slower cut (partials + the merge) than whole (45 vs 22 us), units of ~50 steps 20 % faster.
-    const bool cut = a.split && total >= n_units_all * kMinUnitStepsToCut &&
-                     (a.max_cut_steps <= 0 || total <= n_units_all * a.max_cut_steps);
+    const long long n_units = static_cast<long long>(R) * a.n_pairs;
+    // Cut or whole: compare what the longest-running CTA has to do, in KV steps.  (Dealing whole units out by their
+    // number gave the last CTAs of a causal first chunk twice the mean work: 8192 tokens, 32/8 heads, f16 1045 us,
+    // cut by this rule 667 us; 16 units of one KV head at 128K: 442 us whole, 91 us cut.)
+    // Cut: an equal share and the price of cutting.  A span costs a prologue, an epilogue and (when it cuts a
+    // unit) 128 KB of partials, about as much as kMinSpanSteps KV steps: with little work, fewer CTAs take
+    // longer spans and the others leave at once.
+    long long nc = gridDim.x;
+    const long long by_work = total / kMinSpanSteps;
+    const long long most = by_work > n_units ? by_work : n_units;
+    if (most < nc) nc = most;
+    const long long t_cut = total / nc + kCutCostSteps;
+    // Whole: the longest unit when every unit has a CTA; equal unit counts when units are about equally long;
+    // otherwise a share that ends up to a unit late.
+    const long long g = gridDim.x;
+    const long long t_whole = n_units <= g ? l_max
+                              : l_min * 10 >= l_max * 9 ? ((n_units + g - 1) / g) * l_max
+                                                        : total / g + l_max * 3 / 4;
+    // Long units: with every SM busy the board holds a lower clock, so a cut that gains little on paper loses
+    // (128 units of 1028 steps on 148 SMs, 2 ms per launch: 1923 us whole, 2028 us cut, 0.88 by this count;
+    // 128 units of 236 steps: 503 us whole, 450 us cut).
+    const bool cut = a.split && t_cut * 100 < t_whole * (total > n_units * 512 ? 85 : 100);
+    int row = 0, pair = 0;
+    long long acc = 0;
     if (cut) {
-      // A span costs a prologue, an epilogue and (when it cuts a unit) 128 KB of partials, about
-      // as much as kMinSpanSteps KV steps: with little work, fewer CTAs take longer spans and the
-      // others leave at once.
-      const long long by_work = total / kMinSpanSteps;
-      const long long cap = by_work > n_units_all ? by_work : n_units_all;
-      if (cap < nc) nc = cap;
       if (c < nc) {
         span_begin = total * c / nc;
         span_end = total * (c + 1) / nc;
       }
+    } else if (n_units <= g) {
+      // a unit of its own; its steps need no place among the others'
+      row = static_cast<int>(c / a.n_pairs), pair = static_cast<int>(c % a.n_pairs);
+      if (c < n_units) span_end = 1;
     } else {
-      // whole units only: equal unit counts per CTA
-      const long long nu = static_cast<long long>(R) * a.n_pairs;
-      auto unit_start = [&](long long u) -> long long {
-        if (u >= nu) return total;
-        const int r = static_cast<int>(u / a.n_pairs), p = static_cast<int>(u % a.n_pairs);
-        long long s = sh->row_prefix[r];
-        for (int q = 0; q < p; ++q) s += unit_iters(a, sh->row_count[r], q);
-        return s;
-      };
-      span_begin = unit_start(nu * c / nc);
-      span_end = unit_start(nu * (c + 1) / nc);
+      // the units that start inside an equal share of the steps
+      span_begin = total * c / g;
+      span_end = total * (c + 1) / g;
     }
-    sh->next_x = span_begin;
-    sh->more = span_end > span_begin ? 1 : 0;
-    sh->n_segs = 0;
+    if (span_end > span_begin && (cut || n_units > g)) {
+      locate_unit(a, sh, span_begin, R, lane, &row, &pair, &acc);
+      if (!cut && acc < span_begin) {
+        acc += unit_iters(a, sh->row_count[row], pair);
+        if (++pair == a.n_pairs) pair = 0, ++row;
+        span_begin = acc;
+      }
+    }
+    if (lane == 0) {
+      sh->cut = cut ? 1 : 0;
+      sh->cur_row = row, sh->cur_pair = pair, sh->cur_acc = acc;
+      sh->next_x = span_begin;
+      sh->more = span_end > span_begin && row < R ? 1 : 0;
+      sh->n_segs = 0;
+    }
   }
   __syncthreads();
 
@@ -396,7 +447,8 @@ __global__ void __launch_bounds__(kThreads, 1)
   // role state that lives across segments
   int ring_n = 0;        // ring entries issued (loader) / consumed (MMA)
   uint32_t it = 0;       // KV steps processed so far: parity of s_full / p_part
-  uint32_t seg_seq = 0;  // segments processed so far: parity of q_full / o_done / o_free
+  uint32_t seg_seq = 0;  // segments processed so far: parity of q_full / q_free / o_done / o_free
+  uint32_t q_issued = 0; // Q loads issued (loader)
   bool ok = true;
 
   // The producer warpgroup hands registers to the softmax warpgroups.  The pool is what the CTA got
@@ -415,22 +467,6 @@ __global__ void __launch_bounds__(kThreads, 1)
         for (int si = 0; si < n_segs && ok; ++si) {
           const Segment sg = sh->segs[si];
           const int b = sg.row / a.Hkv, hkv = sg.row % a.Hkv;
-          if (lane == 0) {
-            // Q smem is free once every MMA of the previous segment has completed
-            if (seg_seq > 0) ok = ptx::mbar_wait_bounded(ptx::smem_u32(&sh->o_done), (seg_seq - 1) & 1, abort_flag, limit);
-            if (ok) {
-              const uint32_t q_bytes = 2u * 128u * static_cast<uint32_t>(a.G * a.tpt);
-              for (int tile = 0; tile < 2; ++tile) {
-                const uint32_t bar = ptx::smem_u32(&sh->q_full[tile]);
-                ptx::mbar_expect_tx(bar, q_bytes);
-                for (int h = 0; h < 2; ++h) {
-                  ptx::tma_load_5d(q_smem + tile * kTileBytes + h * kHalfBytes, &q_map, bar, h * 64, 0, hkv,
-                                   (2 * sg.pair + tile) * a.tpt, b);
-                }
-              }
-            }
-          }
-          ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
           for (int base = 2 * sg.j0; base < 2 * sg.j1 && ok; base += 32) {
             // every lane resolves one sub-block of this batch of 32
             const int u = base + lane;
@@ -484,6 +520,23 @@ __global__ void __launch_bounds__(kThreads, 1)
                   for (int h = 0; h < 2; ++h) {
                     ptx::tma_load_4d(dst + h * kHalfBytes, map, bar, h * 64, c0[0], c0[1], c0[2]);
                     if (two) ptx::tma_load_4d(dst + h * kHalfBytes + kBoxBytes, map, bar, h * 64, c1[0], c1[1], c1[2]);
+                  }
+                  if (j == sg.j0 && kv == 0) {
+                    // Q follows the segment's first K tile: its memory is free once the last Q.K^T of the previous
+                    // segment has completed, while that segment's last softmax, P.V and epilogue still run
+                    if (seg_seq > 0) ok = ptx::mbar_wait_bounded(ptx::smem_u32(&sh->q_free), (seg_seq - 1) & 1, abort_flag, limit);
+                    if (ok) {
+                      const uint32_t q_bytes = 2u * 128u * static_cast<uint32_t>(a.G * a.tpt);
+                      for (int tile = 0; tile < 2; ++tile) {
+                        const uint32_t q_bar = ptx::smem_u32(&sh->q_full[tile]);
+                        ptx::mbar_expect_tx(q_bar, q_bytes);
+                        for (int h = 0; h < 2; ++h) {
+                          ptx::tma_load_5d(q_smem + tile * kTileBytes + h * kHalfBytes, &q_map, q_bar, h * 64, 0, hkv,
+                                           (2 * sg.pair + tile) * a.tpt, b);
+                        }
+                      }
+                      ++q_issued;
+                    }
                   }
                 }
               }
@@ -543,6 +596,7 @@ __global__ void __launch_bounds__(kThreads, 1)
               issue_s(1, slot);
               ptx::tc_commit(ptx::smem_u32(&sh->s_full[1]));
               ptx::tc_commit(ptx::smem_u32(&sh->ring_empty[slot]));
+              if (sg.j0 + 1 == sg.j1) ptx::tc_commit(ptx::smem_u32(&sh->q_free));
               ++ring_n;
             }
             for (int j = sg.j0; j < sg.j1 && ok; ++j, ++it) {
@@ -594,6 +648,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 issue_s(1, k_slot);
                 ptx::tc_commit(ptx::smem_u32(&sh->s_full[1]));
                 ptx::tc_commit(ptx::smem_u32(&sh->ring_empty[k_slot]));
+                if (j + 2 == sg.j1) ptx::tc_commit(ptx::smem_u32(&sh->q_free));
               }
             }
             if (ok) ptx::tc_commit(ptx::smem_u32(&sh->o_done));
@@ -609,7 +664,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
     while (true) {
-      if (tid == 0 && sh->more) plan_segments(a, sh, sh->next_x, span_begin, span_end, R);
+      if (tid == 0 && sh->more) plan_segments(a, sh, span_begin, span_end, R);
       else if (tid == 0) sh->n_segs = 0;
       __syncthreads();
       const int n_segs = sh->n_segs;
@@ -638,11 +693,13 @@ __global__ void __launch_bounds__(kThreads, 1)
             if (!ok) break;
             CA_PROF(1)
             ptx::tc_fence_after();
-            const bool masked = (2 * j + 1) >= sg.n_past_sub;  // a chunk or tail sub-block is in this step
+            bool masked = (2 * j + 1) >= sg.n_past_sub;  // a chunk or tail sub-block is in this step
             int lim0 = kSub, lim1 = kSub;
             if (masked) {
               lim0 = visible_cols(2 * j, sg.n_sub, sg.n_past_sub, t + a.q_off);
               lim1 = visible_cols(2 * j + 1, sg.n_sub, sg.n_past_sub, t + a.q_off);
+              // in a long chunk most of these steps lie wholly before the warp's rows (8192 x 8192: 667 -> 599 us)
+              masked = __any_sync(0xffffffffu, lim0 < kSub || lim1 < kSub);
             }
             // the whole S row (128 fp32) comes into registers with one wait
             uint32_t sv[128];
@@ -764,6 +821,10 @@ __global__ void __launch_bounds__(kThreads, 1)
       for (int e = (ring_n > kStages ? ring_n - kStages : 0); e < ring_n; ++e) {
         int dummy = 0;
         ptx::mbar_wait_bounded(ptx::smem_u32(&sh->ring_full[e % kStages]), (e / kStages) & 1, &dummy, 100000000ull);
+      }
+      for (int tile = 0; tile < 2 && q_issued > 0; ++tile) {
+        int dummy = 0;
+        ptx::mbar_wait_bounded(ptx::smem_u32(&sh->q_full[tile]), (q_issued - 1) & 1, &dummy, 100000000ull);
       }
     }
     if (warp == 8 && lane == 0) {
@@ -1108,24 +1169,12 @@ int ca_attn_compact(const ca_attn_params* p, ca_stream_t stream_) {
   // persistent grid: one CTA per SM, never more CTAs than units when units cannot be cut
   const long long n_units = static_cast<long long>(p->B) * p->Hkv * n_pairs;
   int grid = dev.sm_count;
-  // Cutting units costs partial traffic and a combine launch; it pays when whole units would leave SMs
-  // idle (few rows per rank under tensor parallelism, a nearly empty last wave) or unevenly loaded (the
-  // rows of a block table differ in length).  Measured on B200, 128 units on 148 SMs, 128K context:
-  // with ~460 selected blocks per row (236 KV steps per unit) whole units 503 us, cut 450 us in a short
-  // run and 516 vs 512 us in a seconds-long loop (the board then holds a lower clock with every SM busy);
-  // dense attention of the same shape (1028 steps per unit, 2 ms per launch) 1923 us whole, 2028 us cut.
-  // So a launch that already fills more than 80 % of a wave is cut only while its units are short.
-  // 16 units (one KV head of a tensor-parallel rank): 442 us whole, 91 us cut.
-  // (CA_ATTN_SPLIT_PERCENT overrides the 90 % threshold in development builds.)
-  const long long waves = (n_units + dev.sm_count - 1) / dev.sm_count;
-#ifdef CA_ATTN_SPLIT_PERCENT
-  const bool want_split = n_units * 100 < waves * dev.sm_count * CA_ATTN_SPLIT_PERCENT;
-#else
-  const bool want_split = n_units * 100 < waves * dev.sm_count * 90;
-#endif
-  a.max_cut_steps = n_units * 100 >= waves * dev.sm_count * 80 ? 512 : 0;
+  // Units may be cut across CTAs (the kernel decides, from the rows' counts) where the longest possible unit is
+  // longer than what cutting costs; below that the merge launch would only be in the way.
+  const int cap_blocks = p->block_idx && p->block_idx_stride < a.past_blocks ? p->block_idx_stride : a.past_blocks;
+  const long long longest = (static_cast<long long>(cap_blocks) * a.spb + (p->Q - 1 + a.q_off) / kSub + 2) / 2;
   const bool can_split = p->workspace != nullptr && p->workspace_bytes >= workspace_bytes_for(grid);
-  a.split = (want_split && can_split) ? 1 : 0;
+  a.split = (longest > kCutCostSteps && can_split) ? 1 : 0;
   if (!a.split && n_units < grid) grid = static_cast<int>(n_units);
   a.descs = nullptr, a.part_ml = nullptr, a.part_o = nullptr;
   if (a.split) {
