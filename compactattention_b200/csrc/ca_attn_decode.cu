@@ -1,7 +1,7 @@
 // Block-table attention for few query rows (decode): Q * G <= 16 rows per KV head.
 //
 // Bound by the bytes of K and V, so the design is about keeping copies in flight and the result on chip:
-// * the KV of one (batch, KV head) row is cut over the CTAs of a cluster (1..16) and, when rows are too few to
+// * the KV of one (batch, KV head) row is cut over the CTAs of a cluster (1..8) and, when rows are too few to
 //   fill the GPU even so, over several clusters;
 // * a CTA streams 64-token sub-blocks (K and V, 32 KB) through a three-stage TMA ring; two CTAs share an SM, so
 //   192 KB are in flight per SM;
@@ -13,8 +13,8 @@
 //   merged by a dependent launch.
 //
 // Measured on B200 (32/8 heads, bf16; through the 256-row kernel -> here): 8 sequences of 32768 tokens 253 -> 162 us
-// (1.07 GB, 6.64 TB/s), one of 131072 145 -> 106 us, one of 4001 31 -> 8.3 us; one KV head, 131072 tokens 184 -> 24 us;
-// 16 x 8192, 28/4 heads 81 -> 46 us.
+// (1.07 GB, 6.64 TB/s), one of 131072 145 -> 85 us, one of 4001 31 -> 8.3 us; one KV head, 131072 tokens 184 -> 19 us;
+// 16 x 8192, 28/4 heads 81 -> 45 us.
 #include "ca_attn_shared.cuh"
 
 #include <cooperative_groups.h>
@@ -34,9 +34,9 @@ constexpr int kThreads = (kWarps + 1) * 32;
 constexpr int kStages = 3;
 constexpr int kBoxBytes = kSub * 128;       // [64 tokens][64 channels]
 constexpr int kStageBytes = 4 * kBoxBytes;  // K low / high channels, V low / high channels
-constexpr int kMaxCluster = 16;
-constexpr int kMinSubs = 4;        // sub-blocks a CTA should have before its row is cut further
-constexpr int kMaxParts = 64;      // clusters a row may be cut over
+constexpr int kMaxCluster = 8;     // 16 leaves SMs without a place for one: 1 x 131072 tokens 106 us, 8 heads; with 8 85 us
+constexpr int kMinSubs = 2;        // sub-blocks a CTA of a cluster should have (1 x 1024: 5.9 us with 4, 5.1 with 2)
+constexpr int kMinSubsPart = 8;    // ... and of a row that is cut over several clusters, which costs the merge launch
 
 struct Args {
   const void* q;
@@ -440,7 +440,6 @@ static int launch(const Args& a, const CUtensorMap& k_map, const CUtensorMap& v_
     std::lock_guard<std::mutex> lock(mu);
     if (!done[ordinal]) {
       CA_CUDA(cudaFuncSetAttribute(attn_decode_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
-      CA_CUDA(cudaFuncSetAttribute(attn_decode_kernel<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
       done[ordinal] = true;
     }
   }
@@ -494,16 +493,17 @@ int launch_decode(const ca_attn_params* p, const DeviceInfo& dev, cudaStream_t s
   const int blocks = a.block_idx ? (a.block_idx_stride < a.past_blocks ? a.block_idx_stride : a.past_blocks) : a.past_blocks;
   const long long most = static_cast<long long>(blocks) * a.spb + (a.Q - 1 + a.q_off) / kSub + 1;  // sub-blocks of a row
   // A cluster as large as keeps every CTA resident and worth its prologue; rows too few for the GPU even then (one
-  // KV head of a tensor-parallel rank) are cut over several clusters, which costs the merge launch.
-  const int slots_on_gpu = 2 * dev.sm_count;
+  // KV head of a tensor-parallel rank) are cut over several clusters, which costs the merge launch.  Clusters sit
+  // inside a GPC, so not every SM can be part of one: 37 clusters of 8 (every slot of 148 SMs) run in two waves
+  // (131072 tokens of one head: 25 us), 32 in one (19 us).
+  const int places = 2 * dev.sm_count;
   int cs = 1;
-  while (cs < kMaxCluster && R * (2 * cs) <= slots_on_gpu && most >= static_cast<long long>(2 * cs) * kMinSubs) cs *= 2;
+  while (cs < kMaxCluster && R * (2 * cs) <= places && most >= static_cast<long long>(2 * cs) * kMinSubs) cs *= 2;
   a.parts = 1;
   if (cs == kMaxCluster) {
-    long long parts = slots_on_gpu / (R * cs);
-    const long long by_work = most / (cs * 2 * kMinSubs);
+    long long parts = places * 7 / 8 / (R * cs);
+    const long long by_work = most / (cs * kMinSubsPart);
     if (parts > by_work) parts = by_work;
-    if (parts > kMaxParts) parts = kMaxParts;
     const size_t per_part = static_cast<size_t>(R) * kRows * (kHeadDim * sizeof(float) + sizeof(float2));
     if (p->workspace != nullptr && parts > 1 && parts * per_part <= p->workspace_bytes) a.parts = static_cast<int>(parts);
   }
