@@ -7,7 +7,8 @@
 // Here the product is taken transposed, S^T = meanK_tile [128 key blocks x D] . Q^T [D x tokens], so
 // a key block is a TMEM lane: every thread of the epilogue owns one key block and reduces over its
 // own columns (tokens) without any shuffle.  The G query heads of a KV head share the meanK operand:
-// one CTA handles (batch, kv head, q-block), loads the q-block's tokens of all G heads once, and
+// a CTA handles (batch, kv head or a group of its query heads, q-block, share of the key-block tiles), loads the q-block's
+// tokens of its heads once, and
 // walks the visible key-block tiles with a 2-stage TMA ring and a double-buffered TMEM accumulator
 // (2 x 256 columns), so the MMAs of the next tile overlap the reductions of the current one.
 // One warp issues TMA and tcgen05.mma (lane 0); two warpgroups reduce, one per accumulator buffer,
@@ -16,6 +17,8 @@
 // contribute exp2(-inf) = 0 to the sum, so the sum needs no select), and uses packed fp32 pairs
 // for the scale and the sum.  Every wait is bounded.
 #include "ca_common.cuh"
+
+#include <mutex>
 
 namespace ca {
 namespace fpscore {
@@ -30,7 +33,9 @@ constexpr int kMaxCols = 256;       // tokens x heads per MMA pass (UMMA N)
 
 struct Args {
   int B, Q, Hq, Hkv, G, Kb, Qb, bs, P;
-  int heads_per_pass, passes;
+  int heads_per_pass;
+  int heads_per_cta, groups;  // query heads of a KV head that one CTA scores; CTAs that share a KV head's heads
+  int splits;                 // CTAs that share the visible key-block tiles
   float sm_scale;  // D^-0.5 * log2(e)
   float* score;    // [B,Qb,Kb,Hq]
   float* mx;
@@ -100,7 +105,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   const uint32_t smem_base = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem_aligned = smem_raw + (smem_base - ptx::smem_u32(smem_raw));
   // layout: K stage 0 | K stage 1 | Q half 0 [G*bs rows][64] | Q half 1 | barriers
-  const int q_rows = a.G * a.bs;
+  const int q_rows = a.heads_per_cta * a.bs;
   const uint32_t k_smem = smem_base;
   const uint32_t q_smem = smem_base + 2 * kKTileBytes;
   const uint32_t q_half_bytes = static_cast<uint32_t>(q_rows) * 128u;
@@ -108,7 +113,9 @@ __global__ void __launch_bounds__(kThreads, 1)
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int i = blockIdx.x;                       // q-block
-  const int hkv = blockIdx.y, b = blockIdx.z;
+  const int hkv = blockIdx.y / a.groups, b = blockIdx.z / a.splits, split = blockIdx.z % a.splits;
+  const int g0 = blockIdx.y % a.groups * a.heads_per_cta;  // first query head of the KV head's G
+  const int heads = min(a.heads_per_cta, a.G - g0);
   volatile int* abort_flag = &sh->abort_flag;
   const uint64_t limit = a.wait_limit_ns;
 
@@ -117,8 +124,11 @@ __global__ void __launch_bounds__(kThreads, 1)
   const long long last_abs = static_cast<long long>(a.P) + t_end - 1;
   int vis_blocks = static_cast<int>((last_abs + 1) / a.bs);
   if (vis_blocks > a.Kb) vis_blocks = a.Kb;
-  const int n_tiles = (vis_blocks + kTileKeys - 1) / kTileKeys;
-  const int n_work = n_tiles * a.passes;          // (tile, head pass) items, pass fastest
+  const int all_tiles = (vis_blocks + kTileKeys - 1) / kTileKeys;
+  const int tile0 = all_tiles * split / a.splits;
+  const int n_tiles = all_tiles * (split + 1) / a.splits - tile0;
+  const int passes = (heads + a.heads_per_pass - 1) / a.heads_per_pass;
+  const int n_work = n_tiles * passes;            // (tile, head pass) items, pass fastest
 
   if (tid == 0) {
     ptx::mbar_init(ptx::smem_u32(&sh->q_full), 1);
@@ -142,12 +152,12 @@ __global__ void __launch_bounds__(kThreads, 1)
   const uint32_t tmem = sh->tmem_base;
 
   // invisible key blocks keep the reference's -inf initialisation
-  {
-    float* sc = a.score + ((static_cast<long long>(b) * a.Qb + i) * a.Kb) * a.Hq + hkv * a.G;
-    float* mx = a.mx + ((static_cast<long long>(b) * a.Qb + i) * a.Kb) * a.Hq + hkv * a.G;
-    const int first = n_tiles * kTileKeys;
-    for (long long e = static_cast<long long>(first) * a.G + tid; e < static_cast<long long>(a.Kb) * a.G; e += kThreads) {
-      const long long j = e / a.G, g = e % a.G;
+  if (split == 0) {
+    float* sc = a.score + ((static_cast<long long>(b) * a.Qb + i) * a.Kb) * a.Hq + hkv * a.G + g0;
+    float* mx = a.mx + ((static_cast<long long>(b) * a.Qb + i) * a.Kb) * a.Hq + hkv * a.G + g0;
+    const int first = all_tiles * kTileKeys;
+    for (long long e = static_cast<long long>(first) * heads + tid; e < static_cast<long long>(a.Kb) * heads; e += kThreads) {
+      const long long j = e / heads, g = e % heads;
       sc[j * a.Hq + g] = -INFINITY;
       mx[j * a.Hq + g] = -INFINITY;
     }
@@ -162,25 +172,25 @@ __global__ void __launch_bounds__(kThreads, 1)
         return ok;
       };
       // the q-block's tokens of all G heads: one box per (head, d-half)
-      ptx::mbar_expect_tx(ptx::smem_u32(&sh->q_full), 2u * q_half_bytes);
-      for (int g = 0; g < a.G; ++g)
+      ptx::mbar_expect_tx(ptx::smem_u32(&sh->q_full), 2u * static_cast<uint32_t>(heads * a.bs) * 128u);
+      for (int g = 0; g < heads; ++g)
         for (int h = 0; h < 2; ++h)
           ptx::tma_load_4d(q_smem + h * q_half_bytes + g * a.bs * 128, &q_map, ptx::smem_u32(&sh->q_full), h * 64,
-                           hkv * a.G + g, i * a.bs, b);
+                           hkv * a.G + g0 + g, i * a.bs, b);
       auto load_k = [&](int tile) {
         const int s = tile & 1;
         if (tile >= 2 && !wait(&sh->k_empty[s], ((tile >> 1) - 1) & 1)) return;
         ptx::mbar_expect_tx(ptx::smem_u32(&sh->k_full[s]), kKTileBytes);
         for (int h = 0; h < 2; ++h)
           ptx::tma_load_4d(k_smem + s * kKTileBytes + h * kHalfBytesK, &k_map, ptx::smem_u32(&sh->k_full[s]), h * 64, hkv,
-                           tile * kTileKeys, b);
+                           (tile0 + tile) * kTileKeys, b);
       };
       load_k(0);
       wait(&sh->q_full, 0);
       const uint64_t k_desc0 = ptx::make_smem_desc_sw128(k_smem, 0, 1024);
       const uint64_t q_desc0 = ptx::make_smem_desc_sw128(q_smem, 0, 1024);
       for (int w = 0; w < n_work && ok; ++w) {
-        const int tile = w / a.passes, pass = w % a.passes;
+        const int tile = w / passes, pass = w % passes;
         const int s = tile & 1, buf = w & 1;
         if (pass == 0) {
           if (tile + 1 < n_tiles) load_k(tile + 1);  // prefetch the next key tile
@@ -189,7 +199,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (w >= 2 && !wait(&sh->t_empty[buf], ((w >> 1) - 1) & 1)) break;
         ptx::tc_fence_after();
         const int h0 = pass * a.heads_per_pass;
-        const int nh = min(a.heads_per_pass, a.G - h0);
+        const int nh = min(a.heads_per_pass, heads - h0);
         const uint32_t idesc = a.idesc_base | (static_cast<uint32_t>((nh * a.bs) >> 3) << 17);
         const uint64_t kd = k_desc0 + static_cast<uint64_t>(s * (kKTileBytes >> 4));
         const uint64_t qd = q_desc0 + static_cast<uint64_t>((h0 * a.bs * 128) >> 4);
@@ -201,7 +211,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           ptx::mma_ss(tmem + buf * kMaxCols, kd + ko, qd + qo, idesc, k > 0 ? 1u : 0u);
         }
         ptx::tc_commit(ptx::smem_u32(&sh->t_full[buf]));
-        if (pass == a.passes - 1) ptx::tc_commit(ptx::smem_u32(&sh->k_empty[s]));
+        if (pass == passes - 1) ptx::tc_commit(ptx::smem_u32(&sh->k_empty[s]));
       }
     }
   } else {
@@ -212,15 +222,15 @@ __global__ void __launch_bounds__(kThreads, 1)
     const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
     const int c_max = t_end - i * a.bs;  // one past the last real token of the q-block
     for (int w = wg; w < n_work; w += 2) {
-      const int tile = w / a.passes, pass = w % a.passes;
+      const int tile = w / passes, pass = w % passes;
       const int buf = wg;
       ok = ptx::mbar_wait_bounded(ptx::smem_u32(&sh->t_full[buf]), (w >> 1) & 1, abort_flag, limit);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       ptx::tc_fence_after();
-      const int j = tile * kTileKeys + row;  // this thread's key block
+      const int j = (tile0 + tile) * kTileKeys + row;  // this thread's key block
       const int h0 = pass * a.heads_per_pass;
-      const int nh = min(a.heads_per_pass, a.G - h0);
+      const int nh = min(a.heads_per_pass, heads - h0);
       // token t of the q-block is counted iff P + t >= (j+1)*bs - 1  <=>  t >= (j+1)*bs - 1 - P
       const long long t_min_ll = static_cast<long long>(j + 1) * a.bs - 1 - a.P - static_cast<long long>(i) * a.bs;
       const int c_min = t_min_ll < 0 ? 0 : (t_min_ll > a.bs ? a.bs : static_cast<int>(t_min_ll));  // first counted column
@@ -238,7 +248,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       ptx::tc_fence_before();
       ptx::mbar_arrive(ptx::smem_u32(&sh->t_empty[buf]));
       if (j < a.Kb) {
-        const long long o = ((static_cast<long long>(b) * a.Qb + i) * a.Kb + j) * a.Hq + hkv * a.G + h0;
+        const long long o = ((static_cast<long long>(b) * a.Qb + i) * a.Kb + j) * a.Hq + hkv * a.G + g0 + h0;
         if (nh == 4 && (o & 3) == 0) {
           *reinterpret_cast<float4*>(a.score + o) = make_float4(res_p[0], res_p[1], res_p[2], res_p[3]);
           *reinterpret_cast<float4*>(a.mx + o) = make_float4(res_m[0], res_m[1], res_m[2], res_m[3]);
@@ -280,11 +290,28 @@ int launch_fp_score_sm100(const ca_flashprefill_score_params* p, cudaStream_t st
   if (p->D != kD || (bs != 64 && bs != 128) || p->q_dtype != p->k_dtype ||
       (p->q_dtype != CA_DTYPE_BF16 && p->q_dtype != CA_DTYPE_F16))
     return CA_ERR_UNSUPPORTED;
-  const size_t smem = 2 * kKTileBytes + 2 * static_cast<size_t>(G) * bs * 128 + 1024 + sizeof(Shared);
   DeviceInfo dev;
   int rc = get_device_info(&dev);
   if (rc != CA_OK) return rc;
-  if (dev.cc_major != 10 || smem > static_cast<size_t>(dev.smem_optin)) return CA_ERR_UNSUPPORTED;
+  if (dev.cc_major != 10) return CA_ERR_UNSUPPORTED;
+  // A CTA holds the q-block of as many of the KV head's query heads as fit beside the key tiles, in whole MMA
+  // passes: they share the key tiles it loads.  A chunk of few q-blocks leaves SMs idle that way (8 q-blocks of 128
+  // x 8 KV heads = 64 CTAs), so below one CTA per SM every pass gets a CTA of its own and then the key tiles are shared out.
+  // us before -> after: 28/4 heads, block 128 (all seven heads of a group did not fit: the CUDA-core kernel) 1024 of
+  // 64K 330 -> 17.5, 8192 of 64K 2517 -> 70; 256 of 128K, 8/2 heads, block 64 34 -> 17; 1024 of 32K, block 128 18.9 -> 16.8.
+  const int per_pass = kMaxCols / bs;
+  auto smem_of = [&](int heads) { return 2 * kKTileBytes + 2 * static_cast<size_t>(heads) * bs * 128 + 1024 + sizeof(Shared); };
+  int heads = ceil_div(G, per_pass) * per_pass;
+  while (heads > per_pass && smem_of(heads < G ? heads : G) > static_cast<size_t>(dev.smem_optin)) heads -= per_pass;
+  const long long q_ctas = static_cast<long long>(ceil_div(p->Q, bs)) * p->Hkv * p->B;
+  if (q_ctas * ceil_div(G, heads) < dev.sm_count) heads = per_pass;
+  if (heads > G) heads = G;
+  const int groups = ceil_div(G, heads);
+  const size_t smem = smem_of(heads);
+  if (smem > static_cast<size_t>(dev.smem_optin)) return CA_ERR_UNSUPPORTED;
+  long long splits = dev.sm_count / (q_ctas * groups);
+  if (splits > ceil_div(p->Kb, kTileKeys)) splits = ceil_div(p->Kb, kTileKeys);
+  if (splits < 1) splits = 1;
   if ((p->q_stride_b | p->q_stride_t | p->q_stride_h | p->k_stride_b | p->k_stride_blk | p->k_stride_h) % 8 != 0 ||
       (reinterpret_cast<uintptr_t>(p->q) | reinterpret_cast<uintptr_t>(p->mean_k)) % 16 != 0)
     return CA_ERR_UNSUPPORTED;
@@ -315,15 +342,24 @@ int launch_fp_score_sm100(const ca_flashprefill_score_params* p, cudaStream_t st
   a.B = p->B, a.Q = p->Q, a.Hq = p->Hq, a.Hkv = p->Hkv, a.G = G, a.Kb = p->Kb, a.bs = bs;
   a.Qb = ceil_div(p->Q, bs);
   a.P = p->kv_len - p->Q;
-  a.heads_per_pass = kMaxCols / bs;
-  a.passes = ceil_div(G, a.heads_per_pass);
+  a.heads_per_pass = per_pass;
+  a.heads_per_cta = heads, a.groups = groups, a.splits = static_cast<int>(splits);
   a.sm_scale = (1.0f / sqrtf(static_cast<float>(kD))) * 1.4426950408889634f;
   a.score = p->score_raw, a.mx = p->max_raw;
   a.idesc_base = ptx::make_idesc_f16(p->q_dtype == CA_DTYPE_BF16 ? 1u : 0u, kTileKeys, 0, 0, 0);
   a.wait_limit_ns = 2000000000ull;
   a.status = nullptr;
-  CA_CUDA(cudaFuncSetAttribute(fp_score_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-  launch_kernel_as(true, fp_score_kernel, dim3(a.Qb, p->Hkv, p->B), dim3(kThreads), smem, stream, q_map, k_map, a);
+  {
+    // the opt-in shared-memory size is a per-device function attribute: set once per device, to all there is
+    static std::mutex mu;
+    static bool done[64] = {};
+    std::lock_guard<std::mutex> lock(mu);
+    if (!done[dev.ordinal]) {
+      CA_CUDA(cudaFuncSetAttribute(fp_score_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, dev.smem_optin));
+      done[dev.ordinal] = true;
+    }
+  }
+  launch_kernel_as(true, fp_score_kernel, dim3(a.Qb, p->Hkv * groups, p->B * a.splits), dim3(kThreads), smem, stream, q_map, k_map, a);
   CA_LAUNCH_CHECK("fp_score_kernel");
   return CA_OK;
 }
