@@ -176,6 +176,22 @@ def _kv_view(key_states, value_states, k_hf, v_hf) -> ops.KvCacheView:
     return ops.KvCacheView.from_seq_first(key_states.contiguous(), value_states.contiguous())
 
 
+def _select_and_attend(query_states, key_states, value_states, k_hf, v_hf, attention_mask, kv_len, num_kv_heads, num_key_value_groups,
+                       block_size, softmax_scale, keep_recent, rule: dict) -> torch.Tensor:
+    """Row rule (the arguments of ``ops.select_rows``), union and table in one launch, then attention: what
+    ``..._from_keep_block`` does for one table row per KV head, without the packed bits and the statistics."""
+    if query_states.shape[2] != num_kv_heads * num_key_value_groups:
+        raise ValueError("num_key_value_groups does not match the head counts")
+    _check_attention_mask(attention_mask, kv_len)
+    table = ops.select_union_table(num_kv_heads=num_kv_heads, block_size=block_size, keep_recent=keep_recent, **rule)
+    return ops.attn_compact(query_states, _kv_view(key_states, value_states, k_hf, v_hf), kv_len, num_kv_heads, table.block_idx,
+                            table.counts, block_size=block_size, softmax_scale=softmax_scale)
+
+
+# Routes with several table rows per KV head; they go through ..._from_keep_block.
+_SUB_HEAD_IMPLS = ("fi_zero_copy_per_query", "fi_zero_copy_subgroup")
+
+
 def chunked_prefill_column_dense_attention_from_keep_block(
     query_states: torch.Tensor,  # [B, Q, Hq, D]
     key_states: torch.Tensor,  # [B, K, Hkv, D]
@@ -362,11 +378,13 @@ def chunked_prefill_column_dense_attention_forward(
         # nonzero = visible, the conversion the reference's mask builder applies (:372)
         valid = block_attention_mask[..., -q_blocks:, -score_blocks:].to(torch.bool)
 
-    def _select():
-        return ops.select_rows(attn_gate_score, past_blocks - missing, "threshold", valid=valid,
-                               threshold=threshold if isinstance(threshold, torch.Tensor) else float(threshold))
+    rule = dict(score=attn_gate_score, past_blocks=past_blocks - missing, rule="threshold", valid=valid,
+                threshold=threshold if isinstance(threshold, torch.Tensor) else float(threshold))
+    if not timing and not missing and indexed_impl not in _SUB_HEAD_IMPLS:
+        return _select_and_attend(query_states, key_states, value_states, k_hf, v_hf, attention_mask, kv_len, num_kv_heads,
+                                  num_key_value_groups, block_size, softmax_scale, max(int(keep_recent_blocks), 0), rule), None
 
-    bits, select_ms = _timed(_select, timing)
+    bits, select_ms = _timed(lambda: ops.select_rows(**rule), timing)
     if missing:
         # left-pad the packed columns with `missing` never-selected blocks
         full = ops.unpack_bits(bits, score_blocks)

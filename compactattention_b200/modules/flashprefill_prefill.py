@@ -15,6 +15,8 @@ import torch
 
 from .. import ops
 from .attention_forward_chunked_dense import (
+    _SUB_HEAD_IMPLS,
+    _select_and_attend,
     COMPACTATTN_VERSION,
     _check_common,
     _kv_dims,
@@ -87,12 +89,14 @@ def flashprefill_compactattn_prefill_full_kv(
     (score, score_max), select_ms = _timed(_score, measure_timing)
     tail = min(max(int(last_n_block), 0), q_blocks - 1) if q_blocks > 1 else 0
 
-    def _rule():
-        return ops.select_rows(score.permute(0, 3, 1, 2), past_blocks, "alpha_rowmax", alpha=float(alpha),
-                               sink=int(attention_sink), local=int(window_size), min_budget=int(min_budget),
-                               rows_voting=max(q_blocks - tail, 1), score_max=score_max.permute(0, 3, 1, 2))
+    rule = dict(score=score.permute(0, 3, 1, 2), past_blocks=past_blocks, rule="alpha_rowmax", alpha=float(alpha),
+                sink=int(attention_sink), local=int(window_size), min_budget=int(min_budget),
+                rows_voting=max(q_blocks - tail, 1), score_max=score_max.permute(0, 3, 1, 2))
+    if not measure_timing and indexed_impl not in _SUB_HEAD_IMPLS:
+        return _select_and_attend(query_states, key_states, value_states, k_hf, v_hf, attention_mask, kv_len, num_kv_heads,
+                                  num_key_value_groups, block_size, softmax_scale, 0, rule), {}
 
-    bits, union_ms = _timed(_rule, measure_timing)
+    bits, union_ms = _timed(lambda: ops.select_rows(**rule), measure_timing)
     out, compact_stats = chunked_prefill_column_dense_attention_from_keep_block(
         query_states, key_states, value_states, keep_block=None, attention_mask=attention_mask, query_length=q_len,
         softmax_scale=softmax_scale, block_size=block_size, num_key_value_groups=num_key_value_groups, pack_impl=pack_impl,
