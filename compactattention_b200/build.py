@@ -24,6 +24,9 @@ PKG_DIR = Path(__file__).resolve().parent
 CSRC = PKG_DIR / "csrc"
 LIB_PATH = PKG_DIR / "libcompactattn_b200.so"
 STAMP_PATH = PKG_DIR / "libcompactattn_b200.so.stamp"
+CALLS_SOURCE = PKG_DIR / "binding" / "calls.cpp"
+CALLS_PATH = PKG_DIR / "_calls.so"
+CALLS_STAMP_PATH = PKG_DIR / "_calls.so.stamp"
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -73,6 +76,32 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     return LIB_PATH
 
 
+def build_calls(force: bool = False) -> Path:
+    """Compile the native form of the tensor-level wrappers (``binding/calls.cpp``) for this Python and torch."""
+    import sysconfig
+
+    import torch
+
+    h = hashlib.sha256()
+    for f in (CALLS_SOURCE, PKG_DIR.parent / "include" / "compactattn_b200.h"):
+        h.update(f.read_bytes())
+    h.update(f"{torch.__version__} {sys.version}".encode())
+    fp = h.hexdigest()
+    if not force and CALLS_PATH.exists() and CALLS_STAMP_PATH.exists() and CALLS_STAMP_PATH.read_text().strip() == fp:
+        return CALLS_PATH
+    root = Path(torch.__file__).resolve().parent
+    cmd = [shutil.which("g++") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f"-I{root / 'include'}",
+           f"-I{root / 'include' / 'torch' / 'csrc' / 'api' / 'include'}", f"-I{sysconfig.get_paths()['include']}",
+           "-o", str(CALLS_PATH), str(CALLS_SOURCE), f"-L{root / 'lib'}", "-ltorch_python", "-ltorch_cpu", "-lc10"]
+    proc = subprocess.run(cmd, capture_output=True, text=True)
+    if proc.returncode != 0:
+        sys.stderr.write(proc.stdout + proc.stderr)
+        raise RuntimeError(f"g++ failed with exit code {proc.returncode}")
+    CALLS_STAMP_PATH.write_text(fp + "\n")
+    return CALLS_PATH
+
+
 def build_variant(defines: list[str], output: Path, verbose: bool = False) -> Path:
     """Compile the same sources with extra ``-D`` macros into ``output`` (a development build)."""
     output = Path(output).resolve()
@@ -103,6 +132,7 @@ def main() -> None:
         print(build_variant(args.define, Path(args.output), verbose=args.verbose))
     else:
         print(build(force=args.force, verbose=args.verbose))
+        print(build_calls(force=args.force))
 
 
 if __name__ == "__main__":

@@ -13,6 +13,11 @@ import torch
 
 from . import _lib
 
+try:  # the native form of the wrappers below (binding/calls.cpp); everything works without it, only slower to enqueue
+    from . import _calls
+except ImportError:
+    _calls = None
+
 _DTYPES = {torch.bfloat16: _lib.CA_DTYPE_BF16, torch.float16: _lib.CA_DTYPE_F16, torch.float32: _lib.CA_DTYPE_F32}
 
 
@@ -30,6 +35,24 @@ def _stream() -> int:
     if _raw_stream is not None:
         return _raw_stream(torch.cuda.current_device())
     return torch.cuda.current_stream().cuda_stream
+
+
+_NATIVE_CALLS = ("ca_attn_compact", "ca_rope_append", "ca_gate_prepare", "ca_select_union_table", "ca_gate_score_select",
+                 "ca_select_union_scratch_bytes")
+_native_lib = None  # the loaded library whose entry points _calls holds
+
+
+def _native():
+    """The native wrappers, or None (not built, or the calls are being recorded).  Each of them answers None to
+    anything but the plain, valid case, which the Python form then serves or refuses."""
+    global _native_lib
+    if _calls is None or _lib._recording is not None:
+        return None
+    lib = _lib.load()
+    if lib is not _native_lib:
+        _calls.bind(*(C.cast(getattr(lib._cdll, name), C.c_void_p).value for name in _NATIVE_CALLS))
+        _native_lib = lib
+    return _calls
 
 
 def _require_cuda(*tensors: Optional[torch.Tensor]) -> None:
@@ -146,6 +169,16 @@ def attn_compact(
     With a workspace (default: a cached per-stream buffer) the kernel may cut work units across SMs
     and merge the pieces; ``use_workspace=False`` keeps every unit on one SM."""
     _require_cuda(q, kv.k, kv.v, block_idx, counts, out, lse, status)
+    native = _native() if use_workspace else None
+    if native is not None:
+        stream = _stream()
+        ws = _ATTN_WORKSPACES.get((q.device.index, stream)) if workspace is None else workspace
+        if ws is not None:
+            done = native.attn_compact(stream, ws, q, kv.k, kv.v, kv.page_stride, kv.token_stride, kv.head_stride, kv.page_size,
+                                       kv.num_pages, kv.pages_per_seq, kv.head_div, kv.page_table, kv_len, num_kv_heads, block_idx,
+                                       counts, block_size, softmax_scale, out, lse, status)
+            if done is not None:
+                return done
     B, Q, Hq, D = q.shape
     if q.dtype not in (torch.bfloat16, torch.float16) or kv.k.dtype != q.dtype or kv.v.dtype != q.dtype:
         raise ValueError("q, k, v must share dtype bfloat16 or float16")
@@ -370,7 +403,7 @@ def select_union_table(
     out: Optional["BlockTable"] = None,
     scratch: Optional[torch.Tensor] = None,
     score_max: Optional[torch.Tensor] = None,  # as in select_rows
-    _gate=None,  # (GateScoreParams writing `score`, write_scores): set by gate_score_select
+    _gate=None,  # set by gate_score_select: (makes the GateScoreParams that write `score`, write_scores, native arguments)
 ) -> "BlockTable":
     """``select_rows`` followed by ``union_table`` in ONE launch (see ``ca_select_union_table``): row rule,
     Q-block union, GQA union and the per-KV-head block table.  ``scratch`` must be zero on first use and
@@ -380,6 +413,22 @@ def select_union_table(
         raise ValueError(f"{H} score heads is not a multiple of {num_kv_heads} kv heads")
     if Kb - past_blocks != Qb:
         raise ValueError("the score must cover the chunk's own key blocks: Kb - past_blocks must equal Qb")
+    native = None
+    if bits is None and prob_out is None and rule != "mask" and not isinstance(threshold, torch.Tensor):
+        _require_cuda(score, valid)
+        native = _native()
+    if native is not None:
+        stream = _stream()
+        words = _UNION_SCRATCH.get((score.device.index, stream, B * num_kv_heads)) if scratch is None else scratch
+        if words is not None:
+            num, den = topk_ratio if topk_ratio is not None else (0, 1)
+            given = (None,) * 4 if out is None else (out.block_idx, out.counts, out.cache_seqlens, out.pages_per_row)
+            gate = () if _gate is None else (*_gate[2], 1 if _gate[1] else 0)
+            done = native.select_union_table(stream, words, score, past_blocks, RULES[rule], num_kv_heads, block_size, page_size,
+                                             int(keep_recent), valid, int(softmax), float(threshold), float(alpha), int(topk_k), num, den,
+                                             int(min_budget), int(sink), int(local), int(rows_voting), score_max, *given, *gate)
+            if done is not None:
+                return BlockTable(*done) if out is None else out
     p, bits, keep = _select_params(score, past_blocks, rule, valid, softmax, threshold, alpha, topk_k, topk_ratio, min_budget,
                                    sink, local, rows_voting, bits, prob_out, bits_required=False, score_max=score_max)
     dev = score.device
@@ -404,7 +453,7 @@ def select_union_table(
     if scratch.dtype != torch.int32 or not scratch.is_contiguous():
         raise ValueError("scratch must be a contiguous int32 tensor (zero on first use)")
     if _gate is not None:
-        _lib.check(_lib.load().ca_gate_score_select(C.byref(_gate[0]), C.byref(p), C.byref(u), scratch.data_ptr(), scratch.numel() * 4,
+        _lib.check(_lib.load().ca_gate_score_select(C.byref(_gate[0]()), C.byref(p), C.byref(u), scratch.data_ptr(), scratch.numel() * 4,
                                                     1 if _gate[1] else 0, _stream()), "ca_gate_score_select")
     else:
         _lib.check(_lib.load().ca_select_union_table(C.byref(p), C.byref(u), scratch.data_ptr(), scratch.numel() * 4, _stream()),
@@ -620,6 +669,16 @@ def gate_prepare(
 ) -> None:
     """Pool + project + RoPE the chunk's Q and K blocks and append the K blocks, in one launch."""
     _require_cuda(q, k, wq, wk, q_out, k_out)
+    native = _native()
+    if native is not None:
+        q_bits = k_bits = 0
+        for kind in q_kinds:
+            q_bits |= _POOL_BITS[kind]
+        for kind in k_kinds:
+            k_bits |= _POOL_BITS[kind]
+        if native.gate_prepare(_stream(), block_size, q, q_bits, wq, *(rope_q or (None, None)), q_out, 0,
+                               k, k_bits, wk, *(rope_k or (None, None)), k_out, k_out_block_offset):
+            return
     B, L, _, D = q.shape
     if k.shape[0] != B or k.shape[1] != L or k.shape[3] != D:
         raise ValueError("q and k chunks must share batch, length and head dim")
@@ -685,8 +744,14 @@ def gate_score_select(
     score kernel, then the rule + Block-Union + table kernel.  ``scores`` always receives the logits
     (``write_scores`` is kept for callers of an earlier single-launch form and ignored).  ``select_kwargs`` are
     those of ``select_union_table``."""
-    g, scores = _gate_score_params(q_blocks, k_blocks, past_blocks, scale, masked_value, scores)
-    return select_union_table(scores, past_blocks, rule, num_kv_heads=num_kv_heads, _gate=(g, bool(write_scores)), **select_kwargs)
+    _require_cuda(q_blocks, k_blocks, scores)
+    if scores is None:
+        scores = torch.empty((q_blocks.shape[0], q_blocks.shape[2], q_blocks.shape[1], k_blocks.shape[1]), dtype=torch.float32,
+                             device=q_blocks.device)
+    scale = float(scale) if scale is not None else q_blocks.shape[3] ** -0.5
+    gate = (lambda: _gate_score_params(q_blocks, k_blocks, past_blocks, scale, masked_value, scores)[0], bool(write_scores),
+            (q_blocks, k_blocks, scale, masked_value))
+    return select_union_table(scores, past_blocks, rule, num_kv_heads=num_kv_heads, _gate=gate, **select_kwargs)
 
 
 def flashprefill_score(
@@ -772,6 +837,13 @@ def rope_append(
     """One launch for a chunk: RoPE(q) -> q_out, RoPE(k) -> cache pages (+ per-block mean -> mean_k),
     v -> cache pages.  Returns q_out (allocated when q is given and q_out is not)."""
     _require_cuda(q, k, v, cos, sin, cache.k, cache.v, mean_k, q_out, status)
+    native = _native() if q is not None else None
+    if native is not None:
+        done = native.rope_append(_stream(), q, k, v, cos, sin, cache.k, cache.v, cache.page_stride, cache.token_stride,
+                                  cache.head_stride, cache.page_size, cache.num_pages, cache.pages_per_seq, cache.head_div,
+                                  cache.page_table, position, mean_k, block_size, q_out, status)
+        if done is not None:
+            return done
     if k.dim() != 4 or v.shape != k.shape or k.dtype != v.dtype or k.dtype not in (torch.bfloat16, torch.float16):
         raise ValueError("k and v must be [B, Q, Hkv, D] of one 16-bit dtype")
     B, Q, Hkv, D = k.shape

@@ -1,0 +1,144 @@
+"""The native form of the tensor wrappers (``binding/calls.cpp``) against their Python form: the same results bit for
+bit over the options that both take, and the same errors."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from compactattention_b200 import ops as _ops
+    assert _ops._calls is not None, "the native wrappers are not built (python -m compactattention_b200.build)"
+    return _ops
+
+
+def _both(ops, monkeypatch, fn):
+    """``fn()`` through Python and then through the native form, which must have served it."""
+    with monkeypatch.context() as m:
+        m.setattr(ops, "_calls", None)
+        python = fn()
+    fn()  # what the wrappers keep per stream exists from here on
+    seen, real = [], ops._calls
+
+    class Watch:
+        def __getattr__(self, name):
+            def call(*args):
+                out = getattr(real, name)(*args)
+                seen.append((name, out is not None))
+                return out
+            return call
+
+    with monkeypatch.context() as m:
+        m.setattr(ops, "_calls", Watch())
+        native = fn()
+    assert any(served for _, served in seen), seen
+    return python, native
+
+
+def _randn(*shape, dtype=torch.bfloat16, seed=0):
+    return torch.randn(shape, generator=torch.Generator(device="cuda").manual_seed(seed), device="cuda", dtype=torch.float32).to(dtype)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("Q", [1, 130])
+def test_attention(ops, monkeypatch, dtype, Q):
+    B, K, Hq, Hkv, bs = 2, 64 * 9 + Q, 8, 2, 64
+    q, k, v = _randn(B, Q, Hq, 128, dtype=dtype), _randn(B, K, Hkv, 128, dtype=dtype, seed=1), _randn(B, K, Hkv, 128, dtype=dtype, seed=2)
+    kv = ops.KvCacheView.from_seq_first(k, v)
+    idx = torch.arange(9, dtype=torch.int32, device="cuda").repeat(B, Hkv, 1).contiguous()
+    counts = torch.tensor([[9, 4], [1, 0]], dtype=torch.int32, device="cuda")
+    out = torch.empty((B, Q, Hq, 136), dtype=dtype, device="cuda")[..., :128]
+    for kw in ({}, {"softmax_scale": 0.05}, {"out": out}):
+        a, b = _both(ops, monkeypatch, lambda: ops.attn_compact(q, kv, K, Hkv, idx, counts, block_size=bs, **kw).clone())
+        assert torch.equal(a, b)
+        a, b = _both(ops, monkeypatch, lambda: ops.attn_compact(q, kv, K, Hkv, None, None, block_size=bs, **kw).clone())
+        assert torch.equal(a, b)
+    assert ops.attn_compact(q, kv, K, Hkv, None, None, out=out) is out
+    with pytest.raises(ValueError, match="share dtype"):
+        ops.attn_compact(q.float(), kv, K, Hkv, None, None)
+    with pytest.raises(ValueError, match="one row per"):
+        ops.attn_compact(q, kv, K, Hkv, idx[:1].contiguous(), counts)
+    with pytest.raises(RuntimeError, match="kv_len"):
+        ops.attn_compact(q, kv, Q - 1, Hkv, None, None)
+
+
+@pytest.mark.parametrize("tables", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("mean", [True, False])
+def test_append(ops, monkeypatch, tables, mean):
+    from compactattention_b200.paged_cache import PagedKVCache
+    B, Q, Hq, Hkv, pos = 2, 200, 7, 3, 128
+    q, k, v = _randn(B, Q, Hq, 128), _randn(B, Q, Hkv, 128, seed=1), _randn(B, Q, Hkv, 128, seed=2)
+    cos, sin = _randn(1, Q, 128, dtype=tables, seed=3), _randn(1, Q, 128, dtype=tables, seed=4)
+
+    def run():
+        cache = PagedKVCache(B, 512, Hkv, 128, torch.device("cuda"))
+        mean_k = torch.zeros((B, 8, Hkv, 128), dtype=torch.bfloat16, device="cuda") if mean else None
+        rot, n = cache.append_rope(q, k, v, cos, sin, position=pos, mean_k=mean_k)
+        assert n == pos + Q
+        return [rot, cache.k_pages, cache.v_pages] + ([mean_k] if mean else [])
+
+    a, b = _both(ops, monkeypatch, run)
+    assert all(torch.equal(x, y) for x, y in zip(a, b))
+    cache = PagedKVCache(B, 512, Hkv, 128, torch.device("cuda"))
+    with pytest.raises(ValueError, match="do not fit in mean_k"):
+        ops.rope_append(q, k, v, cos, sin, cache.view(), 128, mean_k=torch.zeros((B, 2, Hkv, 128), dtype=torch.bfloat16, device="cuda"))
+    with pytest.raises(ValueError, match="share their strides"):
+        ops.rope_append(q, k, v, cos, sin.repeat(1, 1, 2)[..., :128], cache.view(), 0)
+
+
+@pytest.mark.parametrize("rule,kw", [
+    ("threshold", dict(threshold=0.2)),
+    ("threshold", dict(threshold=0.001, softmax=True, keep_recent=3)),
+    ("topk", dict(topk_ratio=(1, 5), sink=1, local=2)),
+    ("topk", dict(topk_k=3)),
+    ("alpha_rowmax", dict(alpha=0.5, sink=2, local=4, min_budget=5, rows_voting=2)),
+    ("cummass", dict(threshold=0.6, softmax=True)),
+])
+@pytest.mark.parametrize("masked", [False, True])
+def test_selection(ops, monkeypatch, rule, kw, masked):
+    B, H, Hkv, Qb, Kb = 2, 6, 3, 4, 70
+    score = _randn(B, Qb, Kb, H, dtype=torch.float32).permute(0, 3, 1, 2)  # strided, as the training-free score is
+    valid = None
+    if masked:
+        valid = torch.ones((Qb, Kb), dtype=torch.bool, device="cuda").tril(Kb - Qb).view(1, 1, Qb, Kb)
+        valid[..., 5] = False
+
+    def run():
+        t = ops.select_union_table(score, Kb - Qb, rule, num_kv_heads=Hkv, valid=valid, **kw)
+        return [t.block_idx, t.counts, t.cache_seqlens, t.pages_per_row]
+
+    a, b = _both(ops, monkeypatch, run)
+    assert all(torch.equal(x, y) and x.shape == y.shape for x, y in zip(a, b))
+    with pytest.raises(ValueError, match="own key blocks"):
+        ops.select_union_table(score, Kb - Qb - 1, rule, num_kv_heads=Hkv, **kw)
+    with pytest.raises(ValueError, match="not a multiple"):
+        ops.select_union_table(score, Kb - Qb, rule, num_kv_heads=4, **kw)
+
+
+@pytest.mark.parametrize("rope", [True, False])
+def test_gate(ops, monkeypatch, rope):
+    from compactattention_b200.chunk_driver import GateSelectorState, SelectionRule
+    from compactattention_b200.prefill_sparse.attn_gate import ATTNGATE_CLASSES
+    Hq, Hkv, L, past = 8, 2, 300, 40
+    gate = ATTNGATE_CLASSES["Qavg_Kmaxminavg"](64, 128, 128, Hkv, Hq, force_double=True).cuda().to(torch.bfloat16)
+    with torch.no_grad():
+        gate.mask_linear_q.weight.copy_(_randn(*gate.mask_linear_q.weight.shape, seed=5) * 0.05)
+        gate.mask_linear_k.weight.copy_(_randn(*gate.mask_linear_k.weight.shape, seed=6) * 0.05)
+    q, k = _randn(1, L, Hq, 128), _randn(1, L, Hkv, 128, seed=1)
+    nb = -(-L // 64)
+    tables = (_randn(1, nb, 128, dtype=torch.float32, seed=2), _randn(1, nb, 128, dtype=torch.float32, seed=3)) if rope else None
+    rule = SelectionRule(rule="topk", softmax=False, topk_ratio=(1, 4), sink=1, local=2)
+    past_blocks = _randn(1, past, Hkv, 128, seed=7)
+
+    def run():
+        st = GateSelectorState(gate, 1, torch.device("cuda"))
+        st.cache.reserve(past + nb)
+        st.cache.blocks_view()[:, :past].copy_(past_blocks)
+        st.cache.length = past
+        st.append(q, k, tables, tables)
+        t = st.score_select(rule, Hkv, 64)
+        return [st.q_blocks, st.cache.blocks().clone(), st.logits, t.block_idx, t.counts]
+
+    a, b = _both(ops, monkeypatch, run)
+    assert all(torch.equal(x, y) for x, y in zip(a, b))
