@@ -3,8 +3,8 @@
 // one answers None: on anything but the plain case (an argument of another kind, a failed check, an error code), so
 // that checks, messages and every less common form live in ops.py alone.
 //
-// Measured per call (host): attn_compact 7.5 us through Python; the reason this file exists is a decode step or a
-// short chunk, whose kernels take less than that.
+// Measured host time per pass, through Python -> here: a decode step 24 -> 10 us, an append 26 -> 8 us, a gate step
+// (prepare, scores and selection, attention) 98 -> 46 us; the decode and append kernels take 8 and 12 us.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 #include <ATen/ATen.h>

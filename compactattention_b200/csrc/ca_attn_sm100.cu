@@ -47,8 +47,13 @@ constexpr int kMaxSegs = 64;    // segments planned per batch
 constexpr float kRescaleThreshold = 8.0f;  // log2 units; lazy accumulator rescale
 constexpr int kMinSpanSteps = 8;           // shortest span worth a CTA of its own when units are cut
 // What cutting units costs a CTA (partials, the merge), in KV steps of about 2.2 us.  32 units of 27-30 steps: 44 us
-// cut, 66 us whole; of ~6 steps: 45 us cut, 22 us whole; of ~20 steps the two tie (54 us cut, 41 us whole).
-constexpr int kCutCostSteps = 12;
+// cut, 66 us whole; of ~6 steps: 45 us cut, 22 us whole; of ~20 steps 54 us cut, 37-41 us whole.
+constexpr int kCutCostSteps = 15;
+// What a unit costs beside its KV steps (Q, the first step's latency, the epilogue), in steps: the CTA with the ~29
+// short units at the head of a causal first chunk of 8192 tokens ran 1.08 M cycles where one with four long units of
+// the same steps ran 0.82 M, about 10,000 cycles a unit, three steps.
+// us with 0 / 2 / 3 / 4: 8192 x 8192, 32/8 heads 605 / 519 / 504 / 508, 4096 x 4096, 28/4 heads 217 / 153 / 142 / 145.
+constexpr int kUnitSteps = 3;
 // Measured on B200 (sustained 300-launch loop, 128K context, 20 % density): handing P to the MMA warp
 // in two halves 434 us, in one piece 450 us; packed fp32 pairs for the scale and the row sum 421 us.
 // A polynomial exp2 on the FMA pipe for part of the exponentials (2 / 4 / 6 of every 16 pairs) took
@@ -148,7 +153,7 @@ struct Shared {
   int more;            // another batch of segments follows
   int cut;             // spans may end inside a unit
   int cur_row, cur_pair;        // the unit the next segment comes from ...
-  long long cur_acc, next_x;    // ... its first linear KV step, and the step where the next segment starts
+  long long cur_acc;            // ... and where that starts on the line of all units
   int row_count[kMaxRows];
   long long row_prefix[kMaxRows + 1];
   Segment segs[kMaxSegs];
@@ -188,7 +193,10 @@ __device__ __forceinline__ int unit_iters(const KernelArgs& a, int count, int pa
   return (count * a.spb + chunk_subs(a, pair) + 1) >> 1;
 }
 
-// Finds the unit that holds linear KV step x (one warp, all lanes): its row and pair, its first step.
+// A unit's length on the line that the spans are cut from: kUnitSteps, then its KV steps.
+__device__ __forceinline__ int unit_cost(const KernelArgs& a, int count, int pair) { return unit_iters(a, count, pair) + kUnitSteps; }
+
+// Finds the unit that holds position x of the line (one warp, all lanes): its row and pair, where it starts.
 __device__ void locate_unit(const KernelArgs& a, const Shared* sh, long long x, int R, int lane, int* row, int* pair, long long* acc) {
   int lo = 0, hi = R;  // largest row with row_prefix[row] <= x
   while (hi - lo > 1) {
@@ -200,7 +208,7 @@ __device__ void locate_unit(const KernelArgs& a, const Shared* sh, long long x, 
   *row = lo, *pair = 0, *acc = base;
   for (int p0 = 0; p0 < a.n_pairs; p0 += 32) {
     const int p = p0 + lane;
-    const int ni = p < a.n_pairs ? unit_iters(a, count, p) : 0;
+    const int ni = p < a.n_pairs ? unit_cost(a, count, p) : 0;
     int inc = ni;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
@@ -222,34 +230,39 @@ __device__ void locate_unit(const KernelArgs& a, const Shared* sh, long long x, 
 __device__ void plan_segments(const KernelArgs& a, Shared* sh, long long span_begin, long long span_end, int R) {
   int n = 0;
   int row = sh->cur_row, pair = sh->cur_pair;
-  long long acc = sh->cur_acc, x = sh->next_x;
+  long long acc = sh->cur_acc;
   const bool cut = sh->cut != 0;
-  while (x < span_end && n < kMaxSegs && row < R) {
+#pragma unroll 1
+  while (acc < span_end && n < kMaxSegs && row < R) {
     const int count = sh->row_count[row];
     const int ni = unit_iters(a, count, pair);
-    Segment s;
-    s.row = row, s.pair = pair;
-    s.j0 = static_cast<int>(x - acc);
-    const long long rem = span_end - acc;
-    s.j1 = cut && rem < ni ? static_cast<int>(rem) : ni;
-    s.n_past_sub = count * a.spb;
-    s.n_sub = s.n_past_sub + chunk_subs(a, pair);
-    const bool partial = !(s.j0 == 0 && s.j1 == ni);
-    s.slot = partial ? static_cast<int>(2 * blockIdx.x + (x == span_begin ? 0 : 1)) : -1;
-    s.pad = 0;
-    if (partial) {
-      SegDesc d;
-      d.unit = row * a.n_pairs + pair, d.j0 = s.j0, d.j1 = s.j1, d.n_iter = ni;
-      a.descs[s.slot] = d;
+    int j0 = 0, j1 = ni;
+    if (cut) {  // a boundary within the unit's first kUnitSteps cuts nothing off
+      const long long before = span_begin - acc - kUnitSteps;
+      if (before > 0) j0 = static_cast<int>(before);
+      const long long left = span_end - acc - kUnitSteps;
+      if (left < ni) j1 = static_cast<int>(left);
     }
-    sh->segs[n++] = s;
-    x = acc + s.j1;
-    acc += ni;
+    if (j1 > j0) {
+      Segment& s = sh->segs[n++];
+      s.row = row, s.pair = pair, s.j0 = j0, s.j1 = j1;
+      s.n_past_sub = count * a.spb;
+      s.n_sub = s.n_past_sub + chunk_subs(a, pair);
+      s.slot = -1;
+      if (j0 > 0 || j1 < ni) {
+        const int slot = static_cast<int>(2 * blockIdx.x + (j0 > 0 ? 0 : 1));
+        s.slot = slot;
+        SegDesc d;
+        d.unit = row * a.n_pairs + pair, d.j0 = j0, d.j1 = j1, d.n_iter = ni;
+        a.descs[slot] = d;
+      }
+    }
+    acc += ni + kUnitSteps;
     if (++pair == a.n_pairs) pair = 0, ++row;
   }
   sh->n_segs = n;
-  sh->cur_row = row, sh->cur_pair = pair, sh->cur_acc = acc, sh->next_x = x;
-  sh->more = (x < span_end && row < R) ? 1 : 0;
+  sh->cur_row = row, sh->cur_pair = pair, sh->cur_acc = acc;
+  sh->more = (acc < span_end && row < R) ? 1 : 0;
 }
 
 // P = exp2(S*sc + neg_m) for one 128-column row held in registers: packs to 16 bit, stores the four
@@ -343,7 +356,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   }
   ptx::grid_dependency_wait();  // nothing in global memory is touched before this
 
-  // ---- per-row KV-step totals and their prefix (every CTA; a warp per row) ----
+  // ---- per-row totals (KV steps and what units cost beside them) and their prefix (every CTA; a warp per row) ----
   for (int r = warp; r < R; r += kThreads / 32) {
     int count = a.past_blocks;
     if (a.block_idx != nullptr) {
@@ -355,7 +368,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
     }
     int tot = 0;
-    for (int p = lane; p < a.n_pairs; p += 32) tot += unit_iters(a, count, p);
+    for (int p = lane; p < a.n_pairs; p += 32) tot += unit_cost(a, count, p);
     tot = __reduce_add_sync(0xffffffffu, tot);
     if (lane == 0) {
       sh->row_count[r] = count;
@@ -380,15 +393,15 @@ __global__ void __launch_bounds__(kThreads, 1)
     // shortest and longest unit: the first pair of the shortest row, the last pair of the longest
     int c_lo = 0x7fffffff, c_hi = 0;
     for (int r = lane; r < R; r += 32) c_lo = min(c_lo, sh->row_count[r]), c_hi = max(c_hi, sh->row_count[r]);
-    const int l_min = unit_iters(a, __reduce_min_sync(0xffffffffu, c_lo), 0);
-    const int l_max = unit_iters(a, __reduce_max_sync(0xffffffffu, c_hi), a.n_pairs - 1);
+    const int l_min = unit_cost(a, __reduce_min_sync(0xffffffffu, c_lo), 0);
+    const int l_max = unit_cost(a, __reduce_max_sync(0xffffffffu, c_hi), a.n_pairs - 1);
     __syncwarp();
     const long long total = sh->row_prefix[R];
     const long long c = blockIdx.x;
     const long long n_units = static_cast<long long>(R) * a.n_pairs;
     // Cut or whole: compare what the longest-running CTA has to do, in KV steps.  (Dealing whole units out by their
     // number gave the last CTAs of a causal first chunk twice the mean work: 8192 tokens, 32/8 heads, f16 1045 us,
-    // cut by this rule 667 us; 16 units of one KV head at 128K: 442 us whole, 91 us cut.)
+    // cut by this rule 504 us; 16 units of one KV head at 128K: 442 us whole, 91 us cut.)
     // Cut: an equal share and the price of cutting.  A span costs a prologue, an epilogue and (when it cuts a
     // unit) 128 KB of partials, about as much as kMinSpanSteps KV steps: with little work, fewer CTAs take
     // longer spans and the others leave at once.
@@ -426,7 +439,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     if (span_end > span_begin && (cut || n_units > g)) {
       locate_unit(a, sh, span_begin, R, lane, &row, &pair, &acc);
       if (!cut && acc < span_begin) {
-        acc += unit_iters(a, sh->row_count[row], pair);
+        acc += unit_cost(a, sh->row_count[row], pair);
         if (++pair == a.n_pairs) pair = 0, ++row;
         span_begin = acc;
       }
@@ -434,7 +447,6 @@ __global__ void __launch_bounds__(kThreads, 1)
     if (lane == 0) {
       sh->cut = cut ? 1 : 0;
       sh->cur_row = row, sh->cur_pair = pair, sh->cur_acc = acc;
-      sh->next_x = span_begin;
       sh->more = span_end > span_begin && row < R ? 1 : 0;
       sh->n_segs = 0;
     }
@@ -459,7 +471,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   if (warp >= 8) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
     while (true) {
-      __syncthreads();  // thread 0 (softmax side) has planned the next batch
+      __syncthreads();
       const int n_segs = sh->n_segs;
       if (n_segs == 0) break;
       if (warp == 9) {
@@ -698,7 +710,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             if (masked) {
               lim0 = visible_cols(2 * j, sg.n_sub, sg.n_past_sub, t + a.q_off);
               lim1 = visible_cols(2 * j + 1, sg.n_sub, sg.n_past_sub, t + a.q_off);
-              // in a long chunk most of these steps lie wholly before the warp's rows (8192 x 8192: 667 -> 599 us)
+              // in a long chunk most of these steps lie wholly before the warp's rows (8192 x 8192: 667 -> 604 us)
               masked = __any_sync(0xffffffffu, lim0 < kSub || lim1 < kSub);
             }
             // the whole S row (128 fp32) comes into registers with one wait
