@@ -698,15 +698,21 @@ struct PrepSide {
 struct PrepArgs {
   PrepSide q, k;
   int B, L, D, C, bs, nb;
+  int part_kinds;   // pooling kinds that the partials in shared memory have room for
 };
+constexpr int kPrepStageBytes = 32 * 1024;
 
 constexpr int kPrepThreads = 128;
 
-template <int XDT, int WDT>
-__global__ void __launch_bounds__(kPrepThreads) gate_prepare_kernel(const PrepArgs a) {
+// kStage: both sides' weights fit kPrepStageBytes a head; each is copied to shared memory while the tokens are pooled
+// (us a launch with / without, Qavg_Kavg, bf16: 1024 tokens, 32/8 heads 7.5 / 8.6, one KV head 4.4 / 5.0, 2048 12.7 / 15.1,
+// 8192, 28/4 36.2 / 42.7, 256 6.3 / 7.5).  Bounded to five CTAs an SM, the 640 CTAs of 1024 tokens then run in one wave.
+template <int XDT, int WDT, bool kStage>
+__global__ void __launch_bounds__(kPrepThreads, 5) gate_prepare_kernel(const PrepArgs a) {
   ptx::grid_launch_dependents();
   ptx::grid_dependency_wait();  // nothing in global memory is touched before this
-  extern __shared__ float prep_smem[];  // partials [3][phases][D], pooled [3*D], y [C]
+  // partials [part_kinds][phases][D], pooled [3*D], y [C], then the head's staged weight
+  extern __shared__ __align__(16) float prep_smem[];
   const bool is_q = static_cast<int>(blockIdx.y) < a.q.Hw;
   const PrepSide& sd = is_q ? a.q : a.k;
   const int hw = is_q ? blockIdx.y : blockIdx.y - a.q.Hw;  // output / weight head
@@ -715,8 +721,31 @@ __global__ void __launch_bounds__(kPrepThreads) gate_prepare_kernel(const PrepAr
   const int groups = a.D / 8;
   const int phases = kPrepThreads / groups;
   float* part = prep_smem;
-  float* pooled = part + 3 * phases * a.D;
+  float* pooled = part + a.part_kinds * phases * a.D;
   float* y = pooled + 3 * a.D;
+  const int n_kinds = ((sd.kinds & 1) ? 1 : 0) + ((sd.kinds & 2) ? 1 : 0) + ((sd.kinds & 4) ? 1 : 0);
+  const int Cin = n_kinds * a.D;
+  // The head's weight and the block's RoPE row depend on nothing: they are on their way while the tokens are pooled
+  // (one memory latency instead of three in a row).
+  constexpr int kWBytes = WDT == CA_DTYPE_F32 ? 4 : 2;
+  const int w_bytes = Cin * a.C * kWBytes;
+  const bool staged = kStage && sd.w != nullptr;
+  uint8_t* w_sm = reinterpret_cast<uint8_t*>(y + a.C);
+  if (staged) {
+    const uint8_t* w = static_cast<const uint8_t*>(sd.w) + static_cast<long long>(hw) * w_bytes;
+    const uint32_t dst = ptx::smem_u32(w_sm);
+    for (int e = threadIdx.x * 16; e < w_bytes; e += kPrepThreads * 16) {
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + e), "l"(w + e) : "memory");
+    }
+  }
+  const long long rope_row = ((sd.rope_batch > 1 ? static_cast<long long>(b) : 0) * a.nb + blk) * a.C;
+  float rope_c = 0.f, rope_s = 0.f;  // channel threadIdx.x
+  if (sd.cos && static_cast<int>(threadIdx.x) < a.C) {
+    rope_c = sd.cos[rope_row + threadIdx.x];
+    rope_s = sd.sin[rope_row + threadIdx.x];
+  }
+  // where each pooling kind's partials go
+  const int slot_min = sd.kinds & 1, slot_sum = (sd.kinds & 1) + ((sd.kinds >> 1) & 1);
   const int grp = threadIdx.x % groups, ph = threadIdx.x / groups;
   const int t0 = blk * a.bs, t1 = min(t0 + a.bs, a.L);
   float mx[8], mn[8], sm[8];
@@ -743,28 +772,32 @@ __global__ void __launch_bounds__(kPrepThreads) gate_prepare_kernel(const PrepAr
     }
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      part[(0 * phases + ph) * a.D + grp * 8 + i] = mx[i];
-      part[(1 * phases + ph) * a.D + grp * 8 + i] = mn[i];
-      part[(2 * phases + ph) * a.D + grp * 8 + i] = sm[i];
+      if (sd.kinds & 1) part[ph * a.D + grp * 8 + i] = mx[i];
+      if (sd.kinds & 2) part[(slot_min * phases + ph) * a.D + grp * 8 + i] = mn[i];
+      if (sd.kinds & 4) part[(slot_sum * phases + ph) * a.D + grp * 8 + i] = sm[i];
     }
   }
   __syncthreads();
   const float inv_cnt = 1.0f / static_cast<float>(t1 - t0);
-  int n_kinds = 0;
   for (int d = threadIdx.x; d < a.D; d += kPrepThreads) {
-    float rmx = -INFINITY, rmn = INFINITY, rsm = 0.f;
-    for (int p = 0; p < phases; ++p) {
-      rmx = fmaxf(rmx, part[(0 * phases + p) * a.D + d]);
-      rmn = fminf(rmn, part[(1 * phases + p) * a.D + d]);
-      rsm += part[(2 * phases + p) * a.D + d];
-    }
     int c = 0;
-    if (sd.kinds & 1) pooled[(c++) * a.D + d] = rmx;
-    if (sd.kinds & 2) pooled[(c++) * a.D + d] = rmn;
-    if (sd.kinds & 4) pooled[(c++) * a.D + d] = rsm * inv_cnt;
+    if (sd.kinds & 1) {
+      float r = -INFINITY;
+      for (int p = 0; p < phases; ++p) r = fmaxf(r, part[p * a.D + d]);
+      pooled[(c++) * a.D + d] = r;
+    }
+    if (sd.kinds & 2) {
+      float r = INFINITY;
+      for (int p = 0; p < phases; ++p) r = fminf(r, part[(slot_min * phases + p) * a.D + d]);
+      pooled[(c++) * a.D + d] = r;
+    }
+    if (sd.kinds & 4) {
+      float r = 0.f;
+      for (int p = 0; p < phases; ++p) r += part[(slot_sum * phases + p) * a.D + d];
+      pooled[(c++) * a.D + d] = r * inv_cnt;
+    }
   }
-  n_kinds = ((sd.kinds & 1) ? 1 : 0) + ((sd.kinds & 2) ? 1 : 0) + ((sd.kinds & 4) ? 1 : 0);
-  const int Cin = n_kinds * a.D;
+  if (staged) asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
   if (sd.w) {
     // Thread = (8 output channels, input-channel phase): every load is a 128-bit piece of a weight row
@@ -781,7 +814,8 @@ __global__ void __launch_bounds__(kPrepThreads) gate_prepare_kernel(const PrepAr
         for (int u = 0; u < 8; ++u) {
           const int c = c0 + u * cphases;
           if (c < Cin) {
-            load8_t<WDT>(sd.w, wbase + static_cast<long long>(c) * a.C, w[u]);
+            if (kStage) load8_t<WDT>(w_sm, static_cast<long long>(c) * a.C + og * 8, w[u]);
+            else load8_t<WDT>(sd.w, wbase + static_cast<long long>(c) * a.C, w[u]);
           } else {
 #pragma unroll
             for (int i = 0; i < 8; ++i) w[u][i] = 0.f;
@@ -812,9 +846,9 @@ __global__ void __launch_bounds__(kPrepThreads) gate_prepare_kernel(const PrepAr
   for (int o = threadIdx.x; o < a.C; o += kPrepThreads) {
     float v = y[o];
     if (sd.cos) {
-      const long long ro = ((sd.rope_batch > 1 ? static_cast<long long>(b) : 0) * a.nb + blk) * a.C + o;
       const float rot = o < half ? -y[o + half] : y[o - half];
-      v = v * sd.cos[ro] + rot * sd.sin[ro];
+      const bool mine = o == static_cast<int>(threadIdx.x);  // loaded at the start
+      v = v * (mine ? rope_c : sd.cos[rope_row + o]) + rot * (mine ? rope_s : sd.sin[rope_row + o]);
     }
     store_elem(sd.out, b * sd.o_b + static_cast<long long>(sd.out_block_offset + blk) * sd.o_blk + hw * sd.o_h + o, sd.o_dtype, v);
   }
@@ -892,8 +926,23 @@ int ca_gate_prepare(const ca_gate_prepare_params* p, ca_stream_t stream_) {
   a.B = p->B, a.L = p->L, a.D = p->D, a.C = p->C, a.bs = p->block_size;
   a.nb = ceil_div(p->L, p->block_size);
   const int phases = kPrepThreads / (p->D / 8);
-  const size_t smem = (static_cast<size_t>(3) * phases * p->D + 3 * p->D + p->C) * sizeof(float);
-  CA_REQUIRE(smem <= 48 * 1024, "D and C too large for the gate preparation kernel");
+  auto kinds_of = [](int kinds) { return (kinds & 1) + ((kinds >> 1) & 1) + ((kinds >> 2) & 1); };
+  const int nq = kinds_of(p->q.kinds), nk = kinds_of(p->k.kinds);
+  CA_REQUIRE((static_cast<size_t>(3) * phases * p->D + 3 * p->D + p->C) * sizeof(float) <= 48 * 1024,
+             "D and C too large for the gate preparation kernel");
+  a.part_kinds = nq > nk ? nq : nk;
+  size_t smem = (static_cast<size_t>(a.part_kinds) * phases * p->D + 3 * p->D + p->C) * sizeof(float);
+  // Both sides' weights are staged where a head's fits (a gate of 128 x 128 channels in 16 bits: 38 KB a CTA in all);
+  // larger ones are read where they are used (Kmaxminavg with only its query side staged: 19.3 us against 12.2).
+  size_t stage_bytes = 0;
+  bool stage = p->q.w != nullptr || p->k.w != nullptr;
+  for (int i = 0; i < 2; ++i) {
+    const size_t bytes = static_cast<size_t>(i ? nk : nq) * p->D * p->C * (sides[i]->w_dtype == CA_DTYPE_F32 ? 4 : 2);
+    if (sides[i]->w == nullptr) continue;
+    stage = stage && bytes <= kPrepStageBytes && smem + bytes <= 48 * 1024;
+    if (bytes > stage_bytes) stage_bytes = bytes;
+  }
+  if (stage) smem += stage_bytes;
   CA_REQUIRE(p->q.x_dtype == p->k.x_dtype, "q and k tokens must share a dtype");
   const int wdt = p->k.w ? p->k.w_dtype : (p->q.w ? p->q.w_dtype : p->q.x_dtype);
   CA_REQUIRE((p->q.w == nullptr || p->q.w_dtype == wdt) && (p->k.w == nullptr || p->k.w_dtype == wdt), "q and k weights must share a dtype");
@@ -901,7 +950,8 @@ int ca_gate_prepare(const ca_gate_prepare_params* p, ca_stream_t stream_) {
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
 #define CA_PREP_CASE(XD, WD)                                                            \
   if (p->q.x_dtype == XD && wdt == WD) {                                                \
-    launch_kernel_as(true, gate_prepare_kernel<XD, WD>, dim3(grid), dim3(kPrepThreads), smem, stream, a);     \
+    if (stage) launch_kernel_as(true, gate_prepare_kernel<XD, WD, true>, dim3(grid), dim3(kPrepThreads), smem, stream, a); \
+    else launch_kernel_as(true, gate_prepare_kernel<XD, WD, false>, dim3(grid), dim3(kPrepThreads), smem, stream, a);      \
   } else
   CA_PREP_CASE(CA_DTYPE_BF16, CA_DTYPE_BF16)
   CA_PREP_CASE(CA_DTYPE_BF16, CA_DTYPE_F32)
