@@ -245,11 +245,11 @@ extern "C" int ca_rope_append(const ca_rope_append_params* p, ca_stream_t stream
   CA_REQUIRE(grid.y <= 65535 && grid.z <= 65535, "too many heads or batch entries for one launch");
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   if (a.is_bf16) {
-    if (a.rope_f32) launch_kernel(rope_append_kernel<__nv_bfloat16, true>, dim3(grid), dim3(kThreads), smem, stream, a);
-    else launch_kernel(rope_append_kernel<__nv_bfloat16, false>, dim3(grid), dim3(kThreads), smem, stream, a);
+    if (a.rope_f32) launch_kernel_as(true, rope_append_kernel<__nv_bfloat16, true>, dim3(grid), dim3(kThreads), smem, stream, a);
+    else launch_kernel_as(true, rope_append_kernel<__nv_bfloat16, false>, dim3(grid), dim3(kThreads), smem, stream, a);
   } else {
-    if (a.rope_f32) launch_kernel(rope_append_kernel<__half, true>, dim3(grid), dim3(kThreads), smem, stream, a);
-    else launch_kernel(rope_append_kernel<__half, false>, dim3(grid), dim3(kThreads), smem, stream, a);
+    if (a.rope_f32) launch_kernel_as(true, rope_append_kernel<__half, true>, dim3(grid), dim3(kThreads), smem, stream, a);
+    else launch_kernel_as(true, rope_append_kernel<__half, false>, dim3(grid), dim3(kThreads), smem, stream, a);
   }
   CA_LAUNCH_CHECK("rope_append_kernel");
   return CA_OK;

@@ -48,7 +48,7 @@ int ca_abi_version(void);
 int64_t ca_launch_count(void);
 /*
  * Programmatic dependent launch of the kernels that are enqueued plainly otherwise (off by default; the kernels of
- * the path - pooling, gate, scores, selection, table, gather, attention - are always enqueued so): a
+ * the path - append, pooling, gate, scores, selection, table, gather, attention - are always enqueued so): a
  * kernel's CTAs may become resident and run their prologue while the previous kernel in the stream drains; each
  * kernel waits (griddepcontrol.wait) before its first global-memory access, so results do not change.  Returns the
  * previous setting.  No reference counterpart (the reference launches through torch / Triton).
