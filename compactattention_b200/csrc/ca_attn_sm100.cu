@@ -45,10 +45,13 @@ constexpr int kTmemCols = 512;
 constexpr int kMaxRows = 1024;  // (batch x kv heads) rows per launch
 constexpr int kMaxSegs = 64;    // segments planned per batch
 constexpr float kRescaleThreshold = 8.0f;  // log2 units; lazy accumulator rescale
-constexpr int kMinSpanSteps = 8;           // shortest span worth a CTA of its own when units are cut
-// What cutting units costs a CTA (partials, the merge), in KV steps of about 2.2 us.  32 units of 27-30 steps: 44 us
-// cut, 66 us whole; of ~6 steps: 45 us cut, 22 us whole; of ~20 steps 54 us cut, 37-41 us whole.
-constexpr int kCutCostSteps = 15;
+constexpr int kMinSpanSteps = 4;           // shortest span worth a CTA of its own when units are cut
+// What cutting units costs a CTA (partials, the merge), in KV steps of about 2.2 us, with up to ~8 pieces a unit; every
+// further piece costs the merge about kPieceSteps more (4 units of 105 steps in 13 / 21 / 27 / 36 pieces each: 46 / 49 /
+// 53 / 60 us).  Whole against cut, us: 64 units of 1-16 steps 44 / 31, 256 of them 73 / 61, 32 of ~20 37 / 32, 16 units of
+// one KV head at 128K 442 / 77; units of at most 8 steps, one per SM, stay whole (27).
+constexpr float kPieceSteps = 0.45f;
+constexpr int kCutCostSteps = 9;
 // What a unit costs beside its KV steps (Q, the first step's latency, the epilogue), in steps: the CTA with the ~29
 // short units at the head of a causal first chunk of 8192 tokens ran 1.08 M cycles where one with four long units of
 // the same steps ran 0.82 M, about 10,000 cycles a unit, three steps.
@@ -401,14 +404,16 @@ __global__ void __launch_bounds__(kThreads, 1)
     const long long n_units = static_cast<long long>(R) * a.n_pairs;
     // Cut or whole: compare what the longest-running CTA has to do, in KV steps.  (Dealing whole units out by their
     // number gave the last CTAs of a causal first chunk twice the mean work: 8192 tokens, 32/8 heads, f16 1045 us,
-    // cut by this rule 504 us; 16 units of one KV head at 128K: 442 us whole, 91 us cut.)
-    // Cut: an equal share and the price of cutting.  A span costs a prologue, an epilogue and (when it cuts a
-    // unit) 128 KB of partials, about as much as kMinSpanSteps KV steps: with little work, fewer CTAs take
-    // longer spans and the others leave at once.
+    // cut by this rule 504 us.)
+    // Cut: an equal share and the price of cutting.  With little work, fewer CTAs take longer spans (not under
+    // kMinSpanSteps, and no more of them than keep share + merge of nc / n_units pieces smallest); the others leave
+    // at once.
     long long nc = gridDim.x;
     const long long by_work = total / kMinSpanSteps;
     const long long most = by_work > n_units ? by_work : n_units;
     if (most < nc) nc = most;
+    const int best = static_cast<int>(__fsqrt_rn(static_cast<float>(total) * static_cast<float>(n_units) * (1.0f / kPieceSteps)));
+    nc = min(static_cast<int>(nc), max(best, 1));
     const long long t_cut = total / nc + kCutCostSteps;
     // Whole: the longest unit when every unit has a CTA; equal unit counts when units are about equally long;
     // otherwise a share that ends up to a unit late.
