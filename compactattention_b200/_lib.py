@@ -306,6 +306,7 @@ class CallList:
 
     def __init__(self):
         self.calls = []
+        self.keep = []  # scratch tensors of the recorded calls' own
 
     def run(self) -> None:
         for name, fn, args in self.calls:

@@ -159,8 +159,7 @@ class StepScratch:
                                     torch.empty((batch, kv_heads), dtype=torch.int32, device=device),
                                     torch.empty((batch, kv_heads), dtype=torch.int32, device=device),
                                     torch.empty((batch, kv_heads), dtype=torch.int32, device=device))
-        self.union = ops.union_scratch(torch.device(device) if not isinstance(device, torch.device) else device, batch, heads,
-                                       kv_heads, q_blocks, max_blocks)
+        self.union = ops.new_union_scratch(torch.device(device), batch, heads, kv_heads, q_blocks, max_blocks)
         self.status = torch.zeros(1, dtype=torch.int32, device=device)
 
 
@@ -332,11 +331,10 @@ def capture_step(fn, warmup: int = 2) -> "torch.cuda.CUDAGraph":
     selector scores -> row rule -> Block-Union table -> attention at one chunk position — into a CUDA
     graph and returns it; ``graph.replay()`` then enqueues the whole step with one host call.
 
-    The entry points allocate nothing and never synchronise; what the tensor-level wrappers cache per stream
-    (the attention workspace that lets the kernel cut work units, the union scratch of the fused selection) and
-    the library's per-device kernel attributes are set up by the warm-up calls.  Warm-up and capture run on
-    the SAME side stream, so the capture finds those buffers in the cache instead of allocating them inside
-    the graph; their addresses are baked into the graph, and they stay alive in the wrappers' caches.  A step
+    The entry points allocate nothing and never synchronise; the library's per-device kernel attributes are set up
+    by the warm-up calls, and so is the attention workspace of their stream, whose address is baked into the graph.
+    The union scratch of the fused selection, which the wrappers otherwise keep per stream, is allocated and zeroed
+    inside the graph's own memory, so a graph shares none of it with eager calls or with other graphs.  A step
     is only replayable while its shapes hold (the chunk position is baked into the launch parameters), which
     is the case for a layer stack at one chunk position and for a benchmark loop.
     """

@@ -364,18 +364,40 @@ def select_rows(
 _UNION_SCRATCH: dict = {}
 
 
-def union_scratch(device: torch.device, batch: int, heads: int, num_kv_heads: int, q_blocks: int, kv_blocks: int) -> torch.Tensor:
-    """Scratch of the fused selection + table launch: a ticket per KV-head row (zero on entry, left zero by the
-    kernel) followed by room for the rows' packed bits.  One buffer per (device, stream) serves every call on
-    that stream and ticket count (the ticket words must never have held anything else); it only grows."""
-    key = (device.index, _stream(), batch * num_kv_heads)
+def _union_scratch_words(batch: int, heads: int, num_kv_heads: int, q_blocks: int, kv_blocks: int) -> int:
     need = C.c_size_t(0)
     _lib.check(_lib.load().ca_select_union_scratch_bytes(batch, heads, num_kv_heads, q_blocks, kv_blocks, C.byref(need)),
                "ca_select_union_scratch_bytes")
+    return (int(need.value) + 3) // 4
+
+
+def new_union_scratch(device: torch.device, batch: int, heads: int, num_kv_heads: int, q_blocks: int, kv_blocks: int) -> torch.Tensor:
+    """Scratch of the fused selection + table launch: a ticket per KV-head row (zero on entry, left zero by the
+    kernel) followed by room for the rows' packed bits."""
+    return torch.zeros(_union_scratch_words(batch, heads, num_kv_heads, q_blocks, kv_blocks), dtype=torch.int32, device=device)
+
+
+def _call_is_kept() -> bool:
+    """Whether the launches are being kept for later (a graph capture, a call recording) rather than only run.  Such a
+    call may not use the scratch kept per stream: by the time it runs again, that may have been outgrown and freed, be
+    in use on another stream, or never have been zeroed (a capture records the zeroing, it does not do it)."""
+    return _lib._recording is not None or torch.cuda.is_current_stream_capturing()
+
+
+def union_scratch(device: torch.device, batch: int, heads: int, num_kv_heads: int, q_blocks: int, kv_blocks: int) -> torch.Tensor:
+    """``new_union_scratch``, kept: one buffer per (device, stream) serves every call on that stream and ticket count
+    (the ticket words must never have held anything else); it only grows.  A captured or recorded call gets a buffer
+    of its own: part of the graph's memory, and zeroed by each replay; kept alive by the recording."""
+    if _call_is_kept():
+        buf = new_union_scratch(device, batch, heads, num_kv_heads, q_blocks, kv_blocks)
+        if _lib._recording is not None:
+            _lib._recording.keep.append(buf)
+        return buf
+    key = (device.index, _stream(), batch * num_kv_heads)
+    need = _union_scratch_words(batch, heads, num_kv_heads, q_blocks, kv_blocks)
     buf = _UNION_SCRATCH.get(key)
-    if buf is None or buf.numel() * 4 < need.value:
-        buf = torch.zeros((int(need.value) + 3) // 4, dtype=torch.int32, device=device)
-        _UNION_SCRATCH[key] = buf
+    if buf is None or buf.numel() < need:
+        buf = _UNION_SCRATCH[key] = torch.zeros(need, dtype=torch.int32, device=device)
     return buf
 
 
@@ -419,7 +441,9 @@ def select_union_table(
         native = _native()
     if native is not None:
         stream = _stream()
-        words = _UNION_SCRATCH.get((score.device.index, stream, B * num_kv_heads)) if scratch is None else scratch
+        words = scratch
+        if words is None and not _call_is_kept():
+            words = _UNION_SCRATCH.get((score.device.index, stream, B * num_kv_heads))
         if words is not None:
             num, den = topk_ratio if topk_ratio is not None else (0, 1)
             given = (None,) * 4 if out is None else (out.block_idx, out.counts, out.cache_seqlens, out.pages_per_row)
