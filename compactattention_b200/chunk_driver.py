@@ -316,10 +316,9 @@ class GateLayerStep:
             sl.H, sl.Qb, sl.Kb, sl.Pb = gate.num_q_head, nb, Kb, Pb
             p.table.G, p.table.Qin, p.table.Kb, p.table.Pb = gate.num_q_head // self.num_kv_heads, nb, Kb, Pb
             at.block_idx, at.counts = sc.table.block_idx.data_ptr(), sc.table.counts.data_ptr()
-        if at.workspace is None:
-            ws = ops.attn_workspace(q_nope.device, at)
-            at.workspace, at.workspace_bytes = ws.data_ptr(), ws.numel()
-            keep.append(ws)
+        ws = ops.attn_workspace(q_nope.device, at)  # of this call's stream, or of the graph that it is captured into
+        at.workspace, at.workspace_bytes = ws.data_ptr(), ws.numel()
+        keep.append(ws)
         self._keep = keep
         self._lib.check(self._lib.load().ca_chunk_step(ctypes.byref(p), ops._stream()), "ca_chunk_step")
         self.kv.length = max(self.kv.length, kv_len)
@@ -332,9 +331,9 @@ def capture_step(fn, warmup: int = 2) -> "torch.cuda.CUDAGraph":
     graph and returns it; ``graph.replay()`` then enqueues the whole step with one host call.
 
     The entry points allocate nothing and never synchronise; the library's per-device kernel attributes are set up
-    by the warm-up calls, and so is the attention workspace of their stream, whose address is baked into the graph.
-    The union scratch of the fused selection, which the wrappers otherwise keep per stream, is allocated and zeroed
-    inside the graph's own memory, so a graph shares none of it with eager calls or with other graphs.  A step
+    by the warm-up calls.  Scratch that the tensor-level wrappers otherwise keep per stream (the attention workspace
+    that lets the kernel cut work units, the union scratch of the fused selection) is allocated inside the graph's own
+    memory, so a graph shares none of it with eager calls or with other graphs, on whatever streams they run.  A step
     is only replayable while its shapes hold (the chunk position is baked into the launch parameters), which
     is the case for a layer stack at one chunk position and for a benchmark loop.
     """

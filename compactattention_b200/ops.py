@@ -138,14 +138,17 @@ _ATTN_WORKSPACES: dict = {}
 def attn_workspace(device: torch.device, params: "_lib.AttnParams") -> torch.Tensor:
     """Scratch for the attention kernel's split units (partial accumulators of the segments that the
     combine kernel merges).  One buffer per (device, stream): launches on one stream run in order, so
-    they can share it; launches on different streams must not."""
+    they can share it; launches on different streams must not.  A call that is being captured gets a buffer
+    of its own, from the graph's memory: the graph may be replayed on any stream, beside other graphs."""
     key = (device.index, _stream())
-    ws = _ATTN_WORKSPACES.get(key)
+    capturing = torch.cuda.is_current_stream_capturing()
+    ws = None if capturing else _ATTN_WORKSPACES.get(key)
     if ws is None:
         need = C.c_size_t(0)
         _lib.check(_lib.load().ca_attn_workspace_bytes(C.byref(params), C.byref(need)), "ca_attn_workspace_bytes")
         ws = torch.empty(max(int(need.value), 256), dtype=torch.uint8, device=device)
-        _ATTN_WORKSPACES[key] = ws
+        if not capturing:
+            _ATTN_WORKSPACES[key] = ws
     return ws
 
 
@@ -172,7 +175,9 @@ def attn_compact(
     native = _native() if use_workspace else None
     if native is not None:
         stream = _stream()
-        ws = _ATTN_WORKSPACES.get((q.device.index, stream)) if workspace is None else workspace
+        ws = workspace
+        if ws is None and not torch.cuda.is_current_stream_capturing():
+            ws = _ATTN_WORKSPACES.get((q.device.index, stream))
         if ws is not None:
             done = native.attn_compact(stream, ws, q, kv.k, kv.v, kv.page_stride, kv.token_stride, kv.head_stride, kv.page_size,
                                        kv.num_pages, kv.pages_per_seq, kv.head_div, kv.page_table, kv_len, num_kv_heads, block_idx,

@@ -1,4 +1,4 @@
-"""Scratch under CUDA graphs and call recordings: a captured or recorded step shares no tickets or row bits with
+"""Scratch under CUDA graphs and call recordings: a captured or recorded step shares no tickets, row bits or partials with
 eager calls that run (and outgrow the buffers kept per stream) later, nor with other graphs, whatever the replay order."""
 import pytest
 import torch
@@ -82,6 +82,30 @@ def test_the_second_capture_replayed_first(ops, kind):
         graph.replay()
         torch.cuda.synchronize()
         assert torch.equal(out, wants[i])
+
+
+@pytest.mark.parametrize("kind", ["keep", "flash", "gate"])
+def test_graphs_of_one_stream_replayed_on_two(ops, kind):
+    fns = [_step(kind, 512, 16384, s) for s in (5, 6)]
+    wants = [fn().clone() for fn in fns]
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        for fn in fns:
+            fn()
+    torch.cuda.synchronize()
+    graphs = [_capture(fn, side) for fn in fns]
+    streams = [torch.cuda.Stream() for _ in graphs]
+    same = [torch.zeros((), dtype=torch.int64, device="cuda") for _ in graphs]
+    for (_, out) in graphs:
+        out.zero_()
+    torch.cuda.synchronize()
+    for _ in range(20):
+        for (graph, out), st, want, n in zip(graphs, streams, wants, same):
+            with torch.cuda.stream(st):
+                graph.replay()
+                n += (out == want).all()
+    torch.cuda.synchronize()
+    assert [int(n) for n in same] == [20, 20]
 
 
 def test_recorded_calls_keep_their_scratch(ops):
