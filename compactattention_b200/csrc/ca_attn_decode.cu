@@ -16,6 +16,7 @@
 // (1.07 GB, 6.64 TB/s), one of 131072 145 -> 85 us, one of 4001 31 -> 8.3 us; one KV head, 131072 tokens 184 -> 19 us;
 // 16 x 8192, 28/4 heads 81 -> 45 us.
 #include "ca_attn_shared.cuh"
+#include "ca_ring.cuh"
 
 #include <cooperative_groups.h>
 #include <mutex>
@@ -185,12 +186,12 @@ __global__ void __launch_bounds__(kThreads, 2)
   const int n_sub = n_past_sub + (a.Q - 1 + a.q_off) / kSub + 1;
   const long long slices = static_cast<long long>(a.parts) * cs, slice = static_cast<long long>(part) * cs + rank;
   const int u0 = static_cast<int>(n_sub * slice / slices), u1 = static_cast<int>(n_sub * (slice + 1) / slices);
+  int issued = 0;  // ring entries whose copies have been issued (producer lane)
 
   if (warp == kWarps) {
     // =============================== TMA producer ===============================
     const int b = row / a.Hkv, head = (row % a.Hkv) / a.kv_head_div;
     bool ok = true;
-    int n = 0;
     for (int base = u0; base < u1 && ok; base += 32) {
       // every lane resolves one sub-block of this batch of 32
       const int u = base + lane;
@@ -221,11 +222,11 @@ __global__ void __launch_bounds__(kThreads, 2)
         }
       }
       const int m = u1 - base < 32 ? u1 - base : 32;
-      for (int i = 0; i < m && ok; ++i, ++n) {
+      for (int i = 0; i < m && ok; ++i) {
         const int p0 = __shfl_sync(0xffffffffu, page, i), o0 = __shfl_sync(0xffffffffu, off, i);
         if (lane == 0) {
-          const int s = n % kStages;
-          ok = ptx::mbar_wait_bounded(ptx::smem_u32(&sh->empty[s]), ((n / kStages) & 1) ^ 1u, abort_flag, limit);
+          const int s = issued % kStages;
+          ok = ptx::mbar_wait_bounded(ptx::smem_u32(&sh->empty[s]), ((issued / kStages) & 1) ^ 1u, abort_flag, limit);
           if (ok) {
             const uint32_t bar = ptx::smem_u32(&sh->full[s]), dst = ring + s * kStageBytes;
             ptx::mbar_expect_tx(bar, kStageBytes);
@@ -233,16 +234,10 @@ __global__ void __launch_bounds__(kThreads, 2)
             c[a.slot_tok] = o0, c[a.slot_page] = p0, c[a.slot_head] = head;
             for (int h = 0; h < 2; ++h) ptx::tma_load_4d(dst + h * kBoxBytes, &k_map, bar, h * 64, c[0], c[1], c[2]);
             for (int h = 0; h < 2; ++h) ptx::tma_load_4d(dst + (2 + h) * kBoxBytes, &v_map, bar, h * 64, c[0], c[1], c[2]);
+            ++issued;
           }
         }
         ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-      }
-    }
-    if (!ok && lane == 0) {
-      // drain: give copies already issued a bounded chance to land before the CTA exits
-      for (int e = (n > kStages ? n - kStages : 0); e < n; ++e) {
-        int dummy = 0;
-        ptx::mbar_wait_bounded(ptx::smem_u32(&sh->full[e % kStages]), (e / kStages) & 1, &dummy, 100000000ull);
       }
     }
   } else {
@@ -403,6 +398,14 @@ __global__ void __launch_bounds__(kThreads, 2)
     cluster.sync();  // no CTA leaves while its shared memory is read
   }
   __syncthreads();
+  if (sh->abort_flag && warp == kWarps && lane == 0) {
+    // some wait of this CTA expired, maybe a consumer's after the producer had issued everything: give copies already
+    // issued a bounded chance to land before the CTA exits
+    drain_ring(issued, kStages, [&](int s, uint32_t parity) {
+      int dummy = 0;
+      ptx::mbar_wait_bounded(ptx::smem_u32(&sh->full[s]), parity, &dummy, 100000000ull);
+    });
+  }
   if (tid == 0 && sh->abort_flag && a.status) atomicOr(a.status, CA_STATUS_TIMEOUT);
 }
 

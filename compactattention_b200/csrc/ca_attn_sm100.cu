@@ -26,6 +26,7 @@
 // other tile's MMAs.  Every wait is bounded; on expiry the CTA raises CA_STATUS_TIMEOUT, drains
 // what it issued, frees TMEM and returns.
 #include "ca_attn_shared.cuh"
+#include "ca_ring.cuh"
 
 #include <mutex>
 
@@ -835,10 +836,10 @@ __global__ void __launch_bounds__(kThreads, 1)
   if (sh->abort_flag) {
     if (warp == 9 && lane == 0) {
       // drain: give copies already issued a bounded chance to land before the CTA exits
-      for (int e = (ring_n > kStages ? ring_n - kStages : 0); e < ring_n; ++e) {
+      drain_ring(ring_n, kStages, [&](int s, uint32_t parity) {
         int dummy = 0;
-        ptx::mbar_wait_bounded(ptx::smem_u32(&sh->ring_full[e % kStages]), (e / kStages) & 1, &dummy, 100000000ull);
-      }
+        ptx::mbar_wait_bounded(ptx::smem_u32(&sh->ring_full[s]), parity, &dummy, 100000000ull);
+      });
       for (int tile = 0; tile < 2 && q_issued > 0; ++tile) {
         int dummy = 0;
         ptx::mbar_wait_bounded(ptx::smem_u32(&sh->q_full[tile]), (q_issued - 1) & 1, &dummy, 100000000ull);
