@@ -1,7 +1,8 @@
 // Native form of the tensor-level wrappers in ops.py: checks the tensors, fills the C structs and calls the library,
 // without a Python operation per field.  A wrapper tries its function here first and goes through Python when this
-// one answers None: on anything but the plain case (an argument of another kind, a failed check, an error code), so
-// that checks, messages and every less common form live in ops.py alone.
+// one answers None: on anything but the plain case (an argument of another kind, a failed check), so that checks,
+// messages and every less common form live in ops.py alone.  Once the library has been called there is no second try:
+// an error code is raised as ops.py raises it (the first attempt may have enqueued launches, and has consumed the error).
 //
 // Measured host time per pass, through Python -> here: a decode step 24 -> 10 us, an append 26 -> 8 us, a gate step
 // (prepare, scores and selection, attention) 98 -> 46 us; the decode and append kernels take 8 and 12 us.
@@ -25,10 +26,12 @@ struct Library {
   decltype(&ca_select_union_table) select_union_table;
   decltype(&ca_gate_score_select) gate_score_select;
   decltype(&ca_select_union_scratch_bytes) scratch_bytes;
+  decltype(&ca_last_error) last_error;
 };
 Library lib = {};
 
 struct NotPlain {};  // thrown for everything that ops.py should look at
+struct Failed {};    // thrown with a Python error set
 
 void require(bool ok) {
   if (!ok) throw NotPlain();
@@ -112,10 +115,21 @@ ca_kv_layout layout(Args& a, const at::Tensor** k_out, const at::Tensor** v_out)
   return l;
 }
 
+// Calls the library; an error code becomes the RuntimeError of _lib.check().
+template <typename F>
+void enqueue(const char* what, F&& f) {
+  const int rc = f();
+  if (rc == CA_OK) return;
+  PyErr_Format(PyExc_RuntimeError, "%s failed (code %d): %s", what, rc, lib.last_error());
+  throw Failed();
+}
+
 template <typename F>
 PyObject* guarded(F&& body) {
   try {
     return body();
+  } catch (const Failed&) {
+    return nullptr;
   } catch (const NotPlain&) {
   } catch (const std::exception&) {
     // whatever it was, the same call through Python reports it
@@ -133,6 +147,7 @@ PyObject* bind(PyObject*, PyObject* const* v, Py_ssize_t n) {
     lib.select_union_table = reinterpret_cast<decltype(lib.select_union_table)>(a.integer());
     lib.gate_score_select = reinterpret_cast<decltype(lib.gate_score_select)>(a.integer());
     lib.scratch_bytes = reinterpret_cast<decltype(lib.scratch_bytes)>(a.integer());
+    lib.last_error = reinterpret_cast<decltype(lib.last_error)>(a.integer());
     a.done();
     Py_RETURN_TRUE;
   });
@@ -181,7 +196,7 @@ PyObject* attn_compact(PyObject*, PyObject* const* v, Py_ssize_t n) {
     p.lse = static_cast<float*>(ptr(lse));
     p.status = static_cast<int32_t*>(ptr(status));
     p.workspace = ptr(ws), p.workspace_bytes = ws.nbytes();
-    require(lib.attn_compact(&p, stream) == CA_OK);
+    enqueue("ca_attn_compact", [&] { return lib.attn_compact(&p, stream); });
     return THPVariable_Wrap(out);
   });
 }
@@ -227,7 +242,7 @@ PyObject* rope_append(PyObject*, PyObject* const* v, Py_ssize_t n) {
     p.v = ptr(val), p.v_stride_b = val.stride(0), p.v_stride_t = val.stride(1), p.v_stride_h = val.stride(2);
     p.cos = ptr(cos), p.sin = ptr(sin);
     p.cs_stride_b = cos.size(0) == 1 ? 0 : cos.stride(0), p.cs_stride_t = cos.stride(1);
-    require(lib.rope_append(&p, stream) == CA_OK);
+    enqueue("ca_rope_append", [&] { return lib.rope_append(&p, stream); });
     return THPVariable_Wrap(out);
   });
 }
@@ -272,7 +287,7 @@ PyObject* gate_prepare(PyObject*, PyObject* const* v, Py_ssize_t n) {
     a.done();
     require(q->size(0) == k->size(0) && q->size(1) == k->size(1) && q->size(3) == k->size(3) && q_out->size(3) == k_out->size(3));
     p.B = q->size(0), p.L = q->size(1), p.D = q->size(3), p.C = q_out->size(3);
-    require(lib.gate_prepare(&p, stream) == CA_OK);
+    enqueue("ca_gate_prepare", [&] { return lib.gate_prepare(&p, stream); });
     Py_RETURN_TRUE;
   });
 }
@@ -358,9 +373,12 @@ PyObject* select_union_table(PyObject*, PyObject* const* v, Py_ssize_t n) {
       write_scores = a.i32();
     }
     a.done();
-    const int rc = first_gate ? lib.gate_score_select(&g, &p, &u, ptr(scratch), scratch.nbytes(), write_scores, stream)
-                              : lib.select_union_table(&p, &u, ptr(scratch), scratch.nbytes(), stream);
-    require(rc == CA_OK);
+    if (first_gate) {
+      enqueue("ca_gate_score_select",
+              [&] { return lib.gate_score_select(&g, &p, &u, ptr(scratch), scratch.nbytes(), write_scores, stream); });
+    } else {
+      enqueue("ca_select_union_table", [&] { return lib.select_union_table(&p, &u, ptr(scratch), scratch.nbytes(), stream); });
+    }
     PyObject* res = PyTuple_New(4);
     if (res) {
       for (int i = 0; i < 4; ++i) PyTuple_SET_ITEM(res, i, THPVariable_Wrap(out[i]));

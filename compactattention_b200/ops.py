@@ -38,13 +38,14 @@ def _stream() -> int:
 
 
 _NATIVE_CALLS = ("ca_attn_compact", "ca_rope_append", "ca_gate_prepare", "ca_select_union_table", "ca_gate_score_select",
-                 "ca_select_union_scratch_bytes")
+                 "ca_select_union_scratch_bytes", "ca_last_error")
 _native_lib = None  # the loaded library whose entry points _calls holds
 
 
 def _native():
     """The native wrappers, or None (not built, or the calls are being recorded).  Each of them answers None to
-    anything but the plain, valid case, which the Python form then serves or refuses."""
+    anything but the plain, valid case, which the Python form then serves or refuses; what the library itself refuses
+    it raises."""
     global _native_lib
     if _calls is None or _lib._recording is not None:
         return None

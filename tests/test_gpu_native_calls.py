@@ -142,3 +142,61 @@ def test_gate(ops, monkeypatch, rope):
 
     a, b = _both(ops, monkeypatch, run)
     assert all(torch.equal(x, y) for x, y in zip(a, b))
+
+
+# ---- the wrappers around entry points that only note that they were called ----
+
+FAKE = r"""
+#include <unistd.h>
+static int calls, code, sleep_us;
+void set(int c, int us) { calls = 0, code = c, sleep_us = us; }
+int count(void) { return calls; }
+static int enter(void) { ++calls; usleep(sleep_us); return code; }
+int one(const void* p, void* stream) { return enter(); }
+int select_(const void* p, const void* u, void* s, unsigned long n, void* stream) { return enter(); }
+int gate(const void* g, const void* p, const void* u, void* s, unsigned long n, int w, void* stream) { return enter(); }
+int bytes(int B, int H, int Hkv, int Qb, int Kb, unsigned long* n) { *n = 16; return 0; }
+const char* error(void) { return "as told"; }
+"""
+
+
+@pytest.fixture
+def fake(ops, tmp_path):
+    """The native wrappers bound to FAKE instead of the library, and one plain call through each of them."""
+    import ctypes
+    import subprocess
+    (tmp_path / "fake.c").write_text(FAKE)
+    subprocess.run(["gcc", "-shared", "-fPIC", "-o", str(tmp_path / "fake.so"), str(tmp_path / "fake.c")], check=True)
+    lib = ctypes.CDLL(str(tmp_path / "fake.so"))
+    native = ops._native()
+    q, kv = _randn(1, 2, 4, 128), ops.KvCacheView.from_seq_first(_randn(1, 64, 2, 128), _randn(1, 64, 2, 128))
+    ws = torch.empty(1024, dtype=torch.uint8, device="cuda")
+    score, blocks, weight = torch.zeros((1, 4, 1, 3), device="cuda"), _randn(1, 3, 2, 128), _randn(2, 128, 128)
+    qblk = torch.zeros((1, 1, 4, 128), device="cuda")
+    layout = (kv.k, kv.v, kv.page_stride, kv.token_stride, kv.head_stride, kv.page_size, kv.num_pages, kv.pages_per_seq, 0, None)
+    pick = (0, ws[:64].view(torch.int32), score, 2, ops.RULES["topk"], 2, 64, 256, 0, None, 0, 0.0, 0.0, 1, 0, 1, 0, 0, 0, 0, None, None, None,
+            None, None)
+    cs = _randn(1, 2, 128)
+    calls = {
+        "ca_attn_compact": lambda: native.attn_compact(0, ws, q, *layout, 64, 2, None, None, 64, None, None, None, None),
+        "ca_rope_append": lambda: native.rope_append(0, q, q[:, :, :2], q[:, :, :2], cs, cs, *layout, 0, None, 64, None, None),
+        "ca_gate_prepare": lambda: native.gate_prepare(0, 64, q, 4, None, None, None, qblk, 0, q[:, :, :2], 4, weight, None, None,
+                                                       blocks, 0),
+        "ca_select_union_table": lambda: native.select_union_table(*pick),
+        "ca_gate_score_select": lambda: native.select_union_table(*pick, qblk, blocks, 1.0, 0.0, 1),
+    }
+    address = [ctypes.cast(getattr(lib, n), ctypes.c_void_p).value for n in ("one", "one", "one", "select_", "gate", "bytes", "error")]
+    assert native.bind(*address)
+    yield lib, calls
+    ops._native_lib = None  # the next call binds the library again
+
+
+def test_a_library_error_is_raised_and_the_call_not_made_again(fake):
+    lib, calls = fake
+    for name, call in calls.items():
+        lib.set(0, 0)
+        assert call() is not None and lib.count() == 1, name
+        lib.set(-3, 0)
+        with pytest.raises(RuntimeError, match=rf"{name} failed \(code -3\): as told"):
+            call()
+        assert lib.count() == 1, name
