@@ -115,10 +115,13 @@ ca_kv_layout layout(Args& a, const at::Tensor** k_out, const at::Tensor** v_out)
   return l;
 }
 
-// Calls the library; an error code becomes the RuntimeError of _lib.check().
+// Calls the library, without the GIL: a launch waits while the stream's queue is full, and what it waits for may need
+// the GIL itself (a host callback).  An error code becomes the RuntimeError of _lib.check().
 template <typename F>
 void enqueue(const char* what, F&& f) {
+  PyThreadState* const state = PyEval_SaveThread();
   const int rc = f();
+  PyEval_RestoreThread(state);
   if (rc == CA_OK) return;
   PyErr_Format(PyExc_RuntimeError, "%s failed (code %d): %s", what, rc, lib.last_error());
   throw Failed();

@@ -455,6 +455,8 @@ static int launch(const Args& a, const CUtensorMap& k_map, const CUtensorMap& v_
   attr[1].id = cudaLaunchAttributeClusterDimension;
   attr[1].val.clusterDim.x = cs, attr[1].val.clusterDim.y = 1, attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr, cfg.numAttrs = 2;
+  std::unique_lock<std::mutex> pair(pair_mutex(stream), std::defer_lock);
+  if (a.parts > 1) pair.lock();
   cudaLaunchKernelEx(&cfg, attn_decode_kernel<T>, k_map, v_map, a);
   CA_LAUNCH_CHECK("attn_decode_kernel");
   if (a.parts > 1) {

@@ -1020,6 +1020,11 @@ int encode_kv_maps(const ca_attn_params* p, CUtensorMap* k_map, CUtensorMap* v_m
   return rc != CA_OK ? rc : encode_map(v_map, dt, 4, p->kv.v, dims, strides, box, "v");
 }
 
+std::mutex& pair_mutex(cudaStream_t stream) {
+  static std::mutex mu[64];  // more streams than this share; a collision costs a wait, no more
+  return mu[(reinterpret_cast<uintptr_t>(stream) * 0x9E3779B97F4A7C15ull) >> 58];
+}
+
 static int validate(const ca_attn_params* p) {
   CA_REQUIRE(p != nullptr, "params is null");
   CA_REQUIRE(p->q && p->out && p->kv.k && p->kv.v, "q, out, kv.k and kv.v must be non-null");
@@ -1218,6 +1223,8 @@ int ca_attn_compact(const ca_attn_params* p, ca_stream_t stream_) {
       done[ti][dev.ordinal] = true;
     }
   }
+  std::unique_lock<std::mutex> pair(pair_mutex(stream), std::defer_lock);
+  if (a.split) pair.lock();
   if (p->dtype == CA_DTYPE_BF16) {
     // a programmatic dependent launch: barrier set-up, TMEM allocation and descriptor prefetch overlap the tail of
     // the table builder; the kernel waits (griddepcontrol.wait) before it reads anything from global memory

@@ -1,5 +1,7 @@
 """The native form of the tensor wrappers (``binding/calls.cpp``) against their Python form: the same results bit for
 bit over the options that both take, and the same errors."""
+import time
+
 import pytest
 import torch
 
@@ -200,3 +202,50 @@ def test_a_library_error_is_raised_and_the_call_not_made_again(fake):
         with pytest.raises(RuntimeError, match=rf"{name} failed \(code -3\): as told"):
             call()
         assert lib.count() == 1, name
+
+
+def test_other_threads_run_while_a_call_waits(fake):
+    """A launch may wait for the GPU for long; the wrappers let go of the interpreter meanwhile."""
+    import threading
+    lib, calls = fake
+    for name, call in calls.items():
+        lib.set(0, 300000)
+        go, ticks = threading.Event(), []
+
+        def tick():
+            go.wait()
+            for _ in range(5):  # at the earliest once the call has begun: this thread holds the GIL until then
+                ticks.append(time.monotonic())
+                time.sleep(0.01)
+
+        t = threading.Thread(target=tick)
+        t.start()
+        go.set()
+        call()
+        end = time.monotonic()
+        t.join()
+        assert sum(x < end - 0.05 for x in ticks) == 5, name
+
+
+def test_threads_on_one_stream_keep_their_pieces_apart(ops):
+    """Calls whose units are cut (two launches, one workspace per stream) from several threads on one stream."""
+    import threading
+    cases = []
+    for i, (Q, K) in enumerate(((256, 16384), (1, 60000), (300, 12000), (2, 40000))):
+        q, k, v = _randn(1, Q, 4, 128, seed=i), _randn(1, K, 1, 128, seed=i + 10), _randn(1, K, 1, 128, seed=i + 20)
+        kv = ops.KvCacheView.from_seq_first(k, v)
+        cases.append((q, kv, K, ops.attn_compact(q, kv, K, 1, None, None).clone()))
+    torch.cuda.synchronize()
+    bad = []
+
+    def work(q, kv, K, want):
+        outs = [ops.attn_compact(q, kv, K, 1, None, None) for _ in range(100)]
+        torch.cuda.synchronize()
+        bad.append(sum(not torch.equal(o, want) for o in outs))
+
+    threads = [threading.Thread(target=work, args=c) for c in cases]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert bad == [0] * len(cases)
