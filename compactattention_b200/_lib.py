@@ -264,6 +264,7 @@ CA_POOL_MAX, CA_POOL_MIN, CA_POOL_AVG = 1, 2, 4
 _SIGNATURES = {
     "ca_last_error": (C.c_char_p, []),
     "ca_abi_version": (C.c_int, []),
+    "ca_header_hash": (C.c_char_p, []),
     "ca_launch_count": (C.c_int64, []),
     "ca_set_programmatic_launch": (C.c_int, [C.c_int]),
     "ca_attn_workspace_bytes": (C.c_int, [C.POINTER(AttnParams), C.POINTER(C.c_size_t)]),

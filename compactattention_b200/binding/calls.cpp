@@ -390,8 +390,12 @@ PyObject* select_union_table(PyObject*, PyObject* const* v, Py_ssize_t n) {
   });
 }
 
+#define CA_TEXT_OF(x) #x
+#define CA_TEXT(x) CA_TEXT_OF(x)
+PyObject* header_hash(PyObject*, PyObject* const*, Py_ssize_t) { return PyBytes_FromString(CA_TEXT(CA_HEADER_HASH)); }
+
 #define CALL(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(name)), METH_FASTCALL, nullptr}
-PyMethodDef methods[] = {CALL(bind), CALL(attn_compact), CALL(rope_append), CALL(gate_prepare), CALL(select_union_table),
+PyMethodDef methods[] = {CALL(header_hash), CALL(bind), CALL(attn_compact), CALL(rope_append), CALL(gate_prepare), CALL(select_union_table),
                          {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_calls", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 

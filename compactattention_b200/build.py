@@ -37,13 +37,22 @@ NVCC_FLAGS = [
 ]
 
 
+HEADER = PKG_DIR.parent / "include" / "compactattn_b200.h"
+
+
+def header_define() -> str:
+    """The header's hash, compiled into the library and into the native wrappers: both hold its struct layouts, and
+    ``ops._native()`` lets them work together only where the hashes are the same."""
+    return "CA_HEADER_HASH=" + hashlib.sha256(HEADER.read_bytes()).hexdigest()[:16]
+
+
 def sources() -> list[Path]:
     return sorted(CSRC.glob("*.cu"))
 
 
 def _fingerprint() -> str:
     h = hashlib.sha256()
-    files = sorted(list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cuh")) + [PKG_DIR.parent / "include" / "compactattn_b200.h"])
+    files = sorted(list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cuh")) + [HEADER])
     for f in files:
         h.update(f.name.encode())
         h.update(f.read_bytes())
@@ -59,11 +68,17 @@ def find_nvcc() -> str:
 
 
 def build(force: bool = False, verbose: bool = False) -> Path:
-    """Compile every ``csrc/*.cu`` into one shared library; skip when sources are unchanged."""
+    """Compile every ``csrc/*.cu`` into one shared library, and the native wrappers that go with it; skip what is up to date."""
+    path = _build_library(force, verbose)
+    build_calls(force)
+    return path
+
+
+def _build_library(force: bool, verbose: bool) -> Path:
     fp = _fingerprint()
     if not force and LIB_PATH.exists() and STAMP_PATH.exists() and STAMP_PATH.read_text().strip() == fp:
         return LIB_PATH
-    cmd = [find_nvcc(), *NVCC_FLAGS]
+    cmd = [find_nvcc(), *NVCC_FLAGS, f"-D{header_define()}"]
     if verbose:
         cmd += ["-Xptxas", "-v"]
     cmd += ["-o", str(LIB_PATH), *[str(s) for s in sources()]]
@@ -83,14 +98,14 @@ def build_calls(force: bool = False) -> Path:
     import torch
 
     h = hashlib.sha256()
-    for f in (CALLS_SOURCE, PKG_DIR.parent / "include" / "compactattn_b200.h"):
+    for f in (CALLS_SOURCE, HEADER):
         h.update(f.read_bytes())
     h.update(f"{torch.__version__} {sys.version}".encode())
     fp = h.hexdigest()
     if not force and CALLS_PATH.exists() and CALLS_STAMP_PATH.exists() and CALLS_STAMP_PATH.read_text().strip() == fp:
         return CALLS_PATH
     root = Path(torch.__file__).resolve().parent
-    cmd = [shutil.which("g++") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared",
+    cmd = [shutil.which("g++") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D{header_define()}",
            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f"-I{root / 'include'}",
            f"-I{root / 'include' / 'torch' / 'csrc' / 'api' / 'include'}", f"-I{sysconfig.get_paths()['include']}",
            "-o", str(CALLS_PATH), str(CALLS_SOURCE), f"-L{root / 'lib'}", "-ltorch_python", "-ltorch_cpu", "-lc10"]
@@ -107,7 +122,7 @@ def build_variant(defines: list[str], output: Path, verbose: bool = False) -> Pa
     output = Path(output).resolve()
     if output == LIB_PATH:
         raise ValueError("a development build must not overwrite the product library")
-    cmd = [find_nvcc(), *NVCC_FLAGS, *[f"-D{d}" for d in defines]]
+    cmd = [find_nvcc(), *NVCC_FLAGS, f"-D{header_define()}", *[f"-D{d}" for d in defines]]
     if verbose:
         cmd += ["-Xptxas", "-v"]
     cmd += ["-o", str(output), *[str(s) for s in sources()]]
@@ -132,7 +147,7 @@ def main() -> None:
         print(build_variant(args.define, Path(args.output), verbose=args.verbose))
     else:
         print(build(force=args.force, verbose=args.verbose))
-        print(build_calls(force=args.force))
+        print(CALLS_PATH)
 
 
 if __name__ == "__main__":

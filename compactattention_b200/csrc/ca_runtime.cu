@@ -96,6 +96,10 @@ const char* ca_last_error(void) { return ca::last_error_buffer(); }
 
 int ca_abi_version(void) { return 2; }
 
+#define CA_TEXT_OF(x) #x
+#define CA_TEXT(x) CA_TEXT_OF(x)
+const char* ca_header_hash(void) { return CA_TEXT(CA_HEADER_HASH); }
+
 int ca_chunk_step(const ca_chunk_step_params* p, ca_stream_t stream) {
   using namespace ca;
   CA_REQUIRE(p != nullptr, "params is null");

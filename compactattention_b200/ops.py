@@ -6,6 +6,7 @@ from __future__ import annotations
 
 import ctypes as C
 import math
+import warnings
 from dataclasses import dataclass
 from typing import Optional
 
@@ -46,12 +47,17 @@ def _native():
     """The native wrappers, or None (not built, or the calls are being recorded).  Each of them answers None to
     anything but the plain, valid case, which the Python form then serves or refuses; what the library itself refuses
     it raises."""
-    global _native_lib
+    global _calls, _native_lib
     if _calls is None or _lib._recording is not None:
         return None
     lib = _lib.load()
     if lib is not _native_lib:
-        _calls.bind(*(C.cast(getattr(lib._cdll, name), C.c_void_p).value for name in _NATIVE_CALLS))
+        # compiled apart from the library, against a header of the same structs or not at all
+        if getattr(_calls, "header_hash", bytes)() != lib.ca_header_hash() or \
+                not _calls.bind(*(C.cast(getattr(lib._cdll, name), C.c_void_p).value for name in _NATIVE_CALLS)):
+            warnings.warn("the native wrappers were built for another library and are not used: run python -m compactattention_b200.build")
+            _calls = None
+            return None
         _native_lib = lib
     return _calls
 

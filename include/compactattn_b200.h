@@ -44,6 +44,9 @@ typedef void* ca_stream_t; /* cudaStream_t */
 const char* ca_last_error(void);
 /* ABI version; bumped when a struct below changes (2: ca_select_params.threshold_ptr). */
 int ca_abi_version(void);
+/* Hash of this header as the library was compiled with it.  Code that holds its struct layouts in compiled form
+ * compares it with its own before it calls anything else. */
+const char* ca_header_hash(void);
 /* Number of kernel launches the library has enqueued in this process (all entry points). */
 int64_t ca_launch_count(void);
 /*

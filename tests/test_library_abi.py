@@ -143,3 +143,39 @@ def test_recorded_calls_are_reissued_as_they_were(lib):
         with _lib.record():
             with _lib.record():
                 pass
+
+
+def test_native_wrappers_of_another_header_are_not_used(lib, monkeypatch):
+    """The native wrappers hold the header's struct layouts in compiled form; a build of another header, or one that
+    does not take the library's entry points, is left alone (with a warning) and the Python form serves."""
+    from compactattention_b200 import ops
+
+    assert ops._calls.header_hash() == lib.ca_header_hash() and len(lib.ca_header_hash()) == 16
+    real = ops._calls
+
+    class Stale:
+        def __init__(self, digest, bound):
+            self.header_hash, self.bound = (lambda: digest), bound
+
+        def bind(self, *addresses):
+            assert self.bound is not True, "bound in spite of the hash"
+            return self.bound
+
+    for stale in (Stale(b"0" * 16, True), Stale(lib.ca_header_hash(), None), type("Old", (), {"bind": lambda *a: True})()):
+        monkeypatch.setattr(ops, "_native_lib", None)
+        monkeypatch.setattr(ops, "_calls", stale)
+        with pytest.warns(UserWarning, match="another library"):
+            assert ops._native() is None
+        assert ops._native() is None  # and quietly from then on
+    monkeypatch.setattr(ops, "_calls", real)
+    monkeypatch.setattr(ops, "_native_lib", None)
+    assert ops._native() is real
+
+
+def test_building_the_library_refreshes_the_native_wrappers(lib, monkeypatch, tmp_path):
+    from compactattention_b200 import build
+
+    monkeypatch.setattr(build, "CALLS_PATH", tmp_path / "_calls.so")
+    monkeypatch.setattr(build, "CALLS_STAMP_PATH", tmp_path / "_calls.so.stamp")
+    build.build()
+    assert build.CALLS_PATH.exists() and build.CALLS_STAMP_PATH.exists()
