@@ -1,0 +1,89 @@
+// How long the attention kernel's work units are and whether they are cut across CTAs.  Lengths are in KV steps of 128
+// tokens (about 2.2 us).  Plain arithmetic that compiles for the host too.
+#pragma once
+
+#include <math.h>
+
+#ifdef __CUDACC__
+#define CA_PLAN __host__ __device__ __forceinline__
+#else
+#define CA_PLAN inline
+#endif
+
+namespace ca {
+namespace attn {
+
+constexpr int kSub = 64;  // tokens per TMA box / sub-block
+
+constexpr int kMinSpanSteps = 4;           // shortest span worth a CTA of its own when units are cut
+// What cutting units costs a CTA (partials, the merge), in KV steps of about 2.2 us, with up to ~8 pieces a unit; every
+// further piece costs the merge about kPieceSteps more (4 units of 105 steps in 13 / 21 / 27 / 36 pieces each: 46 / 49 /
+// 53 / 60 us).  Whole against cut, us: 64 units of 1-16 steps 44 / 31, 256 of them 73 / 61, 32 of ~20 37 / 32, 16 units of
+// one KV head at 128K 442 / 77; units of at most 8 steps, one per SM, stay whole (27).
+constexpr float kPieceSteps = 0.45f;
+constexpr int kCutCostSteps = 9;
+// What a unit costs beside its KV steps (Q, the first step's latency, the epilogue), in steps: the CTA with the ~29
+// short units at the head of a causal first chunk of 8192 tokens ran 1.08 M cycles where one with four long units of
+// the same steps ran 0.82 M, about 10,000 cycles a unit, three steps.
+// us with 0 / 2 / 3 / 4: 8192 x 8192, 32/8 heads 605 / 519 / 504 / 508, 4096 x 4096, 28/4 heads 217 / 153 / 142 / 145.
+constexpr int kUnitSteps = 3;
+
+struct Units {
+  int Q, tpt;      // chunk tokens; tokens per 128-row tile
+  int n_pairs;     // tile pairs (units) per row
+  int q_off, spb;  // tokens of the chunk region before the first query; sub-blocks per block
+};
+
+// 64-token sub-blocks of the chunk that tile pair `pair` can see.
+CA_PLAN int chunk_subs(const Units& u, int pair) {
+  int t_last = (2 * pair + 2) * u.tpt - 1;
+  if (t_last > u.Q - 1) t_last = u.Q - 1;
+  return (t_last + u.q_off) / kSub + 1;
+}
+CA_PLAN int unit_iters(const Units& u, int count, int pair) { return (count * u.spb + chunk_subs(u, pair) + 1) >> 1; }
+
+// A unit's length on the line that the spans are cut from: kUnitSteps, then its KV steps.
+CA_PLAN int unit_cost(const Units& u, int count, int pair) { return unit_iters(u, count, pair) + kUnitSteps; }
+
+// Cost of the units of a row that are lane's of 32.  A row's whole cost needs 64 bits: a chunk of a million tokens with
+// 128 heads to a KV head has 2^19 units of up to 2^13 steps.
+CA_PLAN int lane_cost(const Units& u, int count, int lane) {
+  int sum = 0;
+  for (int p = lane; p < u.n_pairs; p += 32) sum += unit_cost(u, count, p);
+  return sum;
+}
+CA_PLAN long long row_cost(const Units& u, int count) {
+  long long sum = 0;
+  for (int lane = 0; lane < 32; ++lane) sum += lane_cost(u, count, lane);
+  return sum;
+}
+
+// Cut or whole: compare what the longest-running of g CTAs has to do.  `total` is the cost of all units, l_min and
+// l_max bound a unit's.  *nc: CTAs that share the line when units are cut.  (Dealing whole units out by their number
+// gave the last CTAs of a causal first chunk twice the mean work: 8192 tokens, 32/8 heads, f16 1045 us, cut by this
+// rule 504 us.)
+CA_PLAN bool units_are_cut(long long total, long long n_units, int l_min, int l_max, int g, int* nc_out) {
+  // Cut: an equal share and the price of cutting.  With little work, fewer CTAs take longer spans (not under
+  // kMinSpanSteps, and no more of them than keep share + merge of nc / n_units pieces smallest); the others leave
+  // at once.
+  long long nc = g;
+  const long long by_work = total / kMinSpanSteps;
+  const long long most = by_work > n_units ? by_work : n_units;
+  if (most < nc) nc = most;
+  const int best = static_cast<int>(sqrtf(static_cast<float>(total) * static_cast<float>(n_units) * (1.0f / kPieceSteps)));
+  if (best < nc) nc = best > 1 ? best : 1;
+  *nc_out = static_cast<int>(nc);
+  const long long t_cut = total / nc + kCutCostSteps;
+  // Whole: the longest unit when every unit has a CTA; equal unit counts when units are about equally long;
+  // otherwise a share that ends up to a unit late.
+  const long long t_whole = n_units <= g ? l_max
+                            : l_min * 10LL >= l_max * 9LL ? ((n_units + g - 1) / g) * l_max
+                                                          : total / g + l_max * 3LL / 4;
+  // Long units: with every SM busy the board holds a lower clock, so a cut that gains little on paper loses
+  // (128 units of 1028 steps on 148 SMs, 2 ms per launch: 1923 us whole, 2028 us cut, 0.88 by this count;
+  // 128 units of 236 steps: 503 us whole, 450 us cut).
+  return t_cut * 100 < t_whole * (total > n_units * 512 ? 85 : 100);
+}
+
+}  // namespace attn
+}  // namespace ca

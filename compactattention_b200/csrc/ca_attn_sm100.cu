@@ -25,6 +25,7 @@
 // MMA order S_A0 S_B0 { PV_A(j) S_A(j+1) PV_B(j) S_B(j+1) } so one tile's softmax overlaps the
 // other tile's MMAs.  Every wait is bounded; on expiry the CTA raises CA_STATUS_TIMEOUT, drains
 // what it issued, frees TMEM and returns.
+#include "ca_attn_plan.cuh"
 #include "ca_attn_shared.cuh"
 #include "ca_ring.cuh"
 
@@ -37,7 +38,6 @@ constexpr int kThreads = 384;  // three warpgroups: softmax A, softmax B, {MMA, 
 constexpr int kTileM = 128;
 constexpr int kTileN = 128;
 constexpr int kHeadDim = 128;
-constexpr int kSub = 64;               // tokens per TMA box / sub-block
 constexpr int kHalfBytes = 128 * 128;  // one [128 rows][64 x 16-bit] swizzled half tile
 constexpr int kTileBytes = 2 * kHalfBytes;
 constexpr int kBoxBytes = kSub * 128;  // one [64 tokens][64 x 16-bit] box
@@ -46,18 +46,6 @@ constexpr int kTmemCols = 512;
 constexpr int kMaxRows = 1024;  // (batch x kv heads) rows per launch
 constexpr int kMaxSegs = 64;    // segments planned per batch
 constexpr float kRescaleThreshold = 8.0f;  // log2 units; lazy accumulator rescale
-constexpr int kMinSpanSteps = 4;           // shortest span worth a CTA of its own when units are cut
-// What cutting units costs a CTA (partials, the merge), in KV steps of about 2.2 us, with up to ~8 pieces a unit; every
-// further piece costs the merge about kPieceSteps more (4 units of 105 steps in 13 / 21 / 27 / 36 pieces each: 46 / 49 /
-// 53 / 60 us).  Whole against cut, us: 64 units of 1-16 steps 44 / 31, 256 of them 73 / 61, 32 of ~20 37 / 32, 16 units of
-// one KV head at 128K 442 / 77; units of at most 8 steps, one per SM, stay whole (27).
-constexpr float kPieceSteps = 0.45f;
-constexpr int kCutCostSteps = 9;
-// What a unit costs beside its KV steps (Q, the first step's latency, the epilogue), in steps: the CTA with the ~29
-// short units at the head of a causal first chunk of 8192 tokens ran 1.08 M cycles where one with four long units of
-// the same steps ran 0.82 M, about 10,000 cycles a unit, three steps.
-// us with 0 / 2 / 3 / 4: 8192 x 8192, 32/8 heads 605 / 519 / 504 / 508, 4096 x 4096, 28/4 heads 217 / 153 / 142 / 145.
-constexpr int kUnitSteps = 3;
 // Measured on B200 (sustained 300-launch loop, 128K context, 20 % density): handing P to the MMA warp
 // in two halves 434 us, in one piece 450 us; packed fp32 pairs for the scale and the row sum 421 us.
 // A polynomial exp2 on the FMA pipe for part of the exponentials (2 / 4 / 6 of every 16 pairs) took
@@ -110,15 +98,11 @@ struct Segment {
   int pad;
 };
 
-struct KernelArgs {
-  int Q, G, Hkv, B;
-  int tpt;          // query tokens per 128-row tile = 128 / G
-  int n_pairs;      // tile pairs per row
+struct KernelArgs : Units {  // q_off: 0 unless a dense launch has an unaligned past
+  int G, Hkv, B;
   int past_blocks;  // Pb
-  int spb;          // 64-token sub-blocks per block
   int block_size;
   int past_tokens;  // tokens before the chunk region (a multiple of block_size)
-  int q_off;        // tokens of the chunk region that precede the first query (0 unless a dense launch has an unaligned past)
   int page_size, pages_per_seq, num_pages;
   const int32_t* block_idx;
   int block_idx_stride;
@@ -186,19 +170,6 @@ __device__ __forceinline__ int visible_cols(int u, int n_sub, int n_past_sub, in
   int lim = t - (u - n_past_sub) * kSub + 1;
   return lim < 0 ? 0 : (lim > kSub ? kSub : lim);
 }
-
-// 64-token sub-blocks of the chunk that tile pair `pair` can see.
-__device__ __forceinline__ int chunk_subs(const KernelArgs& a, int pair) {
-  int t_last = (2 * pair + 2) * a.tpt - 1;
-  if (t_last > a.Q - 1) t_last = a.Q - 1;
-  return (t_last + a.q_off) / kSub + 1;
-}
-__device__ __forceinline__ int unit_iters(const KernelArgs& a, int count, int pair) {
-  return (count * a.spb + chunk_subs(a, pair) + 1) >> 1;
-}
-
-// A unit's length on the line that the spans are cut from: kUnitSteps, then its KV steps.
-__device__ __forceinline__ int unit_cost(const KernelArgs& a, int count, int pair) { return unit_iters(a, count, pair) + kUnitSteps; }
 
 // Finds the unit that holds position x of the line (one warp, all lanes): its row and pair, where it starts.
 __device__ void locate_unit(const KernelArgs& a, const Shared* sh, long long x, int R, int lane, int* row, int* pair, long long* acc) {
@@ -371,12 +342,11 @@ __global__ void __launch_bounds__(kThreads, 1)
         count = count < 0 ? 0 : cap;
       }
     }
-    int tot = 0;
-    for (int p = lane; p < a.n_pairs; p += 32) tot += unit_cost(a, count, p);
-    tot = __reduce_add_sync(0xffffffffu, tot);
+    const unsigned part = lane_cost(a, count, lane);  // their sum may need more than 32 bits
+    const unsigned lo = __reduce_add_sync(0xffffffffu, part & 0xffffu), hi = __reduce_add_sync(0xffffffffu, part >> 16);
     if (lane == 0) {
       sh->row_count[r] = count;
-      sh->row_prefix[r + 1] = tot;  // turned into a prefix below
+      sh->row_prefix[r + 1] = (static_cast<long long>(hi) << 16) + lo;  // turned into a prefix below
     }
   }
   if (tid == 0 && a.descs) {
@@ -403,29 +373,9 @@ __global__ void __launch_bounds__(kThreads, 1)
     const long long total = sh->row_prefix[R];
     const long long c = blockIdx.x;
     const long long n_units = static_cast<long long>(R) * a.n_pairs;
-    // Cut or whole: compare what the longest-running CTA has to do, in KV steps.  (Dealing whole units out by their
-    // number gave the last CTAs of a causal first chunk twice the mean work: 8192 tokens, 32/8 heads, f16 1045 us,
-    // cut by this rule 504 us.)
-    // Cut: an equal share and the price of cutting.  With little work, fewer CTAs take longer spans (not under
-    // kMinSpanSteps, and no more of them than keep share + merge of nc / n_units pieces smallest); the others leave
-    // at once.
-    long long nc = gridDim.x;
-    const long long by_work = total / kMinSpanSteps;
-    const long long most = by_work > n_units ? by_work : n_units;
-    if (most < nc) nc = most;
-    const int best = static_cast<int>(__fsqrt_rn(static_cast<float>(total) * static_cast<float>(n_units) * (1.0f / kPieceSteps)));
-    nc = min(static_cast<int>(nc), max(best, 1));
-    const long long t_cut = total / nc + kCutCostSteps;
-    // Whole: the longest unit when every unit has a CTA; equal unit counts when units are about equally long;
-    // otherwise a share that ends up to a unit late.
     const long long g = gridDim.x;
-    const long long t_whole = n_units <= g ? l_max
-                              : l_min * 10 >= l_max * 9 ? ((n_units + g - 1) / g) * l_max
-                                                        : total / g + l_max * 3 / 4;
-    // Long units: with every SM busy the board holds a lower clock, so a cut that gains little on paper loses
-    // (128 units of 1028 steps on 148 SMs, 2 ms per launch: 1923 us whole, 2028 us cut, 0.88 by this count;
-    // 128 units of 236 steps: 503 us whole, 450 us cut).
-    const bool cut = a.split && t_cut * 100 < t_whole * (total > n_units * 512 ? 85 : 100);
+    int nc = 1;
+    const bool cut = a.split && units_are_cut(total, n_units, l_min, l_max, gridDim.x, &nc);
     int row = 0, pair = 0;
     long long acc = 0;
     if (cut) {
