@@ -1,5 +1,6 @@
 // How long the attention kernel's work units are and whether they are cut across CTAs.  Lengths are in KV steps of 128
-// tokens (about 2.2 us).  Plain arithmetic that compiles for the host too.
+// tokens (about 2.2 us).  Plain arithmetic on both sides: the kernel decides from the rows' counts; the host, where it
+// knows them, by the same rule.
 #pragma once
 
 #include <math.h>
@@ -83,6 +84,22 @@ CA_PLAN bool units_are_cut(long long total, long long n_units, int l_min, int l_
   // (128 units of 1028 steps on 148 SMs, 2 ms per launch: 1923 us whole, 2028 us cut, 0.88 by this count;
   // 128 units of 236 steps: 503 us whole, 450 us cut).
   return t_cut * 100 < t_whole * (total > n_units * 512 ? 85 : 100);
+}
+
+// Whether the kernel may cut, i.e. whether the merge has to be enqueued behind it.  Where nothing is cut the merge
+// still costs 2.8 us (2368 CTAs that look and leave; us with / without: 144 units of 9 steps 28.8 / 26.0, a dense call
+// of 144 units of 18 to 27 steps 50.1 / 47.9).  `cap`: the most past blocks a row can have; `dense`: each row has just these.
+CA_PLAN bool may_be_cut(const Units& u, int rows, int cap, bool dense, int g) {
+  const int longest = unit_cost(u, cap, u.n_pairs - 1);
+  if (longest <= kCutCostSteps + kUnitSteps) return false;
+  const long long n_units = static_cast<long long>(rows) * u.n_pairs;
+  if (dense && u.n_pairs <= 512) {  // all is known; with more units than that a row the merge is nothing
+    int nc;
+    return units_are_cut(rows * row_cost(u, cap), n_units, unit_cost(u, cap, 0), longest, g, &nc);
+  }
+  // One unit to a CTA and hardly a CTA without: only rows of unequal length make a cut pay.  Where the densities of rows
+  // differ by a fifth of the past, it takes units that can have some fifty steps for that to be the price of cutting.
+  return !(n_units <= g && n_units * 10 >= 9LL * g && longest <= 48);
 }
 
 }  // namespace attn

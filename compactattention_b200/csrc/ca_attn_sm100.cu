@@ -1142,12 +1142,9 @@ int ca_attn_compact(const ca_attn_params* p, ca_stream_t stream_) {
   // persistent grid: one CTA per SM, never more CTAs than units when units cannot be cut
   const long long n_units = static_cast<long long>(p->B) * p->Hkv * n_pairs;
   int grid = dev.sm_count;
-  // Units may be cut across CTAs (the kernel decides, from the rows' counts) where the longest possible unit is
-  // longer than what cutting costs; below that the merge launch would only be in the way.
   const int cap_blocks = p->block_idx && p->block_idx_stride < a.past_blocks ? p->block_idx_stride : a.past_blocks;
-  const long long longest = (static_cast<long long>(cap_blocks) * a.spb + (p->Q - 1 + a.q_off) / kSub + 2) / 2;
   const bool can_split = p->workspace != nullptr && p->workspace_bytes >= workspace_bytes_for(grid);
-  a.split = (longest > kCutCostSteps && can_split) ? 1 : 0;
+  a.split = can_split && may_be_cut(a, p->B * p->Hkv, cap_blocks, p->block_idx == nullptr, grid) ? 1 : 0;
   if (!a.split && n_units < grid) grid = static_cast<int>(n_units);
   a.descs = nullptr, a.part_ml = nullptr, a.part_o = nullptr;
   if (a.split) {

@@ -17,6 +17,17 @@ int main(int argc, char** argv) {
   auto n = [&](int i) { return std::atoi(argv[i]); };
   const Units u{n(2), 128 / n(3), (n(2) + 128 / n(3) * 2 - 1) / (128 / n(3) * 2), 0, n(4) / 64};  // Q, G, block size
   if (!std::strcmp(argv[1], "row_cost")) std::printf("%lld\n", row_cost(u, n(5)));
+  if (!std::strcmp(argv[1], "may_be_cut")) std::printf("%d\n", may_be_cut(u, n(6), n(5), n(7), 148));
+  if (!std::strcmp(argv[1], "cut")) {  // rows whose counts follow
+    long long total = 0;
+    int lo = 1 << 30, hi = 0, nc;
+    for (int i = 5; i < argc; ++i) {
+      total += row_cost(u, n(i));
+      if (n(i) < lo) lo = n(i);
+      if (n(i) > hi) hi = n(i);
+    }
+    std::printf("%d\n", units_are_cut(total, static_cast<long long>(argc - 5) * u.n_pairs, unit_cost(u, lo, 0), unit_cost(u, hi, u.n_pairs - 1), 148, &nc));
+  }
   return 0;
 }
 """
@@ -42,3 +53,20 @@ def test_a_rows_cost_is_the_sum_of_its_units(plan, Q, G, bs, count):
         subs = count * (bs // 64) + (min(t + tokens, Q) - 1) // 64 + 1
         want += (subs + 1) // 2 + 3
     assert plan("row_cost", Q, G, bs, count) == want
+
+
+@pytest.mark.parametrize("rows", [1, 2, 8, 37, 72, 148, 150])
+@pytest.mark.parametrize("Q,G", [(64, 4), (700, 7), (1152, 4), (2048, 8)])
+@pytest.mark.parametrize("cap", [0, 20, 64, 300])
+def test_dense_launches_merge_where_units_are_cut(plan, rows, Q, G, cap):
+    assert plan("may_be_cut", Q, G, 64, cap, rows, 1) == plan("cut", Q, G, 64, *[cap] * rows)
+
+
+def test_table_launches_merge_where_units_may_be_cut(plan):
+    assert plan("may_be_cut", 128, 4, 64, 62, 72, 0) == 0   # 144 units of at most 32 steps on 148 CTAs: as before they stay whole
+    assert plan("may_be_cut", 128, 4, 64, 200, 72, 0) == 1  # ... of up to 101 steps: a row may be worth cutting
+    assert plan("may_be_cut", 128, 4, 64, 62, 20, 0) == 1   # 40 units: most CTAs would idle
+    assert plan("may_be_cut", 128, 4, 64, 10, 20, 0) == 0   # at most six steps: nothing to gain
+    # whatever the counts, what may not be cut is dealt out whole by the kernel's own rule or was excluded above
+    for counts in ([10] * 20, [0] * 19 + [10], list(range(11)) * 2):
+        assert plan("cut", 128, 4, 64, *counts) == 0

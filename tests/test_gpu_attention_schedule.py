@@ -73,3 +73,21 @@ def test_rows_of_unequal_length(ops):
             want, _ = _reference(q[0, :, h * 4 : h * 4 + 4], k[0, tok, h : h + 1], v[0, tok, h : h + 1], n * bs)
             err = (out[0, :, h * 4 : h * 4 + 4].float() - want).abs()
             assert err.max().item() < 1e-2 and err.mean().item() < 5e-4, (h, workspace, err.max().item())
+
+
+@pytest.mark.parametrize("B,Q,past,Hq,Hkv,cut", [
+    (9, 128, 1152, 32, 8, False),   # a unit to nearly every SM, all of a length
+    (1, 1152, 0, 32, 8, False),
+    (1, 128, 8192, 32, 8, True),    # few units of 65 steps
+])
+def test_the_merge_is_launched_where_units_are_cut(ops, B, Q, past, Hq, Hkv, cut):
+    from compactattention_b200 import _lib
+    K = past + Q
+    g = torch.Generator(device="cuda").manual_seed(Q)
+    q, k, v = (torch.randn((B, n, h, 128), generator=g, device="cuda", dtype=torch.bfloat16) for n, h in ((Q, Hq), (K, Hkv), (K, Hkv)))
+    kv = ops.KvCacheView.from_seq_first(k, v)
+    before = _lib.launch_count()
+    out = ops.attn_compact(q, kv, K, Hkv, None, None)
+    assert _lib.launch_count() - before == (2 if cut else 1)
+    whole = ops.attn_compact(q, kv, K, Hkv, None, None, use_workspace=False)
+    assert torch.equal(out, whole) != cut  # whole units sum their steps in one order, cut ones in another
