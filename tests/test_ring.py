@@ -45,4 +45,4 @@ def test_only_issued_entries_are_counted():
     text = (CSRC / "ca_attn_decode.cu").read_text()
     loads, count = text.rindex("tma_load_4d("), text.index("++issued;")
     assert text.count("++issued") == 1 and loads < count < loads + 200
-    assert "if (sh->abort_flag && warp == kWarps && lane == 0)" in text[text.rindex("cluster.sync();"):]
+    assert "if (sh->abort_flag) give_up(" in text[text.rindex("cluster.sync();"):]
