@@ -15,6 +15,7 @@
 // Measured on B200 (32/8 heads, bf16; through the 256-row kernel -> here): 8 sequences of 32768 tokens 253 -> 162 us
 // (1.07 GB, 6.64 TB/s), one of 131072 145 -> 85 us, one of 4001 31 -> 8.3 us; one KV head, 131072 tokens 184 -> 19 us;
 // 16 x 8192, 28/4 heads 81 -> 45 us.
+#include "ca_attn_plan.cuh"
 #include "ca_attn_shared.cuh"
 #include "ca_ring.cuh"
 
@@ -28,16 +29,13 @@ namespace decode {
 namespace cg = cooperative_groups;
 
 constexpr int kHeadDim = 128;
-constexpr int kSub = 64;
 constexpr int kRows = 16;  // query rows of one mma tile
 constexpr int kWarps = 4;  // consumer warps; one producer warp follows
 constexpr int kThreads = (kWarps + 1) * 32;
 constexpr int kStages = 3;
 constexpr int kBoxBytes = kSub * 128;       // [64 tokens][64 channels]
 constexpr int kStageBytes = 4 * kBoxBytes;  // K low / high channels, V low / high channels
-constexpr int kMaxCluster = 8;     // 16 leaves SMs without a place for one: 1 x 131072 tokens 106 us, 8 heads; with 8 85 us
-constexpr int kMinSubs = 2;        // sub-blocks a CTA of a cluster should have (1 x 1024: 5.9 us with 4, 5.1 with 2)
-constexpr int kMinSubsPart = 8;    // ... and of a row that is cut over several clusters, which costs the merge launch
+constexpr int kMinSubsPart = 8;    // sub-blocks a CTA should have of a row that is cut over several clusters (the merge launch)
 
 struct Args {
   const void* q;
@@ -503,16 +501,12 @@ int launch_decode(const ca_attn_params* p, const DeviceInfo& dev, cudaStream_t s
   const int R = p->B * p->Hkv;
   const int blocks = a.block_idx ? (a.block_idx_stride < a.past_blocks ? a.block_idx_stride : a.past_blocks) : a.past_blocks;
   const long long most = static_cast<long long>(blocks) * a.spb + (a.Q - 1 + a.q_off) / kSub + 1;  // sub-blocks of a row
-  // A cluster as large as keeps every CTA resident and worth its prologue; rows too few for the GPU even then (one
-  // KV head of a tensor-parallel rank) are cut over several clusters, which costs the merge launch.  Clusters sit
-  // inside a GPC, so not every SM can be part of one: 37 clusters of 8 (every slot of 148 SMs) run in two waves
-  // (131072 tokens of one head: 25 us), 32 in one (19 us).
-  const int places = 2 * dev.sm_count;
-  int cs = 1;
-  while (cs < kMaxCluster && R * (2 * cs) <= places && most >= static_cast<long long>(2 * cs) * kMinSubs) cs *= 2;
+  // Rows too few for the GPU even in clusters of 8 (one KV head of a tensor-parallel rank) are cut over several clusters,
+  // which costs the merge launch (131072 tokens of one head: 19 us).
+  const int cs = decode_cluster_size(R, most, dev.sm_count);
   a.parts = 1;
   if (cs == kMaxCluster) {
-    long long parts = places * 7 / 8 / (R * cs);
+    long long parts = decode_places(cs, dev.sm_count) / (R * cs);
     const long long by_work = most / (cs * kMinSubsPart);
     if (parts > by_work) parts = by_work;
     const size_t per_part = static_cast<size_t>(R) * kRows * (kHeadDim * sizeof(float) + sizeof(float2));

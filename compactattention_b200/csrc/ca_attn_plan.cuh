@@ -1,4 +1,5 @@
-// How long the attention kernel's work units are and whether they are cut across CTAs.  Lengths are in KV steps of 128
+// How the attention kernels share their work out: the lengths of the 256-row kernel's units and whether they are cut
+// across CTAs, and (last) the decode kernel's clusters.  Lengths are in KV steps of 128
 // tokens (about 2.2 us).  Plain arithmetic on both sides: the kernel decides from the rows' counts; the host, where it
 // knows them, by the same rule.
 #pragma once
@@ -100,6 +101,33 @@ CA_PLAN bool may_be_cut(const Units& u, int rows, int cap, bool dense, int g) {
   // One unit to a CTA and hardly a CTA without: only rows of unequal length make a cut pay.  Where the densities of rows
   // differ by a fifth of the past, it takes units that can have some fifty steps for that to be the price of cutting.
   return !(n_units <= g && n_units * 10 >= 9LL * g && longest <= 48);
+}
+
+// ---- decode: CTAs of a cluster that share a row of `subs` 64-token sub-blocks ----
+constexpr int kMaxCluster = 8;  // 16 leaves SMs without a place for one: 1 x 131072 tokens 106 us, 8 heads; with 8 85 us
+constexpr int kMinSubs = 2;     // sub-blocks a CTA of a cluster should have (1 x 1024: 5.9 us with 4, 5.1 with 2)
+constexpr int kCtaSubs = 16;    // what a further wave of CTAs costs beside them, in sub-blocks (12 or less: 4 CTAs for 150 rows, 16: 2 for 304)
+
+// Two CTAs share an SM.  Clusters sit inside a GPC, so clusters of 4 and 8 do not reach every place: 37 of 8 (every slot of
+// 148 SMs) run in two waves, 32 in one.  A cluster of 8 also waits until its places in one GPC are all free, so 8 are
+// only used where all fit at once (75 rows of 16384 tokens: 2 CTAs a row 93 us, 8 100).
+CA_PLAN int decode_places(int cluster, int sms) { return cluster < 4 ? 2 * sms : 2 * sms * 7 / 8; }
+
+// The cluster size with the least work in the longest-lived place: waves of CTAs x what one of them has to do.  us with
+// 1 / 2 / 4 / 8 CTAs a row (* chosen): 32 rows of 32768 tokens 251 / 141 / 87 / 85*, 36 of 32768 247 / 141 / 98* / 111, 74 of
+// 8192 67 / 49* / 62 / 57, 150 of 8192 92* / 114 / 103 / 103, 296 of 8192 177* / 179 / 183 / 193, 304 of 8192 219 / 197* / 186 /
+// 197, 400 of 8192 245 / 233* / 239 / 261, 304 of 500 15* / 21 / 29 / 53.  (As large as keeps all CTAs resident, which it was:
+// 36 rows 111, 74 rows 62, 304 rows 219.)
+CA_PLAN int decode_cluster_size(long long rows, long long subs, int sms) {
+  int best = 1;
+  double best_cost = 0;
+  for (int cs = 1; cs <= kMaxCluster && (cs == 1 || subs >= static_cast<long long>(cs) * kMinSubs); cs *= 2) {
+    const long long places = decode_places(cs, sms);
+    if (cs == kMaxCluster && rows * cs > places) break;
+    const double cost = static_cast<double>((rows * cs + places - 1) / places) * (static_cast<double>(subs) / cs + kCtaSubs);
+    if (cs == 1 || cost < best_cost) best = cs, best_cost = cost;
+  }
+  return best;
 }
 
 }  // namespace attn

@@ -15,6 +15,7 @@ using namespace ca::attn;
 
 int main(int argc, char** argv) {
   auto n = [&](int i) { return std::atoi(argv[i]); };
+  if (!std::strcmp(argv[1], "cluster")) return std::printf("%d\n", decode_cluster_size(n(2), n(3), 148)), 0;
   const Units u{n(2), 128 / n(3), (n(2) + 128 / n(3) * 2 - 1) / (128 / n(3) * 2), 0, n(4) / 64};  // Q, G, block size
   if (!std::strcmp(argv[1], "row_cost")) std::printf("%lld\n", row_cost(u, n(5)));
   if (!std::strcmp(argv[1], "may_be_cut")) std::printf("%d\n", may_be_cut(u, n(6), n(5), n(7), 148));
@@ -70,3 +71,17 @@ def test_table_launches_merge_where_units_may_be_cut(plan):
     # whatever the counts, what may not be cut is dealt out whole by the kernel's own rule or was excluded above
     for counts in ([10] * 20, [0] * 19 + [10], list(range(11)) * 2):
         assert plan("cut", 128, 4, 64, *counts) == 0
+
+
+@pytest.mark.parametrize("rows,subs,want", [
+    (1, 1, 1), (1, 3, 1), (1, 4, 2), (8, 16, 8), (32, 512, 8),
+    (33, 512, 4), (36, 512, 4), (37, 512, 4),  # as clusters of 8 they would take two waves
+    (64, 128, 4), (65, 128, 2), (74, 128, 2), (148, 128, 2), (150, 128, 1), (296, 128, 1),
+    (297, 128, 2), (304, 128, 2), (400, 128, 2), (304, 8, 1), (1024, 2048, 2), (1024, 1, 1),
+])
+def test_decode_cluster_size(plan, rows, subs, want):
+    cs = plan("cluster", rows, subs)
+    waves = {c: -(-rows * c // (296 if c < 4 else 259)) for c in (1, 2, 4, 8) if (c == 1 or subs >= 2 * c) and (c < 8 or rows * 8 <= 259)}
+    cost = {c: w * (subs / c + 16) for c, w in waves.items()}
+    assert cost[cs] == min(cost.values())
+    assert cs == want

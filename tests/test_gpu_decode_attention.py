@@ -30,6 +30,9 @@ def _check(out, lse, want, want_lse):
     (3, 2, 4001, 16, 2, torch.float16),    # a cluster per row
     (40, 1, 300, 32, 8, torch.bfloat16),   # more rows than the GPU holds CTAs
     (1, 1, 20000, 4, 1, torch.bfloat16),   # one row: several clusters and the merge launch
+    (33, 1, 1100, 2, 1, torch.bfloat16),   # too many rows for clusters of 8 at once: of 4
+    (74, 1, 600, 2, 1, torch.float16),     # ... and for clusters of 4: of 2
+    (38, 1, 1500, 16, 8, torch.bfloat16),  # more rows than CTAs: clusters in several waves
 ])
 @pytest.mark.parametrize("workspace", [True, False])
 def test_dense_decode_matches_oracle(ops, B, Q, K, Hq, Hkv, dtype, workspace):
