@@ -94,8 +94,7 @@ struct Segment {
   int row, pair;
   int j0, j1;
   int n_sub, n_past_sub;
-  int slot;  // workspace slot of a partial segment, -1: whole unit, written to the output
-  int pad;
+  int slot;  // workspace slot of a partial segment (the unit's first: odd, others: even), -1: whole unit, written to the output
 };
 
 struct KernelArgs : Units {  // q_off: 0 unless a dense launch has an unaligned past
@@ -816,7 +815,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 }
 
 // Merges the segments of every split unit.  One CTA per (attention CTA, tile, 16-column part);
-// the CTAs whose slot holds the first segment of a unit (j0 == 0) walk the following CTAs' head
+// the CTAs whose odd slot holds the first segment of a unit (j0 == 0) walk the following CTAs' even
 // slots until the unit is complete.  Thread = tile row.  The per-segment weights are computed once
 // and kept in shared memory; the loads of the partial accumulators of different segments are
 // independent, so several are in flight per thread.  (The first form of this kernel, one CTA per
@@ -837,17 +836,12 @@ __global__ void __launch_bounds__(kTileM) attn_combine_kernel(const KernelArgs a
   ptx::grid_dependency_wait();  // nothing in global memory is touched before this
   __shared__ int chain_sh[256];
   __shared__ float w_sh[kCombineMaxChain][kTileM];
-  // blockIdx.x = attention CTA; at most one of its two slots holds the first segment of a cut unit
-  // (slot 0 when a unit starts exactly at the span's start, else slot 1)
+  // blockIdx.x = attention CTA; the first segment of a unit that it cut is in its odd slot
   const int tile = blockIdx.y, part = blockIdx.z, r = threadIdx.x;
-  int slot = 2 * blockIdx.x;
-  SegDesc first = a.descs[slot];
-  if (first.unit < 0 || first.j0 != 0) {
-    slot += 1;
-    first = a.descs[slot];
-    if (first.unit < 0 || first.j0 != 0) return;
-  }
-  // chain of slots: this one, then the head slots (even) of the following CTAs
+  const int slot = 2 * blockIdx.x + 1;
+  const SegDesc first = a.descs[slot];
+  if (first.unit < 0) return;
+  // chain of slots: this one, then the even slots of the following CTAs
   // (CTAs whose span is empty leave their slots unused and are skipped)
   __shared__ int n_sh;
   __shared__ SegDesc cand_sh[2 * kTileM];
