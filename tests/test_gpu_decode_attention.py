@@ -70,6 +70,7 @@ def test_table_decode_matches_oracle(ops, bs, Q, Hq, Hkv):
     q, k, v = (torch.randn((B, n, h, 128), generator=g).to(torch.bfloat16) for n, h in ((Q, Hq), (K, Hkv), (K, Hkv)))
     counts = torch.randint(0, Pb + 1, (B, Hkv), generator=g).to(torch.int32)
     counts[0, 0] = 0  # a row that reads nothing but the chunk
+    counts[1, 0] = Pb // 2  # and one with entries, for the check of clamped ones
     idx = torch.full((B, Hkv, Pb), -1, dtype=torch.int32)
     for b in range(B):
         for h in range(Hkv):
@@ -87,6 +88,5 @@ def test_table_decode_matches_oracle(ops, bs, Q, Hq, Hkv):
     # an entry out of range is clamped and reported, as by the kernel for longer chunks
     bad = idx.clone()
     bad[1, 0, 0] = Pb + 3
-    if int(counts[1, 0]) > 0:
-        ops.attn_compact(q.cuda(), kv, K, Hkv, bad.cuda(), counts.cuda(), block_size=bs, status=status)
-        assert int(status.item()) == 2
+    ops.attn_compact(q.cuda(), kv, K, Hkv, bad.cuda(), counts.cuda(), block_size=bs, status=status)
+    assert int(status.item()) == 2

@@ -15,8 +15,8 @@ def ops():
     return _ops
 
 
-def _both(ops, monkeypatch, fn):
-    """``fn()`` through Python and then through the native form, which must have served it."""
+def _both(ops, monkeypatch, fn, *names):
+    """``fn()`` through Python and then through the native form, which must have served every call, of just these names."""
     with monkeypatch.context() as m:
         m.setattr(ops, "_calls", None)
         python = fn()
@@ -34,7 +34,7 @@ def _both(ops, monkeypatch, fn):
     with monkeypatch.context() as m:
         m.setattr(ops, "_calls", Watch())
         native = fn()
-    assert any(served for _, served in seen), seen
+    assert [name for name, _ in seen] == list(names) and all(served for _, served in seen), seen
     return python, native
 
 
@@ -52,9 +52,9 @@ def test_attention(ops, monkeypatch, dtype, Q):
     counts = torch.tensor([[9, 4], [1, 0]], dtype=torch.int32, device="cuda")
     out = torch.empty((B, Q, Hq, 136), dtype=dtype, device="cuda")[..., :128]
     for kw in ({}, {"softmax_scale": 0.05}, {"out": out}):
-        a, b = _both(ops, monkeypatch, lambda: ops.attn_compact(q, kv, K, Hkv, idx, counts, block_size=bs, **kw).clone())
+        a, b = _both(ops, monkeypatch, lambda: ops.attn_compact(q, kv, K, Hkv, idx, counts, block_size=bs, **kw).clone(), "attn_compact")
         assert torch.equal(a, b)
-        a, b = _both(ops, monkeypatch, lambda: ops.attn_compact(q, kv, K, Hkv, None, None, block_size=bs, **kw).clone())
+        a, b = _both(ops, monkeypatch, lambda: ops.attn_compact(q, kv, K, Hkv, None, None, block_size=bs, **kw).clone(), "attn_compact")
         assert torch.equal(a, b)
     assert ops.attn_compact(q, kv, K, Hkv, None, None, out=out) is out
     with pytest.raises(ValueError, match="share dtype"):
@@ -80,7 +80,7 @@ def test_append(ops, monkeypatch, tables, mean):
         assert n == pos + Q
         return [rot, cache.k_pages, cache.v_pages] + ([mean_k] if mean else [])
 
-    a, b = _both(ops, monkeypatch, run)
+    a, b = _both(ops, monkeypatch, run, "rope_append")
     assert all(torch.equal(x, y) for x, y in zip(a, b))
     cache = PagedKVCache(B, 512, Hkv, 128, torch.device("cuda"))
     with pytest.raises(ValueError, match="do not fit in mean_k"):
@@ -110,7 +110,7 @@ def test_selection(ops, monkeypatch, rule, kw, masked):
         t = ops.select_union_table(score, Kb - Qb, rule, num_kv_heads=Hkv, valid=valid, **kw)
         return [t.block_idx, t.counts, t.cache_seqlens, t.pages_per_row]
 
-    a, b = _both(ops, monkeypatch, run)
+    a, b = _both(ops, monkeypatch, run, "select_union_table")
     assert all(torch.equal(x, y) and x.shape == y.shape for x, y in zip(a, b))
     with pytest.raises(ValueError, match="own key blocks"):
         ops.select_union_table(score, Kb - Qb - 1, rule, num_kv_heads=Hkv, **kw)
@@ -142,7 +142,7 @@ def test_gate(ops, monkeypatch, rope):
         t = st.score_select(rule, Hkv, 64)
         return [st.q_blocks, st.cache.blocks().clone(), st.logits, t.block_idx, t.counts]
 
-    a, b = _both(ops, monkeypatch, run)
+    a, b = _both(ops, monkeypatch, run, "gate_prepare", "select_union_table")
     assert all(torch.equal(x, y) for x, y in zip(a, b))
 
 
