@@ -59,7 +59,7 @@ def parse_args():
     ap.add_argument("--no-sustained", action="store_true", help="skip the seconds-long repeat of the timed loop")
     ap.add_argument("--sustained-seconds", type=float, default=1.0)
     ap.add_argument("--dependent-launch", action="store_true",
-                    help="enqueue programmatic dependent launches instead of plain ones (for A/B timing)")
+                    help="enqueue the launches that are plain otherwise as programmatic dependents too (for A/B timing)")
     ap.add_argument("--no-call-lists", action="store_true",
                     help="fill the parameter blocks of every library call afresh in every step (the tensor-level wrappers) "
                          "instead of re-issuing the calls recorded once per layer state")
@@ -660,7 +660,7 @@ def run_native(args):
                                          if own_exchange is not None else (own_exchange_note or "NCCL"))),
             "l2": f"steps rotate over {len(layers)} layer states ({len(layers) * 2 * K * hkv * D * 2 / 2**30:.1f} GiB of KV), more than L2",
             "launches_per_step": launches / args.steps,
-            "programmatic_dependent_launch": args.dependent_launch,
+            "programmatic_dependent_launch": True,  # the kernels of the path always are, with or without --dependent-launch
             "host_side": ("library calls re-issued from parameter blocks kept per layer state" if not args.no_call_lists
                           else "parameter blocks filled afresh every step by the tensor-level wrappers"),
             "step_us": {k: round(v, 1) for k, v in step_stats.items()},

@@ -12,7 +12,7 @@
 //   scratch in global memory.  Only rows cut over several clusters leave partials in the workspace and are
 //   merged by a dependent launch.
 //
-// Measured on B200 (32/8 heads, bf16; through the 256-row kernel -> here): 8 sequences of 32768 tokens 253 -> 162 us
+// Measured on B200 (32/8 heads, bf16; through the 256-row kernel -> here): 8 sequences of 32768 tokens 267 -> 162 us
 // (1.07 GB, 6.64 TB/s), one of 131072 145 -> 85 us, one of 4001 31 -> 8.3 us; one KV head, 131072 tokens 184 -> 19 us;
 // 16 x 8192, 28/4 heads 81 -> 45 us.
 #include "ca_attn_plan.cuh"

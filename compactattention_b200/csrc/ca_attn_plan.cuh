@@ -81,9 +81,12 @@ CA_PLAN bool units_are_cut(long long total, long long n_units, int l_min, int l_
   const long long t_whole = n_units <= g ? l_max
                             : l_min * 10LL >= l_max * 9LL ? ((n_units + g - 1) / g) * l_max
                                                           : total / g + l_max * 3LL / 4;
-  // Long units: with every SM busy the board holds a lower clock, so a cut that gains little on paper loses
-  // (128 units of 1028 steps on 148 SMs, 2 ms per launch: 1923 us whole, 2028 us cut, 0.88 by this count;
-  // 128 units of 236 steps: 503 us whole, 450 us cut).
+  // Long units: whole, the units of a KV head walk through its K and V side by side and share them in L2; pieces are
+  // at different places, and with every SM busy the board holds a lower clock.  So a cut that gains little on paper loses.
+  // Dense, 32/8 heads, 128 units (0.88 by this count), us cut / whole, one launch at a time; in a loop of a second
+  // (power cap): 121 steps 275 / 285; 272 / 273, 249 steps 503 / 527; 577 / 543, 377 steps 765 / 768; 890 / 810, 505 steps
+  // 1028 / 1000; 1204 / 1078, 761 steps 1563 / 1465; 1819 / 1612, 1017 steps 2092 / 1924; 2430 / 2128.  256 units: 241 steps
+  // 946 / 1023; 1103 / 1075, 497 steps 1989 / 1956; 2284 / 2150.  The line lies where single launches break even.
   return t_cut * 100 < t_whole * (total > n_units * 512 ? 85 : 100);
 }
 

@@ -9,12 +9,14 @@
 // order and are causally masked (bottom-right aligned), which is what
 // compact_attn/kernels/varlen/indexed_dense_prefill_direct_triton.py:155-241 computes.
 //
-// Scheduling: a persistent grid of one CTA per SM.  The KV steps of all units are laid end to end
-// and cut into equal spans, one per CTA ("stream-K"), so the SMs stay balanced whatever the
-// per-row block counts are and however few rows a tensor-parallel rank owns.  A unit that falls
-// entirely inside one span is written straight to the output; a unit cut by a span boundary
-// leaves per-segment partials (unnormalised O, running max, running sum) in the workspace and a
-// small combine kernel merges them.  Without a workspace the spans snap to unit boundaries.
+// Scheduling (ca_attn_plan.cuh): a persistent grid of one CTA per SM.  All units are laid end to end, each as
+// long as its KV steps and what it costs beside them, and the kernel decides from the rows' counts whether this
+// line is cut into equal spans ("stream-K": the SMs stay balanced whatever the per-row block counts are and
+// however few rows a tensor-parallel rank owns) or units stay whole: one per CTA where there are enough CTAs,
+// else those that start inside an equal share of the line.  A unit that falls entirely inside one span is written
+// straight to the output; a unit cut by a span boundary leaves per-segment partials (unnormalised O, running
+// max, running sum) in the workspace and a small combine kernel merges them; it is launched where units may be
+// cut.  Without a workspace units stay whole.
 //
 // Warp roles (384 threads): warps 0-3 softmax of tile A, warps 4-7 softmax of tile B (thread =
 // TMEM lane = tile row), warp 8 lane 0 issues every tcgen05.mma, warp 9 issues every TMA, warps
