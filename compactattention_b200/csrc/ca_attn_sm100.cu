@@ -19,7 +19,7 @@
 // cut.  Without a workspace units stay whole.
 //
 // Warp roles (384 threads): warps 0-3 softmax of tile A, warps 4-7 softmax of tile B (thread =
-// TMEM lane = tile row), warp 8 lane 0 issues every tcgen05.mma, warp 9 issues every TMA, warps
+// TMEM lane = tile row), warp 8 issues every tcgen05.mma, warp 9 issues every TMA, warps
 // 10-11 idle.  The third warpgroup gives its registers to the softmax warpgroups (setmaxnreg),
 // which hold a whole 128-column S row per thread.
 // TMEM (512 columns): S_A | S_B | O_A | O_B, 128 fp32 columns each; P (16-bit) overwrites the
@@ -52,9 +52,6 @@ constexpr float kRescaleThreshold = 8.0f;  // log2 units; lazy accumulator resca
 // A polynomial exp2 on the FMA pipe for part of the exponentials (2 / 4 / 6 of every 16 pairs) took
 // 486 / 499 / 518 us against 485 us without: with the softmax warps of both tiles on every scheduler
 // the added instructions cost more than the MUFU operations they replace, so there is none.
-#ifndef CA_ATTN_P_PARTS
-#define CA_ATTN_P_PARTS 2
-#endif
 #ifndef CA_ATTN_PROFILE
 #define CA_ATTN_PROFILE 0
 #endif
@@ -65,15 +62,14 @@ constexpr float kRescaleThreshold = 8.0f;  // log2 units; lazy accumulator resca
 // shape whose units stay whole); 0 restores a plain launch.
 #define CA_ATTN_MERGE_DEPENDENT 1
 #endif
-static_assert(CA_ATTN_P_PARTS == 1 || CA_ATTN_P_PARTS == 2, "P is handed over in one or two pieces");
-constexpr int kPParts = CA_ATTN_P_PARTS;  // P is handed to the MMA warp in this many pieces so P.V overlaps the softmax
+constexpr int kPParts = 2;  // P is handed to the MMA warp in this many pieces (of 4 MMAs each) so P.V overlaps the softmax
 
 // Optional cycle accounting (development builds only, -DCA_ATTN_PROFILE=1): one thread of each role
 // adds the clock cycles between consecutive marks to per-CTA counters.
 #if CA_ATTN_PROFILE
 __device__ long long g_prof[160][32];
-#define CA_PROF_DECL long long prof_t = clock64(); long long prof_acc[10] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
-#define CA_PROF(i) { const long long prof_n = clock64(); prof_acc[i] += prof_n - prof_t; prof_t = prof_n; }
+#define CA_PROF_DECL unsigned prof_t = clock(); unsigned prof_acc[10] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
+#define CA_PROF(i) { const unsigned prof_n = clock(); prof_acc[i] += prof_n - prof_t; prof_t = prof_n; }
 #define CA_PROF_FLUSH(base) { for (int prof_i = 0; prof_i < 10; ++prof_i) g_prof[blockIdx.x][(base) + prof_i] = prof_acc[prof_i]; }
 #else
 #define CA_PROF_DECL
@@ -516,7 +512,12 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
       } else if (warp == 8) {
         // =============================== MMA issuer ===============================
-        if (lane == 0) {
+        {
+          // The warp stays converged and one elected lane issues.  From a branch that one lane takes, the MMAs and commits of a
+          // KV step took that lane 2850 cycles, 83 % of the step (1024 x 106K keys, 32/8 heads); from the converged warp 1790.
+          // us before / after, single launches and at the power cap: that shape 472 / 458, 535 / 528; 8192 x 8192, f16 538 / 512,
+          // 580 / 562; 8192 x 40K, 28/4 heads 3379 / 3305, 3914 / 3823.
+          const uint32_t lead = ptx::elect_one();
           const uint32_t tS[2] = {tmem + 0u, tmem + 128u};
           const uint32_t tO[2] = {tmem + 256u, tmem + 384u};
           // Descriptors: one base per operand buffer, then a constant added per MMA (the start address
@@ -528,27 +529,18 @@ __global__ void __launch_bounds__(kThreads, 1)
           const uint64_t v_desc0 = ptx::make_smem_desc_sw128(ring_smem, kHalfBytes, 1024);
           const uint32_t idesc_qk = a.idesc_qk, idesc_pv = a.idesc_pv;
           auto issue_s = [&](int tile, int slot) {
-            const uint64_t qd = q_desc[tile];
-            const uint64_t kd = k_desc0 + static_cast<uint64_t>(slot * (kTileBytes >> 4));
-  #pragma unroll
-            for (int k = 0; k < 8; ++k) {
-              const uint64_t o = static_cast<uint64_t>(((k >> 2) * kHalfBytes + (k & 3) * 32) >> 4);
-              ptx::mma_ss(tS[tile], qd + o, kd + o, idesc_qk, k > 0 ? 1u : 0u);
-            }
+            ptx::mma_ss_128x128x128(lead, tS[tile], q_desc[tile], k_desc0 + static_cast<uint64_t>(slot * (kTileBytes >> 4)), idesc_qk);
           };
-          // k-steps [k0, k1) of O += P.V; kN compile-time so the loop unrolls
-          auto issue_pv = [&](int tile, int slot, int k0, int k1, bool first) {
-            const uint64_t vd = v_desc0 + static_cast<uint64_t>(slot * (kTileBytes >> 4));
-  #pragma unroll
-            for (int k = 0; k < 8; ++k) {
-              if (k >= k0 && k < k1) {
-                ptx::mma_ts(tO[tile], tS[tile] + k * 8, vd + static_cast<uint64_t>(k * (2048 >> 4)), idesc_pv,
-                            (first && k == 0) ? 0u : 1u);
-              }
-            }
+          // a half (4 k-steps) of O += P.V
+          auto issue_pv = [&](int tile, int slot, int half, bool first) {
+            ptx::mma_ts_128x128x64(lead, tO[tile], tS[tile] + half * 32, v_desc0 + static_cast<uint64_t>(slot * (kTileBytes >> 4) + half * (8192 >> 4)),
+                                   idesc_pv, (first && half == 0) ? 0u : 1u);
           };
           auto wait = [&](uint64_t* bar, uint32_t parity) {
-            if (ok) ok = ptx::mbar_wait_bounded(ptx::smem_u32(bar), parity, abort_flag, limit);
+            if (ok) {
+              ok = ptx::mbar_wait_bounded(ptx::smem_u32(bar), parity, abort_flag, limit);
+              ok = __all_sync(0xffffffffu, ok);
+            }
             return ok;
           };
           CA_PROF_DECL
@@ -561,11 +553,11 @@ __global__ void __launch_bounds__(kThreads, 1)
               if (!(wait(&sh->q_full[0], qpar) && wait(&sh->q_full[1], qpar) && wait(&sh->ring_full[slot], phase))) break;
               ptx::tc_fence_after();
               issue_s(0, slot);
-              ptx::tc_commit(ptx::smem_u32(&sh->s_full[0]));
+              ptx::tc_commit_if(lead, ptx::smem_u32(&sh->s_full[0]));
               issue_s(1, slot);
-              ptx::tc_commit(ptx::smem_u32(&sh->s_full[1]));
-              ptx::tc_commit(ptx::smem_u32(&sh->ring_empty[slot]));
-              if (sg.j0 + 1 == sg.j1) ptx::tc_commit(ptx::smem_u32(&sh->q_free));
+              ptx::tc_commit_if(lead, ptx::smem_u32(&sh->s_full[1]));
+              ptx::tc_commit_if(lead, ptx::smem_u32(&sh->ring_empty[slot]));
+              if (sg.j0 + 1 == sg.j1) ptx::tc_commit_if(lead, ptx::smem_u32(&sh->q_free));
               ++ring_n;
             }
             for (int j = sg.j0; j < sg.j1 && ok; ++j, ++it) {
@@ -576,7 +568,7 @@ __global__ void __launch_bounds__(kThreads, 1)
               const int k_slot = ring_n % kStages;
               const uint32_t k_phase = (ring_n / kStages) & 1;
               if (more) ++ring_n;
-              const int ksteps = ((2 * j + 1) < sg.n_sub) ? 8 : 4;
+              const bool two = (2 * j + 1) < sg.n_sub;
               const bool first = j == sg.j0;
               CA_PROF(0)
               if (!wait(&sh->ring_full[v_slot], v_phase)) break;
@@ -589,8 +581,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 // the accumulator is free once the previous segment's epilogue has read it
                 if (q == 0 && first && seg_seq > 0 && !wait(&sh->o_free[0], (seg_seq - 1) & 1)) break;
                 ptx::tc_fence_after();
-                const int k1 = (q + 1) * (8 / kPParts);
-                issue_pv(0, v_slot, q * (8 / kPParts), k1 < ksteps ? k1 : ksteps, first);
+                if (q == 0 || two) issue_pv(0, v_slot, q, first);
               }
               if (!ok) break;
               CA_PROF(0)
@@ -599,7 +590,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 CA_PROF(4)
                 ptx::tc_fence_after();
                 issue_s(0, k_slot);
-                ptx::tc_commit(ptx::smem_u32(&sh->s_full[0]));
+                ptx::tc_commit_if(lead, ptx::smem_u32(&sh->s_full[0]));
               }
               for (int q = 0; q < kPParts && ok; ++q) {
                 CA_PROF(0)
@@ -608,23 +599,22 @@ __global__ void __launch_bounds__(kThreads, 1)
                 // the accumulator is free once the previous segment's epilogue has read it
                 if (q == 0 && first && seg_seq > 0 && !wait(&sh->o_free[1], (seg_seq - 1) & 1)) break;
                 ptx::tc_fence_after();
-                const int k1 = (q + 1) * (8 / kPParts);
-                issue_pv(1, v_slot, q * (8 / kPParts), k1 < ksteps ? k1 : ksteps, first);
+                if (q == 0 || two) issue_pv(1, v_slot, q, first);
               }
               if (!ok) break;
-              ptx::tc_commit(ptx::smem_u32(&sh->ring_empty[v_slot]));
+              ptx::tc_commit_if(lead, ptx::smem_u32(&sh->ring_empty[v_slot]));
               if (more) {
                 issue_s(1, k_slot);
-                ptx::tc_commit(ptx::smem_u32(&sh->s_full[1]));
-                ptx::tc_commit(ptx::smem_u32(&sh->ring_empty[k_slot]));
-                if (j + 2 == sg.j1) ptx::tc_commit(ptx::smem_u32(&sh->q_free));
+                ptx::tc_commit_if(lead, ptx::smem_u32(&sh->s_full[1]));
+                ptx::tc_commit_if(lead, ptx::smem_u32(&sh->ring_empty[k_slot]));
+                if (j + 2 == sg.j1) ptx::tc_commit_if(lead, ptx::smem_u32(&sh->q_free));
               }
             }
-            if (ok) ptx::tc_commit(ptx::smem_u32(&sh->o_done));
+            if (ok) ptx::tc_commit_if(lead, ptx::smem_u32(&sh->o_done));
             ++seg_seq;
             CA_PROF(7)
           }
-          CA_PROF_FLUSH(0)
+          if (lane == 0) CA_PROF_FLUSH(0)
         }
       }
       ok = __syncthreads_and(ok ? 1 : 0) != 0;  // all roles finished this batch (or aborted)
@@ -796,9 +786,9 @@ __global__ void __launch_bounds__(kThreads, 1)
         ptx::mbar_wait_bounded(ptx::smem_u32(&sh->q_full[tile]), (q_issued - 1) & 1, &dummy, 100000000ull);
       }
     }
-    if (warp == 8 && lane == 0) {
+    if (warp == 8) {
       // drain the tensor pipe (bounded) before TMEM is released
-      ptx::tc_commit(ptx::smem_u32(&sh->drain));
+      ptx::tc_commit_if(ptx::elect_one(), ptx::smem_u32(&sh->drain));
       int dummy = 0;
       ptx::mbar_wait_bounded(ptx::smem_u32(&sh->drain), 0, &dummy, 100000000ull);
     }

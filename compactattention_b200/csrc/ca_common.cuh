@@ -254,6 +254,51 @@ __device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_
       : "memory");
 }
 
+// One elected lane of a converged warp.
+__device__ __forceinline__ uint32_t elect_one() {
+  uint32_t pred;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(pred));
+  return pred;
+}
+// tcgen05.commit of the lane with lead != 0.
+__device__ __forceinline__ void tc_commit_if(uint32_t lead, uint32_t bar) {
+  asm volatile("{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %1, 0;\n\t@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar), "r"(lead)
+               : "memory");
+}
+// A whole tile product from one lane of a converged warp (lead != 0): D[tmem] = A[smem] * B[smem]^T, 128 x 128 x 128, both operands
+// K-major in two 128-byte-swizzled halves of 16 KB.  One block, so that nothing comes between the instructions.
+__device__ __forceinline__ void mma_ss_128x128x128(uint32_t lead, uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc) {
+  asm volatile(
+      "{\n\t.reg .pred p, t, e;\n\t.reg .b64 da, db;\n\t.reg .b32 a;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\tsetp.eq.b32 t, 0, 0;\n\t"
+      "setp.ne.b32 e, %5, 0;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
+      "add.s64 da, %1, 2;\n\tadd.s64 db, %2, 2;\n\t@e tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, t;\n\t"
+      "add.s64 da, %1, 4;\n\tadd.s64 db, %2, 4;\n\t@e tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, t;\n\t"
+      "add.s64 da, %1, 6;\n\tadd.s64 db, %2, 6;\n\t@e tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, t;\n\t"
+      "add.s64 da, %1, 1024;\n\tadd.s64 db, %2, 1024;\n\t@e tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, t;\n\t"
+      "add.s64 da, %1, 1026;\n\tadd.s64 db, %2, 1026;\n\t@e tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, t;\n\t"
+      "add.s64 da, %1, 1028;\n\tadd.s64 db, %2, 1028;\n\t@e tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, t;\n\t"
+      "add.s64 da, %1, 1030;\n\tadd.s64 db, %2, 1030;\n\t@e tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, t;\n\t"
+      "}" ::"r"(d_tmem),
+      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(0), "r"(lead)
+      : "memory");
+}
+// The same for D[tmem] (+)= A[tmem] * B[smem], 128 x 128 x 64, B MN-major: `accumulate` is the first instruction's.
+__device__ __forceinline__ void mma_ts_128x128x64(uint32_t lead, uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, t, e;\n\t.reg .b64 da, db;\n\t.reg .b32 a;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\tsetp.eq.b32 t, 0, 0;\n\t"
+      "setp.ne.b32 e, %5, 0;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
+      "add.s32 a, %1, 8;\n\tadd.s64 db, %2, 128;\n\t@e tcgen05.mma.cta_group::1.kind::f16 [%0], [a], db, %3, t;\n\t"
+      "add.s32 a, %1, 16;\n\tadd.s64 db, %2, 256;\n\t@e tcgen05.mma.cta_group::1.kind::f16 [%0], [a], db, %3, t;\n\t"
+      "add.s32 a, %1, 24;\n\tadd.s64 db, %2, 384;\n\t@e tcgen05.mma.cta_group::1.kind::f16 [%0], [a], db, %3, t;\n\t"
+      "}" ::"r"(d_tmem),
+      "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(lead)
+      : "memory");
+}
+
 // 32 lanes x 32-bit, 32 consecutive columns: thread i of the warp receives TMEM lane
 // (lane_base + i), registers j = columns col..col+31.
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
