@@ -22,10 +22,13 @@
 // TMEM lane = tile row), warp 8 issues every tcgen05.mma, warp 9 issues every TMA, warps
 // 10-11 idle.  The third warpgroup gives its registers to the softmax warpgroups (setmaxnreg),
 // which hold a whole 128-column S row per thread.
-// TMEM (512 columns): S_A | S_B | O_A | O_B, 128 fp32 columns each; P (16-bit) overwrites the
-// first 64 columns of its S and feeds the P.V MMA straight from TMEM.
-// MMA order S_A0 S_B0 { PV_A(j) S_A(j+1) PV_B(j) S_B(j+1) } so one tile's softmax overlaps the
-// other tile's MMAs.  Every wait is bounded; on expiry the CTA raises CA_STATUS_TIMEOUT, drains
+// TMEM (512 columns): S | P_A | P_B | O_A | O_B, of 128, 64, 64, 128 and 128 columns.  S is one buffer that the tiles
+// take in turn: a softmax warpgroup moves its S into registers at once and gives the buffer back; P (16-bit) has a place
+// of its own and feeds the P.V MMA straight from TMEM.  So S(j+1) does not wait for P.V(j), as it did when each tile had
+// its own S and P lay over it (S -> softmax -> P -> P.V -> next S was one chain of about 3300 cycles a step).
+// MMA order S_A0 S_B0 { S_A(j+1) PV_A(j) S_B(j+1) PV_B(j) }.  With the chain / without, us, single launches and at the
+// power cap: 1024 x 106K keys, 32/8 heads 458 / 435, 528 / 511; 8192 x 8192, f16 512 / 490, 562 / 549; 8192 x 40K,
+// 28/4 heads 3305 / 3191, 3823 / 3684.  Every wait is bounded; on expiry the CTA raises CA_STATUS_TIMEOUT, drains
 // what it issued, frees TMEM and returns.
 #include "ca_attn_plan.cuh"
 #include "ca_attn_shared.cuh"
@@ -112,6 +115,7 @@ struct KernelArgs : Units {  // q_off: 0 unless a dense launch has an unaligned 
   int32_t* status;
   uint32_t idesc_qk, idesc_pv;
   unsigned long long wait_limit_ns;
+  unsigned int wait_limit_us;
   // K/V tensor-map dimensions 1..3 are ordered by ascending stride at encode time; these give the
   // coordinate slot (0..2) of the token, page and head coordinates.
   int slot_tok, slot_page, slot_head;
@@ -122,15 +126,18 @@ struct KernelArgs : Units {  // q_off: 0 unless a dense launch has an unaligned 
   float* part_o;       // [2 * gridDim.x][kPartialOFloats]
 };
 
+struct TileBars {
+  uint64_t s_full, p_part[2], o_free;  // the last piece of P in use completes it
+};
+
 struct Shared {
   uint64_t q_full[2];
   uint64_t q_free;
   uint64_t ring_full[kStages];
   uint64_t ring_empty[kStages];
-  uint64_t s_full[2];
-  uint64_t p_part[2][4];  // [tile][piece]; the last piece in use completes P
-  uint64_t o_done;
-  uint64_t o_free[2];
+  uint64_t s_free;      // the warpgroup whose turn it was has S in registers
+  TileBars tile[2];
+  uint64_t pv_done[2];  // P has been read, O is up to date
   uint64_t drain;
   uint32_t tmem_base;
   int abort_flag;
@@ -240,9 +247,9 @@ __device__ void plan_segments(const KernelArgs& a, Shared* sh, long long span_be
 // P = exp2(S*sc + neg_m) for one 128-column row held in registers: packs to 16 bit, stores the four
 // 32-column chunks over S in TMEM, signals the MMA warp after each of the kPParts pieces.  The scale
 // and the row sum use packed fp32 pairs.  Returns the row sum of P.
-template <typename T>
-__device__ __forceinline__ float exp_pack_store(const uint32_t (&sv)[128], float sc, float neg_m, uint32_t tS,
-                                                uint32_t p_part_bar) {
+template <typename T, typename Free>
+__device__ __forceinline__ float exp_pack_store(const uint32_t (&sv)[128], float sc, float neg_m, uint32_t tP,
+                                                uint32_t p_part_bar, Free p_free) {
   float2 l2 = make_float2(0.f, 0.f);
   const float2 sc2 = make_float2(sc, sc);
   const float2 nm2 = make_float2(neg_m, neg_m);
@@ -258,7 +265,8 @@ __device__ __forceinline__ float exp_pack_store(const uint32_t (&sv)[128], float
       l2 = __fadd2_rn(l2, pr);
       pk[i >> 1] = pack2<T>(pr.x, pr.y);
     }
-    ptx::tmem_st16(tS + c * 16, pk);
+    if (c == 0) p_free();
+    ptx::tmem_st16(tP + c * 16, pk);
     if ((c + 1) % (4 / kPParts) == 0) {
       // a piece of P is in TMEM: let the MMA warp run P.V on it (the last piece completes P)
       ptx::tc_wait_st();
@@ -279,6 +287,8 @@ __global__ void __launch_bounds__(kThreads, 1)
   const uint32_t q_smem = smem_base;                      // Q_A, Q_B
   const uint32_t ring_smem = smem_base + 2 * kTileBytes;  // kStages slots
   Shared* sh = reinterpret_cast<Shared*>(smem_aligned + 2 * kTileBytes + kStages * kTileBytes);
+
+  const uint32_t sh_addr = ring_smem + kStages * kTileBytes;
 
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
@@ -304,15 +314,17 @@ __global__ void __launch_bounds__(kThreads, 1)
       ptx::mbar_init(ptx::smem_u32(&sh->ring_full[s]), 1);
       ptx::mbar_init(ptx::smem_u32(&sh->ring_empty[s]), 1);
     }
-    ptx::mbar_init(ptx::smem_u32(&sh->s_full[0]), 1);
-    ptx::mbar_init(ptx::smem_u32(&sh->s_full[1]), 1);
-    for (int q = 0; q < 4; ++q) {
-      ptx::mbar_init(ptx::smem_u32(&sh->p_part[0][q]), 128);
-      ptx::mbar_init(ptx::smem_u32(&sh->p_part[1][q]), 128);
+    ptx::mbar_init(ptx::smem_u32(&sh->tile[0].s_full), 1);
+    ptx::mbar_init(ptx::smem_u32(&sh->tile[1].s_full), 1);
+    ptx::mbar_init(ptx::smem_u32(&sh->s_free), 128);
+    ptx::mbar_init(ptx::smem_u32(&sh->pv_done[0]), 1);
+    ptx::mbar_init(ptx::smem_u32(&sh->pv_done[1]), 1);
+    for (int q = 0; q < 2; ++q) {
+      ptx::mbar_init(ptx::smem_u32(&sh->tile[0].p_part[q]), 128);
+      ptx::mbar_init(ptx::smem_u32(&sh->tile[1].p_part[q]), 128);
     }
-    ptx::mbar_init(ptx::smem_u32(&sh->o_done), 1);
-    ptx::mbar_init(ptx::smem_u32(&sh->o_free[0]), 128);
-    ptx::mbar_init(ptx::smem_u32(&sh->o_free[1]), 128);
+    ptx::mbar_init(ptx::smem_u32(&sh->tile[0].o_free), 128);
+    ptx::mbar_init(ptx::smem_u32(&sh->tile[1].o_free), 128);
     ptx::mbar_init(ptx::smem_u32(&sh->drain), 1);
     ptx::mbar_fence_init();
     ptx::fence_proxy_async_smem();
@@ -432,6 +444,26 @@ __global__ void __launch_bounds__(kThreads, 1)
         for (int si = 0; si < n_segs && ok; ++si) {
           const Segment sg = sh->segs[si];
           const int b = sg.row / a.Hkv, hkv = sg.row % a.Hkv;
+          int vp0 = 0, vo0 = 0, vp1 = 0, vo1 = 0;
+          bool v_two = true;
+          // one ring entry: the two (or one) 64-token sub-blocks of a K or V tile
+          auto load_tile = [&](const CUtensorMap& map, int p0, int o0, int p1, int o1, bool two) {
+            const int slot = ring_n % kStages;
+            const uint32_t phase = (ring_n / kStages) & 1;
+            if (ok) ok = ptx::mbar_wait_bounded(ptx::smem_u32(&sh->ring_empty[slot]), phase ^ 1u, abort_flag, limit);
+            if (!ok) return;
+            const uint32_t bar = ptx::smem_u32(&sh->ring_full[slot]);
+            const uint32_t dst = ring_smem + slot * kTileBytes;
+            ptx::mbar_expect_tx(bar, two ? 4u * kBoxBytes : 2u * kBoxBytes);
+            int c0[3], c1[3];
+            c0[a.slot_tok] = o0, c0[a.slot_page] = p0, c0[a.slot_head] = hkv / a.kv_head_div;
+            c1[a.slot_tok] = o1, c1[a.slot_page] = p1, c1[a.slot_head] = hkv / a.kv_head_div;
+            for (int h = 0; h < 2; ++h) {
+              ptx::tma_load_4d(dst + h * kHalfBytes, &map, bar, h * 64, c0[0], c0[1], c0[2]);
+              if (two) ptx::tma_load_4d(dst + h * kHalfBytes + kBoxBytes, &map, bar, h * 64, c1[0], c1[1], c1[2]);
+            }
+            ++ring_n;
+          };
           for (int base = 2 * sg.j0; base < 2 * sg.j1 && ok; base += 32) {
             // every lane resolves one sub-block of this batch of 32
             const int u = base + lane;
@@ -470,44 +502,34 @@ __global__ void __launch_bounds__(kThreads, 1)
               const int o1 = __shfl_sync(0xffffffffu, off, 2 * i + 1);
               const bool two = (2 * j + 1) < sg.n_sub;
               if (lane == 0) {
-                for (int kv = 0; kv < 2 && ok; ++kv, ++ring_n) {
-                  const int slot = ring_n % kStages;
-                  const uint32_t phase = (ring_n / kStages) & 1;
-                  ok = ptx::mbar_wait_bounded(ptx::smem_u32(&sh->ring_empty[slot]), phase ^ 1u, abort_flag, limit);
-                  if (!ok) break;
-                  const uint32_t bar = ptx::smem_u32(&sh->ring_full[slot]);
-                  const CUtensorMap* map = kv == 0 ? &k_map : &v_map;
-                  const uint32_t dst = ring_smem + slot * kTileBytes;
-                  ptx::mbar_expect_tx(bar, two ? 4u * kBoxBytes : 2u * kBoxBytes);
-                  int c0[3], c1[3];
-                  c0[a.slot_tok] = o0, c0[a.slot_page] = p0, c0[a.slot_head] = hkv / a.kv_head_div;
-                  c1[a.slot_tok] = o1, c1[a.slot_page] = p1, c1[a.slot_head] = hkv / a.kv_head_div;
-                  for (int h = 0; h < 2; ++h) {
-                    ptx::tma_load_4d(dst + h * kHalfBytes, map, bar, h * 64, c0[0], c0[1], c0[2]);
-                    if (two) ptx::tma_load_4d(dst + h * kHalfBytes + kBoxBytes, map, bar, h * 64, c1[0], c1[1], c1[2]);
-                  }
-                  if (j == sg.j0 && kv == 0) {
-                    // Q follows the segment's first K tile: its memory is free once the last Q.K^T of the previous
-                    // segment has completed, while that segment's last softmax, P.V and epilogue still run
-                    if (seg_seq > 0) ok = ptx::mbar_wait_bounded(ptx::smem_u32(&sh->q_free), (seg_seq - 1) & 1, abort_flag, limit);
-                    if (ok) {
-                      const uint32_t q_bytes = 2u * 128u * static_cast<uint32_t>(a.G * a.tpt);
-                      for (int tile = 0; tile < 2; ++tile) {
-                        const uint32_t q_bar = ptx::smem_u32(&sh->q_full[tile]);
-                        ptx::mbar_expect_tx(q_bar, q_bytes);
-                        for (int h = 0; h < 2; ++h) {
-                          ptx::tma_load_5d(q_smem + tile * kTileBytes + h * kHalfBytes, &q_map, q_bar, h * 64, 0, hkv,
-                                           (2 * sg.pair + tile) * a.tpt, b);
-                        }
+                // in the order in which the issuer takes them: K of this step, V of the one before
+                load_tile(k_map, p0, o0, p1, o1, two);
+                if (j == sg.j0) {
+                  // Q follows the segment's first K tile: its memory is free once the last Q.K^T of the previous
+                  // segment has completed, while that segment's last softmax, P.V and epilogue still run
+                  if (ok && seg_seq > 0) ok = ptx::mbar_wait_bounded(ptx::smem_u32(&sh->q_free), (seg_seq - 1) & 1, abort_flag, limit);
+                  if (ok) {
+                    const uint32_t q_bytes = 2u * 128u * static_cast<uint32_t>(a.G * a.tpt);
+                    for (int tile = 0; tile < 2; ++tile) {
+                      const uint32_t q_bar = ptx::smem_u32(&sh->q_full[tile]);
+                      ptx::mbar_expect_tx(q_bar, q_bytes);
+                      for (int h = 0; h < 2; ++h) {
+                        ptx::tma_load_5d(q_smem + tile * kTileBytes + h * kHalfBytes, &q_map, q_bar, h * 64, 0, hkv,
+                                         (2 * sg.pair + tile) * a.tpt, b);
                       }
-                      ++q_issued;
                     }
+                    ++q_issued;
                   }
+                } else {
+                  load_tile(v_map, vp0, vo0, vp1, vo1, true);  // only a unit's last step can have one sub-block
                 }
+                vp0 = p0, vo0 = o0, vp1 = p1, vo1 = o1, v_two = two;
               }
               ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
             }
           }
+          if (ok && lane == 0) load_tile(v_map, vp0, vo0, vp1, vo1, v_two);
+          ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
           ++seg_seq;
         }
       } else if (warp == 8) {
@@ -518,7 +540,8 @@ __global__ void __launch_bounds__(kThreads, 1)
           // us before / after, single launches and at the power cap: that shape 472 / 458, 535 / 528; 8192 x 8192, f16 538 / 512,
           // 580 / 562; 8192 x 40K, 28/4 heads 3379 / 3305, 3914 / 3823.
           const uint32_t lead = ptx::elect_one();
-          const uint32_t tS[2] = {tmem + 0u, tmem + 128u};
+          const uint32_t tS = tmem;
+          const uint32_t tP[2] = {tmem + 128u, tmem + 192u};
           const uint32_t tO[2] = {tmem + 256u, tmem + 384u};
           // Descriptors: one base per operand buffer, then a constant added per MMA (the start address
           // sits in the low 14 bits in 16-byte units and never carries), so the single issuing thread
@@ -529,11 +552,11 @@ __global__ void __launch_bounds__(kThreads, 1)
           const uint64_t v_desc0 = ptx::make_smem_desc_sw128(ring_smem, kHalfBytes, 1024);
           const uint32_t idesc_qk = a.idesc_qk, idesc_pv = a.idesc_pv;
           auto issue_s = [&](int tile, int slot) {
-            ptx::mma_ss_128x128x128(lead, tS[tile], q_desc[tile], k_desc0 + static_cast<uint64_t>(slot * (kTileBytes >> 4)), idesc_qk);
+            ptx::mma_ss_128x128x128(lead, tS, q_desc[tile], k_desc0 + static_cast<uint64_t>(slot * (kTileBytes >> 4)), idesc_qk);
           };
           // a half (4 k-steps) of O += P.V
           auto issue_pv = [&](int tile, int slot, int half, bool first) {
-            ptx::mma_ts_128x128x64(lead, tO[tile], tS[tile] + half * 32, v_desc0 + static_cast<uint64_t>(slot * (kTileBytes >> 4) + half * (8192 >> 4)),
+            ptx::mma_ts_128x128x64(lead, tO[tile], tP[tile] + half * 32, v_desc0 + static_cast<uint64_t>(slot * (kTileBytes >> 4) + half * (8192 >> 4)),
                                    idesc_pv, (first && half == 0) ? 0u : 1u);
           };
           auto wait = [&](uint64_t* bar, uint32_t parity) {
@@ -544,6 +567,8 @@ __global__ void __launch_bounds__(kThreads, 1)
             return ok;
           };
           CA_PROF_DECL
+          // S is one buffer for both tiles: the next one may go there once the other tile's warpgroup has taken its own
+          auto wait_s_free = [&](uint32_t n) { return n == 0 || wait(&sh->s_free, (n - 1) & 1); };
           for (int si = 0; si < n_segs && ok; ++si) {
             const Segment sg = sh->segs[si];
             const uint32_t qpar = seg_seq & 1;
@@ -551,66 +576,64 @@ __global__ void __launch_bounds__(kThreads, 1)
               const int slot = ring_n % kStages;
               const uint32_t phase = (ring_n / kStages) & 1;
               if (!(wait(&sh->q_full[0], qpar) && wait(&sh->q_full[1], qpar) && wait(&sh->ring_full[slot], phase))) break;
+              if (!wait_s_free(2 * it)) break;
               ptx::tc_fence_after();
               issue_s(0, slot);
-              ptx::tc_commit_if(lead, ptx::smem_u32(&sh->s_full[0]));
+              ptx::tc_commit_if(lead, ptx::smem_u32(&sh->tile[0].s_full));
+              if (!wait_s_free(2 * it + 1)) break;
+              ptx::tc_fence_after();
               issue_s(1, slot);
-              ptx::tc_commit_if(lead, ptx::smem_u32(&sh->s_full[1]));
+              ptx::tc_commit_if(lead, ptx::smem_u32(&sh->tile[1].s_full));
               ptx::tc_commit_if(lead, ptx::smem_u32(&sh->ring_empty[slot]));
               if (sg.j0 + 1 == sg.j1) ptx::tc_commit_if(lead, ptx::smem_u32(&sh->q_free));
               ++ring_n;
             }
             for (int j = sg.j0; j < sg.j1 && ok; ++j, ++it) {
-              const int v_slot = ring_n % kStages;
-              const uint32_t v_phase = (ring_n / kStages) & 1;
-              ++ring_n;
               const bool more = (j + 1) < sg.j1;
               const int k_slot = ring_n % kStages;
               const uint32_t k_phase = (ring_n / kStages) & 1;
               if (more) ++ring_n;
+              const int v_slot = ring_n % kStages;
+              const uint32_t v_phase = (ring_n / kStages) & 1;
+              ++ring_n;
               const bool two = (2 * j + 1) < sg.n_sub;
               const bool first = j == sg.j0;
-              CA_PROF(0)
-              if (!wait(&sh->ring_full[v_slot], v_phase)) break;
-              CA_PROF(1)
-              // P arrives in pieces so P.V starts while the softmax still works
-              for (int q = 0; q < kPParts && ok; ++q) {
-                if (q > 0) CA_PROF(0)
-                if (!wait(&sh->p_part[0][q], it & 1)) break;
-                CA_PROF(2 + q)
-                // the accumulator is free once the previous segment's epilogue has read it
-                if (q == 0 && first && seg_seq > 0 && !wait(&sh->o_free[0], (seg_seq - 1) & 1)) break;
-                ptx::tc_fence_after();
-                if (q == 0 || two) issue_pv(0, v_slot, q, first);
-              }
-              if (!ok) break;
-              CA_PROF(0)
-              if (more) {
-                if (!wait(&sh->ring_full[k_slot], k_phase)) break;
-                CA_PROF(4)
-                ptx::tc_fence_after();
-                issue_s(0, k_slot);
-                ptx::tc_commit_if(lead, ptx::smem_u32(&sh->s_full[0]));
-              }
-              for (int q = 0; q < kPParts && ok; ++q) {
+#pragma unroll
+              for (int tile = 0; tile < 2; ++tile) {
                 CA_PROF(0)
-                if (!wait(&sh->p_part[1][q], it & 1)) break;
-                CA_PROF(5 + q)
-                // the accumulator is free once the previous segment's epilogue has read it
-                if (q == 0 && first && seg_seq > 0 && !wait(&sh->o_free[1], (seg_seq - 1) & 1)) break;
-                ptx::tc_fence_after();
-                if (q == 0 || two) issue_pv(1, v_slot, q, first);
+                if (more) {
+                  if (tile == 0 && !wait(&sh->ring_full[k_slot], k_phase)) break;
+                  CA_PROF(4)
+                  if (!wait_s_free(2 * it + 2 + tile)) break;
+                  CA_PROF(6)
+                  ptx::tc_fence_after();
+                  issue_s(tile, k_slot);
+                  ptx::tc_commit_if(lead, ptx::smem_u32(&sh->tile[tile].s_full));
+                  if (tile == 1) {
+                    ptx::tc_commit_if(lead, ptx::smem_u32(&sh->ring_empty[k_slot]));
+                    if (j + 2 == sg.j1) ptx::tc_commit_if(lead, ptx::smem_u32(&sh->q_free));
+                  }
+                }
+                CA_PROF(0)
+                if (tile == 0 && !wait(&sh->ring_full[v_slot], v_phase)) break;
+                CA_PROF(1)
+                // P arrives in pieces so P.V starts while the softmax still works
+#pragma unroll
+                for (int q = 0; q < kPParts && ok; ++q) {
+                  if (q > 0) CA_PROF(0)
+                  if (!wait(&sh->tile[tile].p_part[q], it & 1)) break;
+                  if (tile == 0) { CA_PROF(2) } else { CA_PROF(5) }
+                  // the accumulator is free once the previous segment's epilogue has read it
+                  if (q == 0 && first && seg_seq > 0 && !wait(&sh->tile[tile].o_free, (seg_seq - 1) & 1)) break;
+                  ptx::tc_fence_after();
+                  if (q == 0 || two) issue_pv(tile, v_slot, q, first);
+                }
+                if (!ok) break;
+                ptx::tc_commit_if(lead, ptx::smem_u32(&sh->pv_done[tile]));
               }
               if (!ok) break;
               ptx::tc_commit_if(lead, ptx::smem_u32(&sh->ring_empty[v_slot]));
-              if (more) {
-                issue_s(1, k_slot);
-                ptx::tc_commit_if(lead, ptx::smem_u32(&sh->s_full[1]));
-                ptx::tc_commit_if(lead, ptx::smem_u32(&sh->ring_empty[k_slot]));
-                if (j + 2 == sg.j1) ptx::tc_commit_if(lead, ptx::smem_u32(&sh->q_free));
-              }
             }
-            if (ok) ptx::tc_commit_if(lead, ptx::smem_u32(&sh->o_done));
             ++seg_seq;
             CA_PROF(7)
           }
@@ -633,8 +656,11 @@ __global__ void __launch_bounds__(kThreads, 1)
         const int tile = warp >> 2;  // 0: A, 1: B
         const int r = tid & 127;     // tile row = TMEM lane
         const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
-        const uint32_t tS = tmem + lane_base + tile * 128u;
+        const uint32_t tS = tmem + lane_base;
+        const uint32_t tP = tmem + lane_base + 128u + tile * 64u;
         const uint32_t tO = tmem + lane_base + 256u + tile * 128u;
+        const uint32_t tile_bars = sh_addr + offsetof(Shared, tile) + tile * sizeof(TileBars);
+        const uint32_t abort_addr = sh_addr + offsetof(Shared, abort_flag);
         const float sc = a.scale_log2;
         uint32_t v[32];
         CA_PROF_DECL
@@ -647,7 +673,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           float l_run = 0.f;
           for (int j = sg.j0; j < sg.j1; ++j, ++it) {
             CA_PROF(0)
-            ok = ptx::mbar_wait_bounded(ptx::smem_u32(&sh->s_full[tile]), it & 1, abort_flag, limit);
+            ok = ptx::mbar_wait_lean(tile_bars + offsetof(TileBars, s_full), it & 1, abort_addr, a.wait_limit_us);
             ok = __all_sync(0xffffffffu, ok);  // keep the warp converged for the collective TMEM ops
             if (!ok) break;
             CA_PROF(1)
@@ -667,6 +693,8 @@ __global__ void __launch_bounds__(kThreads, 1)
             ptx::tmem_ld32_row<64>(tS + 64, sv);
             ptx::tmem_ld32_row<96>(tS + 96, sv);
             ptx::tc_wait_ld();
+            ptx::tc_fence_before();
+            ptx::mbar_arrive(sh_addr + offsetof(Shared, s_free));
             CA_PROF(2)
             if (masked) {
   #pragma unroll
@@ -690,29 +718,40 @@ __global__ void __launch_bounds__(kThreads, 1)
             if (__any_sync(0xffffffffu, need)) {
               const float alpha = need ? (m_run == -INFINITY ? 0.f : ptx::ex2((m_run - m_new) * sc)) : 1.0f;
               if (j > sg.j0) {
-  #pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                  ptx::tmem_ld32(tO + c * 32, v);
+                ptx::mbar_wait_lean(sh_addr + static_cast<uint32_t>(offsetof(Shared, pv_done)) + tile * 8, (it - 1) & 1, abort_addr, a.wait_limit_us);
+                __syncwarp();
+                ptx::tc_fence_after();
+  #pragma unroll 1  // more columns in flight beside the row of S spill (452 us instead of 435)
+                for (int c = 0; c < 8; ++c) {
+                  uint32_t w[16];
+                  ptx::tmem_ld16(tO + c * 16, w);
                   ptx::tc_wait_ld();
   #pragma unroll
-                  for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * alpha);
-                  ptx::tmem_st32(tO + c * 32, v);
+                  for (int i = 0; i < 16; ++i) w[i] = __float_as_uint(__uint_as_float(w[i]) * alpha);
+                  ptx::tmem_st16(tO + c * 16, w);
+                  ptx::tc_wait_st();
                 }
-                ptx::tc_wait_st();
               }
               l_run *= alpha;
               if (need) m_run = m_new;
             }
-            // P = exp2(S*sc - m*sc) -> 16-bit, written over S.  Masked entries are -inf -> 0; a row
+            // P = exp2(S*sc - m*sc) -> 16-bit, where the P before it was.  Masked entries are -inf -> 0; a row
             // that has seen nothing yet (m = -inf) produces zeros.
             const float neg_m = m_run == -INFINITY ? 0.f : -m_run * sc;
-            const uint32_t half_bar = ptx::smem_u32(&sh->p_part[tile][0]);
+            const uint32_t half_bar = tile_bars + offsetof(TileBars, p_part);
             CA_PROF(3)
-            l_run += exp_pack_store<T>(sv, sc, neg_m, tS, half_bar);
+            auto p_free = [&] {  // a fresh barrier counts its phase -1 as complete
+              ok = ptx::mbar_wait_lean(sh_addr + static_cast<uint32_t>(offsetof(Shared, pv_done)) + tile * 8, (it - 1) & 1, abort_addr, a.wait_limit_us);
+              __syncwarp();
+              ptx::tc_fence_after();
+            };
+            l_run += exp_pack_store<T>(sv, sc, neg_m, tP, half_bar, p_free);
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
             CA_PROF(4)
 
           }
-          if (ok) ok = ptx::mbar_wait_bounded(ptx::smem_u32(&sh->o_done), seg_seq & 1, abort_flag, limit);
+          if (ok) ok = ptx::mbar_wait_lean(sh_addr + static_cast<uint32_t>(offsetof(Shared, pv_done)) + tile * 8, (it - 1) & 1, abort_addr, a.wait_limit_us);
           ok = __all_sync(0xffffffffu, ok);
           if (!ok) break;
           ptx::tc_fence_after();
@@ -762,7 +801,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           }
           // the accumulator may be overwritten by the next segment
           ptx::tc_fence_before();
-          ptx::mbar_arrive(ptx::smem_u32(&sh->o_free[tile]));
+          ptx::mbar_arrive(tile_bars + offsetof(TileBars, o_free));
           ++seg_seq;
           CA_PROF(5)
         }
@@ -1120,6 +1159,7 @@ int ca_attn_compact(const ca_attn_params* p, ca_stream_t stream_) {
   a.idesc_qk = ptx::make_idesc_f16(fmt, kTileM, kTileN, 0, 0);
   a.idesc_pv = ptx::make_idesc_f16(fmt, kTileM, kHeadDim, 0, 1);
   a.wait_limit_ns = 2000000000ull;
+  a.wait_limit_us = 2000000u;
   a.kv_head_div = p->kv.head_div > 1 ? p->kv.head_div : 1;
   a.slot_tok = slots[0];
   a.slot_page = slots[1];

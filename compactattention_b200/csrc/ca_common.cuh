@@ -180,6 +180,26 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity,
   }
 }
 
+// The same with few registers, for a wait among many live values: the flag by its shared-memory address, the time in units of
+// 1.024 us.
+__device__ __forceinline__ bool mbar_wait_lean(uint32_t bar, uint32_t parity, uint32_t abort_addr, uint32_t limit_us) {
+  uint32_t t0 = 0;
+  while (true) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (mbar_try_wait(bar, parity)) return true;
+    const uint32_t now = static_cast<uint32_t>(globaltimer_ns() >> 10) | 1u;
+    uint32_t gone;
+    asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(gone) : "r"(abort_addr) : "memory");
+    if (gone) return false;
+    if (t0 == 0) t0 = now;
+    if (now - t0 > limit_us) {
+      asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(abort_addr), "r"(1u) : "memory");
+      return false;
+    }
+  }
+}
+
 __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }

@@ -5,7 +5,7 @@ benchmark's attention shape (chunk 1024 at the end of a 131072-token cache, 32 q
 few CTAs, the clock cycles per 128-token KV step that each role spent between its marks:
 
 * MMA issuer: issuing (which includes being held by the tensor pipe's queue), and the waits for the
-  V tile, the pieces of P of tile A, the K tile, the pieces of P of tile B;
+  V tile, the pieces of P of tile A, the K tile, the pieces of P of tile B, the S buffer;
 * softmax warpgroups: waiting for S, loading S from TMEM, row max + rescale decision,
   exponentials + P store, epilogue.
 
@@ -24,7 +24,7 @@ import torch
 
 from . import _lib, build
 
-MMA_BUCKETS = ["issue", "wait V", "wait pA0", "wait pA1", "wait K", "wait pB0", "wait pB1", "segment end"]
+MMA_BUCKETS = ["issue", "wait V", "wait P of A", "-", "wait K", "wait P of B", "wait for S to be free", "segment end"]
 SOFTMAX_BUCKETS = ["loop", "wait S", "load S", "row max", "exp + store P", "epilogue"]
 
 
