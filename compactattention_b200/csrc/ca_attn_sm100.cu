@@ -731,6 +731,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                   ptx::tmem_st16(tO + c * 16, w);
                   ptx::tc_wait_st();
                 }
+                ptx::tc_wait_st();  // not needed for what it waits for: without it the loop over the steps spills 38 bytes
               }
               l_run *= alpha;
               if (need) m_run = m_new;
