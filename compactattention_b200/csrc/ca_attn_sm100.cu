@@ -846,63 +846,55 @@ __global__ void __launch_bounds__(kThreads, 1)
 #endif
 }
 
-// Merges the segments of every split unit.  One CTA per (attention CTA, tile, 16-column part);
-// the CTAs whose odd slot holds the first segment of a unit (j0 == 0) walk the following CTAs' even
-// slots until the unit is complete.  Thread = tile row.  The per-segment weights are computed once
-// and kept in shared memory; the loads of the partial accumulators of different segments are
-// independent, so several are in flight per thread.  (The first form of this kernel, one CTA per
-// (slot, tile) with the weights recomputed inside the column loop, took 70-80 us for the 16 units
-// of a tensor-parallel rank with one KV head - longer than the attention kernel itself.)
-#ifndef CA_ATTN_COMBINE_PARTS
-#define CA_ATTN_COMBINE_PARTS 8
-#endif
-// Measured (us, attention + merge): 1 KV head 95.3 / 87.4 / 85.4 with 4 / 8 / 16 parts, 4 KV heads
-// 229.5 / 227 / 235, a small shape with whole units 30.4 / 30.8 / 32.9: 8 is the balanced choice.
-constexpr int kCombineParts = CA_ATTN_COMBINE_PARTS;    // column parts per tile (16 must be divisible by it)
-constexpr int kCombineC8 = kHeadDim / 8 / kCombineParts;  // 8-column groups per part
-constexpr int kCombineMaxChain = 32;                    // segments whose weights are cached in shared memory
+// Merges the segments of every split unit.  One CTA per (attention CTA, tile, column part); the CTAs whose odd slot
+// holds the first segment of a unit (j0 == 0) find the unit's others in the even slots of the CTAs that follow.  Thread =
+// tile row.  A chain of memory latencies (descriptors, maxima and sums, accumulators), so all that can be asked for at once is:
+// the descriptors by all threads together, and the accumulators of kBatch segments while the maxima are still on their way.
+// Against one thread walking the descriptors and weights kept in shared memory before any accumulator was loaded, us of attention and
+// merge in a loop: 256 x 8K, 8 KV heads, 27.1 -> 24.9; 1024 x 128K, one KV head 71.4 -> 69.0; 1024 x 32K 227.0 -> 225.9.  Batches of 8
+// in 16 parts where a unit has five pieces or more: 28.5, 70.2.
+constexpr int kMergeAhead = 2 * kTileM;  // following CTAs looked at
+constexpr int kBatch = 4;                // segments in flight
+constexpr int kParts = 8;                // column parts per tile
 
 template <typename T>
 __global__ void __launch_bounds__(kTileM) attn_combine_kernel(const KernelArgs a, int n_slots) {
+  constexpr int kC8 = kHeadDim / 8 / kParts;  // 8-column groups per part
   ptx::grid_launch_dependents();
   ptx::grid_dependency_wait();  // nothing in global memory is touched before this
-  __shared__ int chain_sh[256];
-  __shared__ float w_sh[kCombineMaxChain][kTileM];
+  __shared__ int chain_sh[1 + kMergeAhead];
+  __shared__ uint32_t hit_sh[kMergeAhead / 32];
+  __shared__ int steps_sh[kMergeAhead / 32];
   // blockIdx.x = attention CTA; the first segment of a unit that it cut is in its odd slot
   const int tile = blockIdx.y, part = blockIdx.z, r = threadIdx.x;
   const int slot = 2 * blockIdx.x + 1;
   const SegDesc first = a.descs[slot];
   if (first.unit < 0) return;
-  // chain of slots: this one, then the even slots of the following CTAs
-  // (CTAs whose span is empty leave their slots unused and are skipped)
-  __shared__ int n_sh;
-  __shared__ SegDesc cand_sh[2 * kTileM];
-  // the head slots of the following CTAs, fetched by all threads at once (a one-thread walk over
-  // global memory costs a dependent load per segment)
-  for (int i = r; i < 2 * kTileM; i += kTileM) {
+#pragma unroll
+  for (int i = r; i < kMergeAhead; i += kTileM) {
     const int s = (slot / 2 + 1 + i) * 2;
     SegDesc d;
     d.unit = -1, d.j0 = 0, d.j1 = 0, d.n_iter = 0;
     if (s < n_slots) d = a.descs[s];
-    cand_sh[i] = d;
+    const bool mine = d.unit == first.unit;  // unused slots hold -1
+    const uint32_t hits = __ballot_sync(0xffffffffu, mine);
+    const int steps = __reduce_add_sync(0xffffffffu, mine ? d.j1 - d.j0 : 0);
+    if ((r & 31) == 0) hit_sh[i >> 5] = hits, steps_sh[i >> 5] = steps;
   }
   __syncthreads();
-  if (r == 0) {
-    int n = 0;
-    chain_sh[n++] = slot;
-    int reached = first.j1;
-    for (int i = 0; i < 2 * kTileM && reached < first.n_iter && n < 256; ++i) {
-      const SegDesc d = cand_sh[i];
-      if (d.unit < 0) continue;
-      if (d.unit != first.unit || d.j0 != reached) break;
-      chain_sh[n++] = (slot / 2 + 1 + i) * 2;
-      reached = d.j1;
+  int n = 1, steps = first.j1 - first.j0;
+#pragma unroll
+  for (int w = 0; w < kMergeAhead / 32; ++w) {
+    const uint32_t hits = hit_sh[w];
+    if ((r >> 5) == (w & (kTileM / 32 - 1)) && ((hits >> (r & 31)) & 1u)) {
+      chain_sh[n + __popc(hits & ((1u << (r & 31)) - 1u))] = (slot / 2 + 1 + w * 32 + (r & 31)) * 2;
     }
-    n_sh = reached == first.n_iter ? n : -1;
+    n += __popc(hits);
+    steps += steps_sh[w];
   }
+  if (r == 0) chain_sh[0] = slot;
   __syncthreads();
-  const int n = n_sh;
-  if (n < 0) {
+  if (first.j0 != 0 || steps != first.n_iter) {
     if (r == 0 && part == 0 && a.status) atomicOr(a.status, CA_STATUS_BAD_INDEX);
     return;
   }
@@ -912,50 +904,62 @@ __global__ void __launch_bounds__(kTileM) attn_combine_kernel(const KernelArgs a
   const int g = r % a.G;
   const bool live = (r < a.tpt * a.G) && (t < a.Q);
   const float sc = a.scale_log2;
-  auto ml_of = [&](int i) { return a.part_ml + static_cast<long long>(chain_sh[i]) * kPartialMLFloats + (tile * kTileM + r) * 2; };
+  float4 x[kBatch][2];
+  auto load_o = [&](int i0, int cc) {
+#pragma unroll
+    for (int k = 0; k < kBatch; ++k) {
+      if (i0 + k >= n) break;
+      const float* po = a.part_o + static_cast<long long>(chain_sh[i0 + k]) * kPartialOFloats + tile * (kTileM * kHeadDim);
+      const int c4 = 2 * (part * kC8 + cc);
+      x[k][0] = *reinterpret_cast<const float4*>(po + (static_cast<long long>(c4) * kTileM + r) * 4);
+      x[k][1] = *reinterpret_cast<const float4*>(po + (static_cast<long long>(c4 + 1) * kTileM + r) * 4);
+    }
+  };
+  auto ml_of = [&](int i) {
+    return __ldg(reinterpret_cast<const float2*>(a.part_ml + static_cast<long long>(chain_sh[i]) * kPartialMLFloats + (tile * kTileM + r) * 2));
+  };
+  load_o(0, 0);
   float m = -INFINITY;
-#pragma unroll 8
-  for (int i = 0; i < n; ++i) m = fmaxf(m, __ldg(ml_of(i)));
+#pragma unroll kBatch
+  for (int i = 0; i < n; ++i) m = fmaxf(m, ml_of(i).x);
   float l = 0.f;
-#pragma unroll 8
-  for (int i = 0; i < n; ++i) {
-    const float2 ml = __ldg(reinterpret_cast<const float2*>(ml_of(i)));
-    const float w = ml.x == -INFINITY ? 0.f : ptx::ex2((ml.x - m) * sc);
-    if (i < kCombineMaxChain) w_sh[i][r] = w;
-    l += ml.y * w;
+  float acc[kC8][8] = {};
+  for (int i0 = 0; i0 < n; i0 += kBatch) {
+    float w[kBatch];
+#pragma unroll
+    for (int k = 0; k < kBatch; ++k) {
+      if (i0 + k >= n) break;
+      const float2 ml = ml_of(i0 + k);
+      w[k] = ml.x == -INFINITY ? 0.f : ptx::ex2((ml.x - m) * sc);
+      l += ml.y * w[k];
+    }
+#pragma unroll
+    for (int cc = 0; cc < kC8; ++cc) {
+      if (i0 > 0 || cc > 0) load_o(i0, cc);
+#pragma unroll
+      for (int k = 0; k < kBatch; ++k) {
+        if (i0 + k >= n) break;
+        acc[cc][0] += w[k] * x[k][0].x, acc[cc][1] += w[k] * x[k][0].y, acc[cc][2] += w[k] * x[k][0].z, acc[cc][3] += w[k] * x[k][0].w;
+        acc[cc][4] += w[k] * x[k][1].x, acc[cc][5] += w[k] * x[k][1].y, acc[cc][6] += w[k] * x[k][1].z, acc[cc][7] += w[k] * x[k][1].w;
+      }
+    }
   }
   const float inv_l = 1.0f / l;
-  auto weight = [&](int i) {
-    if (i < kCombineMaxChain) return w_sh[i][r];  // written by this very thread
-    const float ms = ml_of(i)[0];
-    return ms == -INFINITY ? 0.f : ptx::ex2((ms - m) * sc);
-  };
   T* orow = reinterpret_cast<T*>(a.out) + b * a.o_stride_b + static_cast<long long>(t) * a.o_stride_t +
             static_cast<long long>(hkv * a.G + g) * a.o_stride_h;
+  if (live) {
 #pragma unroll
-  for (int cc = 0; cc < kCombineC8; ++cc) {
-    const int c8 = part * kCombineC8 + cc;
-    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-#pragma unroll 4
-    for (int i = 0; i < n; ++i) {
-      const float w = weight(i);
-      const float* po = a.part_o + static_cast<long long>(chain_sh[i]) * kPartialOFloats + tile * (kTileM * kHeadDim);
-      const float4 x0 = *reinterpret_cast<const float4*>(po + (static_cast<long long>(2 * c8) * kTileM + r) * 4);
-      const float4 x1 = *reinterpret_cast<const float4*>(po + (static_cast<long long>(2 * c8 + 1) * kTileM + r) * 4);
-      acc[0] += w * x0.x, acc[1] += w * x0.y, acc[2] += w * x0.z, acc[3] += w * x0.w;
-      acc[4] += w * x1.x, acc[5] += w * x1.y, acc[6] += w * x1.z, acc[7] += w * x1.w;
-    }
-    if (live) {
+    for (int cc = 0; cc < kC8; ++cc) {
       uint4 w;
-      w.x = pack2<T>(acc[0] * inv_l, acc[1] * inv_l);
-      w.y = pack2<T>(acc[2] * inv_l, acc[3] * inv_l);
-      w.z = pack2<T>(acc[4] * inv_l, acc[5] * inv_l);
-      w.w = pack2<T>(acc[6] * inv_l, acc[7] * inv_l);
-      *reinterpret_cast<uint4*>(orow + c8 * 8) = w;
+      w.x = pack2<T>(acc[cc][0] * inv_l, acc[cc][1] * inv_l);
+      w.y = pack2<T>(acc[cc][2] * inv_l, acc[cc][3] * inv_l);
+      w.z = pack2<T>(acc[cc][4] * inv_l, acc[cc][5] * inv_l);
+      w.w = pack2<T>(acc[cc][6] * inv_l, acc[cc][7] * inv_l);
+      *reinterpret_cast<uint4*>(orow + (part * kC8 + cc) * 8) = w;
     }
-  }
-  if (live && part == 0 && a.lse) {
-    a.lse[(static_cast<long long>(b) * (a.Hkv * a.G) + hkv * a.G + g) * a.Q + t] = 0.6931471805599453f * (m * sc + log2f(l));
+    if (part == 0 && a.lse) {
+      a.lse[(static_cast<long long>(b) * (a.Hkv * a.G) + hkv * a.G + g) * a.Q + t] = 0.6931471805599453f * (m * sc + log2f(l));
+    }
   }
 }
 
@@ -1209,9 +1213,9 @@ int ca_attn_compact(const ca_attn_params* p, ca_stream_t stream_) {
   CA_LAUNCH_CHECK("attn_compact_kernel");
   if (a.split) {
     if (p->dtype == CA_DTYPE_BF16) {
-      launch_kernel_as(CA_ATTN_MERGE_DEPENDENT != 0, attn_combine_kernel<__nv_bfloat16>, dim3(grid, 2, kCombineParts), dim3(kTileM), 0, stream, a, 2 * grid);
+      launch_kernel_as(CA_ATTN_MERGE_DEPENDENT != 0, attn_combine_kernel<__nv_bfloat16>, dim3(grid, 2, kParts), dim3(kTileM), 0, stream, a, 2 * grid);
     } else {
-      launch_kernel_as(CA_ATTN_MERGE_DEPENDENT != 0, attn_combine_kernel<__half>, dim3(grid, 2, kCombineParts), dim3(kTileM), 0, stream, a, 2 * grid);
+      launch_kernel_as(CA_ATTN_MERGE_DEPENDENT != 0, attn_combine_kernel<__half>, dim3(grid, 2, kParts), dim3(kTileM), 0, stream, a, 2 * grid);
     }
     CA_LAUNCH_CHECK("attn_combine_kernel");
   }
