@@ -515,6 +515,193 @@ __device__ void select_row(const RowArgs& a, const Team& tm, TeamShared* ts, uns
   }
 }
 
+// A row of at most 2048 contiguous f32 scores under the threshold or the top-k rule, without leaving registers: a thread
+// owns eight consecutive entries and packs their bits itself.  The general form above writes scores and flags to shared memory and
+// reads them back, and its radix passes queue on the few bins that a row's exponents fall into; a row is bound by instruction issue
+// and by the number of barriers, and this has four for top-k and none for a threshold.
+// us a pass, before / after: 2 x 1000 of 64K, 28/4 heads, threshold 300 / 292.5; one KV head of 128K, top-k 93.2 / 90.3; 8 KV heads
+// 541.5 / 536.6.  The row-max rule on raw scores stays in the general form: with its 256 blocks a row a single warp would have all
+// the exponentials (1024 of 32K, 173.9 / 176.9).
+// Top-k: 256 bins over [lowest, highest] score (x -> bin is monotone, equal scores share a bin), the entries of the bin that holds
+// the k-th largest are ranked against each other by (key, lower index), as the general form orders them.  Returns false, with
+// nothing written, where that does not hold or pay: a visible score that is not finite, more than kFastTies entries in that bin.
+constexpr int kFastPer = 8;
+constexpr int kFastTies = 512;
+struct FastShared {
+  float lo[kRowThreads / 32], hi[kRowThreads / 32];
+  int hist[256];
+  int n_valid, n_cand, odd;
+  uint32_t kth_key;
+  int kth_j;
+  uint32_t cand_key[kFastTies];
+  int cand_j[kFastTies];
+};
+
+__device__ __forceinline__ bool fast_applies(const RowArgs& a) {
+  return a.Kb <= kRowThreads * kFastPer && a.score_dtype == CA_DTYPE_F32 && a.s_k == 1 && !a.softmax && !a.prob_out && !a.score_max &&
+         (a.rule == CA_RULE_THRESHOLD || a.rule == CA_RULE_TOPK);
+}
+
+// Loads the eight floats at p[0..7], those with j0 + u >= n as 0.
+__device__ __forceinline__ void load8(const float* p, int j0, int n, float (&x)[kFastPer]) {
+  if (j0 + kFastPer <= n && (reinterpret_cast<uintptr_t>(p) & 15) == 0) {
+    const float4 v0 = __ldg(reinterpret_cast<const float4*>(p)), v1 = __ldg(reinterpret_cast<const float4*>(p) + 1);
+    x[0] = v0.x, x[1] = v0.y, x[2] = v0.z, x[3] = v0.w, x[4] = v1.x, x[5] = v1.y, x[6] = v1.z, x[7] = v1.w;
+  } else {
+#pragma unroll
+    for (int u = 0; u < kFastPer; ++u) x[u] = j0 + u < n ? __ldg(p + u) : 0.f;
+  }
+}
+
+__device__ bool select_row_fast(const RowArgs& a, FastShared* fs, TeamShared* ts, int b, int h, int i) {
+  const Team tm{static_cast<int>(threadIdx.x), kRowThreads, 0};
+  const int tid = tm.tid, lane = tid & 31;
+  const int j0 = tid * kFastPer;
+  const int diag = a.Pb + i;
+  const long long s_off = b * a.s_b + h * a.s_h + i * a.s_q + j0;
+  float x[kFastPer];
+  load8(reinterpret_cast<const float*>(a.score) + s_off, j0, a.Kb, x);
+  uint32_t ok = 0;  // visible entries
+  if (a.valid) {
+    const uint8_t* v = a.valid + b * a.v_b + h * a.v_h + i * a.v_q;
+    if (a.v_k == 1 && j0 + kFastPer <= a.Kb && (reinterpret_cast<uintptr_t>(v + j0) & 7) == 0) {
+      const uint2 w = __ldg(reinterpret_cast<const uint2*>(v + j0));
+#pragma unroll
+      for (int u = 0; u < kFastPer; ++u) ok |= (((u < 4 ? w.x : w.y) >> (8 * (u & 3))) & 0xffu) != 0 ? 1u << u : 0u;
+    } else {
+#pragma unroll
+      for (int u = 0; u < kFastPer; ++u)
+        if (j0 + u < a.Kb && v[(j0 + u) * a.v_k] != 0) ok |= 1u << u;
+    }
+  } else {
+    const int last = diag < a.Kb - 1 ? diag : a.Kb - 1;
+    const int c = last - j0 + 1;
+    ok = c <= 0 ? 0u : c >= kFastPer ? 0xffu : (1u << c) - 1u;
+  }
+  uint32_t keep = 0;
+  if (a.rule == CA_RULE_THRESHOLD) {
+    const float thr = a.threshold_ptr ? __ldg(a.threshold_ptr + b * a.threshold_stride) : a.threshold;
+#pragma unroll
+    for (int u = 0; u < kFastPer; ++u) keep |= (x[u] > thr ? 1u : 0u) << u;
+  } else {
+    float lo = INFINITY, hi = -INFINITY;
+    bool odd = false;
+#pragma unroll
+    for (int u = 0; u < kFastPer; ++u) {
+      if ((ok >> u) & 1u) {
+        lo = fminf(lo, x[u]), hi = fmaxf(hi, x[u]);
+        odd |= !(fabsf(x[u]) < INFINITY);
+      }
+    }
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) {
+      lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, d));
+      hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, d));
+    }
+    const int cnt = __reduce_add_sync(0xffffffffu, __popc(ok));
+    fs->hist[tid] = 0;
+    if (tid == 0) fs->n_cand = 0;
+    if (lane == 0) fs->lo[tid >> 5] = lo, fs->hi[tid >> 5] = hi, ts->warp_sums[tid >> 5] = cnt;
+    if (__syncthreads_or(odd ? 1 : 0)) return false;
+    int n_valid = 0;
+#pragma unroll
+    for (int w = 0; w < kRowThreads / 32; ++w) {
+      lo = fminf(lo, fs->lo[w]), hi = fmaxf(hi, fs->hi[w]);
+      n_valid += ts->warp_sums[w];
+    }
+    if (!a.valid) n_valid = diag + 1 < a.Kb ? diag + 1 : a.Kb;
+    int k = a.topk_k > 0 ? a.topk_k
+                         : static_cast<int>((static_cast<long long>(a.topk_num) * n_valid + a.topk_den / 2) / a.topk_den);
+    if (k < 1) k = 1;
+    if (k > n_valid) k = n_valid;
+    if (k >= n_valid) {
+      keep = ok;  // all of them (none, if none is visible)
+    } else {
+      const float scale = 255.9f / (hi - lo);
+      int bin[kFastPer];
+#pragma unroll
+      for (int u = 0; u < kFastPer; ++u) {
+        // 0 .. 255; a NaN (equal scores and an infinite scale) is 0
+        bin[u] = ((ok >> u) & 1u) ? min(255, max(0, __float2int_rz((x[u] - lo) * scale))) : -1;
+        if (bin[u] >= 0) atomicAdd(&fs->hist[bin[u]], 1);
+      }
+      __syncthreads();
+      // every warp finds the bin that holds the k-th largest: lane l owns bins 255-8l .. 248-8l
+      int mine = 0, c[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) c[u] = fs->hist[255 - 8 * lane - u], mine += c[u];
+      int inc = mine;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const int nb = __shfl_up_sync(0xffffffffu, inc, d);
+        if (lane >= d) inc += nb;
+      }
+      const int owner = __ffs(__ballot_sync(0xffffffffu, inc >= k)) - 1;
+      int left = k - (inc - mine), cut = 0, at = 0;
+      bool found = false;
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        if (!found) {
+          if (c[u] >= left) found = true, cut = 255 - 8 * lane - u, at = c[u];
+          else left -= c[u];
+        }
+      }
+      cut = __shfl_sync(0xffffffffu, cut, owner);   // the bin
+      left = __shfl_sync(0xffffffffu, left, owner);  // entries wanted of it
+      at = __shfl_sync(0xffffffffu, at, owner);      // entries in it
+      if (at > kFastTies) return false;
+      uint32_t in_cut = 0;
+#pragma unroll
+      for (int u = 0; u < kFastPer; ++u) {
+        if (bin[u] > cut) keep |= 1u << u;
+        if (bin[u] == cut) in_cut |= 1u << u;
+      }
+      if (left == at) {
+        keep |= in_cut;
+      } else {
+#pragma unroll
+        for (int u = 0; u < kFastPer; ++u) {
+          if ((in_cut >> u) & 1u) {
+            const int o = atomicAdd(&fs->n_cand, 1);
+            fs->cand_key[o] = order_key(x[u]), fs->cand_j[o] = j0 + u;
+          }
+        }
+        __syncthreads();
+        for (int q = tid; q < at; q += kRowThreads) {
+          const uint32_t key = fs->cand_key[q];
+          const int j = fs->cand_j[q];
+          int before = 0;
+          for (int o = 0; o < at; ++o) {
+            const uint32_t other = fs->cand_key[o];
+            before += other > key || (other == key && fs->cand_j[o] < j);
+          }
+          if (before == left - 1) fs->kth_key = key, fs->kth_j = j;  // just one entry has this place
+        }
+        __syncthreads();
+        const uint32_t kth_key = fs->kth_key;
+        const int kth_j = fs->kth_j;
+#pragma unroll
+        for (int u = 0; u < kFastPer; ++u) {
+          const uint32_t key = order_key(x[u]);
+          if (((in_cut >> u) & 1u) && (key > kth_key || (key == kth_key && j0 + u <= kth_j))) keep |= 1u << u;
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < kFastPer; ++u) {
+    const int d = diag - (j0 + u);
+    if (d >= 0 && (j0 + u < a.sink || d < a.local)) keep |= 1u << u;
+  }
+  uint32_t word = (keep & ok) << (8 * (tid & 3));
+  word |= __shfl_xor_sync(0xffffffffu, word, 1);
+  word |= __shfl_xor_sync(0xffffffffu, word, 2);
+  if ((tid & 3) == 0 && (j0 >> 5) < a.W && a.bits) {
+    a.bits[((static_cast<long long>(b) * a.H + h) * a.Qb + i) * a.W + (j0 >> 5)] = word;
+  }
+  return true;
+}
+
 __global__ void __launch_bounds__(kRowThreads, 4) select_rows_kernel(const RowArgs a) {
   ptx::grid_launch_dependents();
   ptx::grid_dependency_wait();  // nothing in global memory is touched before this
@@ -526,7 +713,10 @@ __global__ void __launch_bounds__(kRowThreads, 4) select_rows_kernel(const RowAr
   const int h = (blockIdx.x / a.Qb) % a.H;
   const int b = blockIdx.x / (a.Qb * a.H);
   SEL_MARK(true, tm.tid, 0);
-  select_row(a, tm, &ts, dyn_smem, b, h, i, false);
+  __shared__ FastShared fs;
+  bool done = false;
+  if (i < a.rows_voting && fast_applies(a)) done = select_row_fast(a, &fs, &ts, b, h, i);
+  if (!done) select_row(a, tm, &ts, dyn_smem, b, h, i, false);
   SEL_MARK(true, tm.tid, 7);
   if (!a.fuse) return;
   const int kv_row = b * (a.H / a.G) + h / a.G;
