@@ -537,7 +537,7 @@ struct FastShared {
   int cand_j[kFastTies];
 };
 
-__device__ __forceinline__ bool fast_applies(const RowArgs& a) {
+inline bool fast_applies(const RowArgs& a) {
   return a.Kb <= kRowThreads * kFastPer && a.score_dtype == CA_DTYPE_F32 && a.s_k == 1 && !a.softmax && !a.prob_out && !a.score_max &&
          (a.rule == CA_RULE_THRESHOLD || a.rule == CA_RULE_TOPK);
 }
@@ -702,6 +702,8 @@ __device__ bool select_row_fast(const RowArgs& a, FastShared* fs, TeamShared* ts
   return true;
 }
 
+// kFast: launched where fast_applies; a kernel of its own, since beside it the general form is slower (1024 of 32K 171.1 / 172.5 us).
+template <bool kFast>
 __global__ void __launch_bounds__(kRowThreads, 4) select_rows_kernel(const RowArgs a) {
   ptx::grid_launch_dependents();
   ptx::grid_dependency_wait();  // nothing in global memory is touched before this
@@ -713,9 +715,11 @@ __global__ void __launch_bounds__(kRowThreads, 4) select_rows_kernel(const RowAr
   const int h = (blockIdx.x / a.Qb) % a.H;
   const int b = blockIdx.x / (a.Qb * a.H);
   SEL_MARK(true, tm.tid, 0);
-  __shared__ FastShared fs;
   bool done = false;
-  if (i < a.rows_voting && fast_applies(a)) done = select_row_fast(a, &fs, &ts, b, h, i);
+  if constexpr (kFast) {
+    __shared__ FastShared fs;
+    if (i < a.rows_voting) done = select_row_fast(a, &fs, &ts, b, h, i);
+  }
   if (!done) select_row(a, tm, &ts, dyn_smem, b, h, i, false);
   SEL_MARK(true, tm.tid, 7);
   if (!a.fuse) return;
@@ -1196,7 +1200,7 @@ static int fill_row_args(const ca_select_params* p, ca::select::RowArgs* out, si
     std::lock_guard<std::mutex> lock(mu);
     if (!done[dev.ordinal]) {
       const int max_smem = ((kMaxKb * 6 + 15) / 16) * 16 + kMaxKb * 8;
-      CA_CUDA(cudaFuncSetAttribute(select_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem));
+      CA_CUDA(cudaFuncSetAttribute(select_rows_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem));
       done[dev.ordinal] = true;
     }
   }
@@ -1212,7 +1216,7 @@ int ca_select_rows(const ca_select_params* p, ca_stream_t stream_) {
   size_t smem = 0;
   int rc = fill_row_args(p, &a, &smem, true);
   if (rc != CA_OK) return rc;
-  launch_kernel_as(true, select_rows_kernel, dim3(p->B * p->H * p->Qb), dim3(kRowThreads), smem, static_cast<cudaStream_t>(stream_), a);
+  launch_kernel_as(true, fast_applies(a) ? select_rows_kernel<true> : select_rows_kernel<false>, dim3(p->B * p->H * p->Qb), dim3(kRowThreads), smem, static_cast<cudaStream_t>(stream_), a);
   CA_LAUNCH_CHECK("select_rows_kernel");
   return CA_OK;
 }
@@ -1278,7 +1282,7 @@ int ca_select_union_table(const ca_select_params* p, const ca_union_params* u, v
   size_t smem = 0;
   int rc = fill_fused_args(p, u, scratch, scratch_bytes, &a, &smem);
   if (rc != CA_OK) return rc;
-  launch_kernel_as(true, select_rows_kernel, dim3(p->B * p->H * p->Qb), dim3(kRowThreads), smem, static_cast<cudaStream_t>(stream_), a);
+  launch_kernel_as(true, fast_applies(a) ? select_rows_kernel<true> : select_rows_kernel<false>, dim3(p->B * p->H * p->Qb), dim3(kRowThreads), smem, static_cast<cudaStream_t>(stream_), a);
   CA_LAUNCH_CHECK("select_rows_kernel");
   return CA_OK;
 }
@@ -1302,7 +1306,7 @@ int ca_gate_score_select(const ca_gate_score_params* g, const ca_select_params* 
   (void)write_scores;  // the logits always pass through score->out
   rc = ca_gate_scores(g, stream_);
   if (rc != CA_OK) return rc;
-  launch_kernel_as(true, select_rows_kernel, dim3(p->B * p->H * p->Qb), dim3(kRowThreads), row_smem, stream, a);
+  launch_kernel_as(true, fast_applies(a) ? select_rows_kernel<true> : select_rows_kernel<false>, dim3(p->B * p->H * p->Qb), dim3(kRowThreads), row_smem, stream, a);
   CA_LAUNCH_CHECK("select_rows_kernel");
   return CA_OK;
 }
