@@ -718,8 +718,9 @@ __global__ void __launch_bounds__(kThreads, 1)
             if (__any_sync(0xffffffffu, need)) {
               const float alpha = need ? (m_run == -INFINITY ? 0.f : ptx::ex2((m_run - m_new) * sc)) : 1.0f;
               if (j > sg.j0) {
-                ptx::mbar_wait_lean(sh_addr + static_cast<uint32_t>(offsetof(Shared, pv_done)) + tile * 8, (it - 1) & 1, abort_addr, a.wait_limit_us);
-                __syncwarp();
+                ok = ptx::mbar_wait_lean(sh_addr + static_cast<uint32_t>(offsetof(Shared, pv_done)) + tile * 8, (it - 1) & 1, abort_addr, a.wait_limit_us);
+                ok = __ballot_sync(0xffffffffu, ok) == 0xffffffffu;
+                if (!ok) break;  // a P.V may still be writing the accumulator
                 ptx::tc_fence_after();
   #pragma unroll 1  // more columns in flight beside the row of S spill (452 us instead of 435)
                 for (int c = 0; c < 8; ++c) {

@@ -1,0 +1,23 @@
+"""What the kernels do with a wait that ran out, read from their sources: a wait without a reader of its result goes on to touch
+what it waited for."""
+import re
+from pathlib import Path
+
+CSRC = Path(__file__).resolve().parent.parent / "compactattention_b200" / "csrc"
+
+
+def _without_comments(path):
+    return re.sub(r"//[^\n]*", "", re.sub(r"/\*.*?\*/", "", path.read_text(), flags=re.S))
+
+
+def test_no_wait_result_is_dropped():
+    """Only the drains after an abort (their flag is a dummy) may ignore how their wait ended."""
+    seen = 0
+    for path in sorted(CSRC.glob("*.cu")):
+        text = _without_comments(path)
+        for call in re.finditer(r"ptx::mbar_wait_\w+\(", text):
+            statement = text[call.start():text.index(";", call.start())]
+            before = text[:call.start()].rstrip()[-1]
+            seen += 1
+            assert before not in "{};)" or "&dummy" in statement, f"{path.name}: {statement}"
+    assert seen > 15
