@@ -57,24 +57,34 @@ int get_device_info(DeviceInfo* out) {
   return CA_OK;
 }
 
-// One CTA waits, with the bounded wait every tcgen05 / TMA kernel of the library uses, on a barrier nothing
-// ever arrives on: the wait must end after `limit_ns` with the abort flag set, and the kernel must return.
+// One CTA waits, with each of the two wait routines behind every mbarrier wait of the tcgen05 / TMA kernels in turn, on a barrier
+// nothing ever arrives on: the wait must end after `limit_ns` with the abort flag set, and the kernel must return.
+// *waited_ns: the longer of the two waits; CA_STATUS_TIMEOUT is raised only if both ended as they should, not before the limit.
 __global__ void selftest_bounded_wait_kernel(unsigned long long limit_ns, int32_t* status, unsigned long long* waited_ns) {
   __shared__ uint64_t bar;
   __shared__ int abort_flag;
   if (threadIdx.x == 0) {
-    abort_flag = 0;
     ptx::mbar_init(ptx::smem_u32(&bar), 1);
     ptx::mbar_fence_init();
   }
-  __syncthreads();
-  const uint64_t t0 = ptx::globaltimer_ns();
-  // every thread waits like the roles of a kernel do; the first to pass the limit raises the flag, the others see it
-  const bool ok = ptx::mbar_wait_bounded(ptx::smem_u32(&bar), 0, &abort_flag, limit_ns);
-  __syncthreads();
+  uint64_t longest = 0;
+  bool ended = true;
+  for (int routine = 0; routine < 2; ++routine) {
+    if (threadIdx.x == 0) abort_flag = 0;
+    __syncthreads();
+    const uint64_t t0 = ptx::globaltimer_ns();
+    // every thread waits like the roles of a kernel do; the first to pass the limit raises the flag, the others see it
+    const bool ok = routine == 0 ? ptx::mbar_wait_bounded(ptx::smem_u32(&bar), 0, &abort_flag, limit_ns)
+                                 : ptx::mbar_wait_lean(ptx::smem_u32(&bar), 0, ptx::smem_u32(&abort_flag), static_cast<uint32_t>((limit_ns + 999) / 1000));
+    const bool none = __syncthreads_or(ok ? 1 : 0) == 0;
+    const uint64_t waited = ptx::globaltimer_ns() - t0;
+    ended = ended && none && *const_cast<volatile int*>(&abort_flag) != 0 && waited >= limit_ns;
+    longest = waited > longest ? waited : longest;
+    __syncthreads();
+  }
   if (threadIdx.x == 0) {
-    if (waited_ns) *waited_ns = ptx::globaltimer_ns() - t0;
-    if (!ok && abort_flag && status) atomicOr(status, CA_STATUS_TIMEOUT);
+    if (waited_ns) *waited_ns = longest;
+    if (ended && status) atomicOr(status, CA_STATUS_TIMEOUT);
   }
 }
 

@@ -233,9 +233,9 @@ def test_step_replays_from_a_cuda_graph(ops):
 
 
 def test_a_bounded_wait_runs_out_and_the_context_stays_usable(ops):
-    """The wait routine behind every mbarrier wait of the tcgen05 / TMA kernels, on a barrier nothing arrives on:
-    it must give up after the limit (not before, not much later), report CA_STATUS_TIMEOUT, and leave the
-    context able to run the attention kernel afterwards."""
+    """The two wait routines behind every mbarrier wait of the tcgen05 / TMA kernels, on a barrier nothing arrives on:
+    each must give up after the limit (not before, not much later), CA_STATUS_TIMEOUT is reported, and the
+    context stays able to run the attention kernel afterwards."""
     from compactattention_b200 import _lib
     status = torch.zeros(1, dtype=torch.int32, device="cuda")
     waited = torch.zeros(1, dtype=torch.int64, device="cuda")

@@ -21,3 +21,10 @@ def test_no_wait_result_is_dropped():
             seen += 1
             assert before not in "{};)" or "&dummy" in statement, f"{path.name}: {statement}"
     assert seen > 15
+
+
+def test_the_self_test_runs_every_wait_routine():
+    """``ca_selftest_bounded_wait`` lets each of them run out (a GPU test reads how that ended)."""
+    routines = re.findall(r"\bbool (mbar_wait_\w+)\(", _without_comments(CSRC / "ca_common.cuh"))
+    kernel = _without_comments(CSRC / "ca_runtime.cu").split("selftest_bounded_wait_kernel(", 1)[1].split("extern \"C\"")[0]
+    assert len(routines) >= 2 and all(f"{name}(" in kernel for name in routines)
