@@ -920,7 +920,7 @@ __global__ void __launch_bounds__(kTileM) attn_combine_kernel(const KernelArgs a
     }
   };
   auto ml_of = [&](int i) {
-    return __ldg(reinterpret_cast<const float2*>(a.part_ml + static_cast<long long>(chain_sh[i]) * kPartialMLFloats + (tile * kTileM + r) * 2));
+    return *reinterpret_cast<const float2*>(a.part_ml + static_cast<long long>(chain_sh[i]) * kPartialMLFloats + (tile * kTileM + r) * 2);
   };
   load_o(0, 0);
   float m = -INFINITY;

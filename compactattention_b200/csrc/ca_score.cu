@@ -432,7 +432,7 @@ __global__ void __launch_bounds__(kGateThreads) gate_scores3_kernel(const GateAr
   const uint16_t* kp = reinterpret_cast<const uint16_t*>(a.k) + b * a.k_b + static_cast<long long>(jc) * a.k_blk + hk * a.k_h;
   uint4 raw[16];
 #pragma unroll
-  for (int u = 0; u < 16; ++u) raw[u] = __ldg(reinterpret_cast<const uint4*>(kp + u * 8));
+  for (int u = 0; u < 16; ++u) raw[u] = *reinterpret_cast<const uint4*>(kp + u * 8);
   for (int e = threadIdx.x * 8; e < kGateRows * 128; e += kGateThreads * 8) {
     const int i = e / 128, c = e % 128;
     float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};

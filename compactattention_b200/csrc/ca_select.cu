@@ -357,7 +357,7 @@ __device__ void select_row(const RowArgs& a, const Team& tm, TeamShared* ts, uns
   float exp_max = -INFINITY;  // with score_max: the row's largest exponent
   if (a.score_max) {
     float m = -INFINITY;
-    for (int j = tm.tid; j < a.Kb; j += tm.nt) m = fmaxf(m, __ldg(a.score_max + s_off + j * a.s_k));
+    for (int j = tm.tid; j < a.Kb; j += tm.nt) m = fmaxf(m, a.score_max[s_off + j * a.s_k]);
     exp_max = block_reduce_max(tm, m, ts->red);
   }
   for (int base = 0; base < a.Kb; base += tm.nt * 8) {
@@ -374,7 +374,7 @@ __device__ void select_row(const RowArgs& a, const Team& tm, TeamShared* ts, uns
         } else {
           x[u] = load_score(a.score, s_off + j * a.s_k, a.score_dtype);
           if (a.score_max) {
-            const float e = __ldg(a.score_max + s_off + j * a.s_k);
+            const float e = a.score_max[s_off + j * a.s_k];
             x[u] = e == -INFINITY ? 0.f : x[u] * exp2f(e - exp_max);
           }
         }
@@ -417,7 +417,7 @@ __device__ void select_row(const RowArgs& a, const Team& tm, TeamShared* ts, uns
 
   SEL_MARK(tm.bar <= 1, tm.tid, 5);
   // ---- the rule ----
-  const float thr = a.threshold_ptr ? __ldg(a.threshold_ptr + b * a.threshold_stride) : a.threshold;
+  const float thr = a.threshold_ptr ? a.threshold_ptr[b * a.threshold_stride] : a.threshold;
   if (a.rule == CA_RULE_THRESHOLD) {
     for (int j = tm.tid; j < a.Kb; j += tm.nt) keep[j] = s[j] > thr;  // -inf never passes
   } else if (a.rule == CA_RULE_MASK) {
@@ -545,11 +545,11 @@ inline bool fast_applies(const RowArgs& a) {
 // Loads the eight floats at p[0..7], those with j0 + u >= n as 0.
 __device__ __forceinline__ void load8(const float* p, int j0, int n, float (&x)[kFastPer]) {
   if (j0 + kFastPer <= n && (reinterpret_cast<uintptr_t>(p) & 15) == 0) {
-    const float4 v0 = __ldg(reinterpret_cast<const float4*>(p)), v1 = __ldg(reinterpret_cast<const float4*>(p) + 1);
+    const float4 v0 = *reinterpret_cast<const float4*>(p), v1 = reinterpret_cast<const float4*>(p)[1];
     x[0] = v0.x, x[1] = v0.y, x[2] = v0.z, x[3] = v0.w, x[4] = v1.x, x[5] = v1.y, x[6] = v1.z, x[7] = v1.w;
   } else {
 #pragma unroll
-    for (int u = 0; u < kFastPer; ++u) x[u] = j0 + u < n ? __ldg(p + u) : 0.f;
+    for (int u = 0; u < kFastPer; ++u) x[u] = j0 + u < n ? p[u] : 0.f;
   }
 }
 
@@ -565,7 +565,7 @@ __device__ bool select_row_fast(const RowArgs& a, FastShared* fs, TeamShared* ts
   if (a.valid) {
     const uint8_t* v = a.valid + b * a.v_b + h * a.v_h + i * a.v_q;
     if (a.v_k == 1 && j0 + kFastPer <= a.Kb && (reinterpret_cast<uintptr_t>(v + j0) & 7) == 0) {
-      const uint2 w = __ldg(reinterpret_cast<const uint2*>(v + j0));
+      const uint2 w = *reinterpret_cast<const uint2*>(v + j0);
 #pragma unroll
       for (int u = 0; u < kFastPer; ++u) ok |= (((u < 4 ? w.x : w.y) >> (8 * (u & 3))) & 0xffu) != 0 ? 1u << u : 0u;
     } else {
@@ -580,7 +580,7 @@ __device__ bool select_row_fast(const RowArgs& a, FastShared* fs, TeamShared* ts
   }
   uint32_t keep = 0;
   if (a.rule == CA_RULE_THRESHOLD) {
-    const float thr = a.threshold_ptr ? __ldg(a.threshold_ptr + b * a.threshold_stride) : a.threshold;
+    const float thr = a.threshold_ptr ? a.threshold_ptr[b * a.threshold_stride] : a.threshold;
 #pragma unroll
     for (int u = 0; u < kFastPer; ++u) keep |= (x[u] > thr ? 1u : 0u) << u;
   } else {
@@ -889,8 +889,8 @@ __global__ void __launch_bounds__(kGtThreads) gate_scores_tc_kernel(const __grid
         const int i = rr / a.G, g = rr - i * a.G;
         const long long off = b * a.q_b + i * a.q_blk + static_cast<long long>(hk * a.G + g) * a.q_h + piece * 8;
         if (a.q_dtype == CA_DTYPE_F32) {
-          const float4 x0 = __ldg(reinterpret_cast<const float4*>(reinterpret_cast<const float*>(a.q) + off));
-          const float4 x1 = __ldg(reinterpret_cast<const float4*>(reinterpret_cast<const float*>(a.q) + off + 4));
+          const float4 x0 = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(a.q) + off);
+          const float4 x1 = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(a.q) + off + 4);
           v[u][0] = x0.x, v[u][1] = x0.y, v[u][2] = x0.z, v[u][3] = x0.w, v[u][4] = x1.x, v[u][5] = x1.y, v[u][6] = x1.z, v[u][7] = x1.w;
         } else {
 #pragma unroll

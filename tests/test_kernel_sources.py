@@ -1,5 +1,6 @@
-"""What the kernels do with a wait that ran out, read from their sources: a wait without a reader of its result goes on to touch
-what it waited for."""
+"""Contracts of the kernels that their sources show and no run can be relied on to break: a wait without a reader of its result
+goes on to touch what it waited for; a load through the non-coherent path promises that nobody writes the address while the kernel
+lives, which a programmatic dependent launch cannot promise of what the launch before it writes."""
 import re
 from pathlib import Path
 
@@ -28,3 +29,12 @@ def test_the_self_test_runs_every_wait_routine():
     routines = re.findall(r"\bbool (mbar_wait_\w+)\(", _without_comments(CSRC / "ca_common.cuh"))
     kernel = _without_comments(CSRC / "ca_runtime.cu").split("selftest_bounded_wait_kernel(", 1)[1].split("extern \"C\"")[0]
     assert len(routines) >= 2 and all(f"{name}(" in kernel for name in routines)
+
+
+def test_dependent_launches_load_coherently():
+    """Every kernel here may be resident while the launch before it still writes, and its pointers come as plain arguments, so
+    only an ordinary load stays behind the dependency wait by contract."""
+    for path in sorted(CSRC.glob("*.cu*")):
+        text = _without_comments(path)
+        found = re.findall(r"__ldg|ld\.global\.nc|const\s[^,;(){}]*\*\s*__restrict__", text)
+        assert not found, f"{path.name}: {found}"
