@@ -33,7 +33,8 @@ __device__ __forceinline__ float load_score(const void* base, long long off, int
 
 // Monotone map float -> uint32 (larger float -> larger key); -0 and +0 differ but compare adjacent.
 __device__ __forceinline__ uint32_t order_key(float f) {
-  uint32_t u = __float_as_uint(f);
+  uint32_t u;
+  asm("mov.b32 %0, %1;" : "=r"(u) : "f"(f));  // opaque: setting the sign bit of a float's bits may become -|f|, and a NaN loses its sign there
   return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
 
@@ -518,23 +519,33 @@ __device__ void select_row(const RowArgs& a, const Team& tm, TeamShared* ts, uns
 // A row of at most 2048 contiguous f32 scores under the threshold or the top-k rule, without leaving registers: a thread
 // owns eight consecutive entries and packs their bits itself.  The general form above writes scores and flags to shared memory and
 // reads them back, and its radix passes queue on the few bins that a row's exponents fall into; a row is bound by instruction issue
-// and by the number of barriers, and this has four for top-k and none for a threshold.
-// us a pass, before / after: 2 x 1000 of 64K, 28/4 heads, threshold 300 / 292.5; one KV head of 128K, top-k 93.2 / 90.3; 8 KV heads
-// 541.5 / 536.6.  The row-max rule on raw scores stays in the general form: with its 256 blocks a row a single warp would have all
-// the exponentials (1024 of 32K, 173.9 / 176.9).
-// Top-k: 256 bins over [lowest, highest] score (x -> bin is monotone, equal scores share a bin), the entries of the bin that holds
-// the k-th largest are ranked against each other by (key, lower index), as the general form orders them.  Returns false, with
-// nothing written, where that does not hold or pay: a visible score that is not finite, more than kFastTies entries in that bin.
+// and by the number of barriers, and this has five for top-k where one level is enough and none for a threshold.
+// Top-k: the competing entries go into 256 bins, everything above the bin that holds the k-th largest is kept, and that bin's
+// entries compete for what is left, until all of them are wanted or at most kFastRank are left, which are ranked against each other
+// by (key, lower index), as the general form orders them.  Bins divide the order-preserving keys evenly, which are close to the
+// logarithm where all scores have one sign, as probabilities do; scores of both signs, as logits are, would crowd into the few
+// bins of their exponents, so for them the first two levels divide the scores evenly, from the lowest to the highest but for one
+// thread of each warp (a sink far above the others would stretch the bins).  x -> bin is monotone in either case, equal scores share
+// a bin.  A level by keys takes 8 bits off their range, and equal keys are told apart by index: eight levels at most.
+// As in the general form, what is not visible competes as -inf: that matters only if k reaches into the visible -inf.
+// us for 512 rows, general form / this (2.4 of either is the launch): 20 % of 2048 logits 8.9 / 6.1, of 256 6.5 / 5.7; of
+// softmax(3 z) 8.9 / 6.2, 6.5 / 5.8; beside one score of 100 8.8 / 6.1, 6.5 / 5.7; all equal 14.2 / 6.2, 7.8 / 6.0; a third of the digits
+// alike 14.5 / 7.3, 7.9 / 6.5.  Slower only where many outliers take a second level: every 97th logit 1e4 times larger 8.9 / 8.5, 6.5 / 7.7.
+// A threshold 5.5 / 2.4, 3.7 / 2.4.  (Bins by score alone, one level, up to 512 ranked or the general form on top: softmax(3 z) 13.3, 23.6;
+// one score of 100 42, 8.8.)  28 heads x 128 rows of 2048: 45.8 / 28.6.  Finding the bin in every warp instead of one and a barrier: 6.2 for 5.8.
+// The row-max rule on raw scores stays in the general form: with its 256 blocks a row a single warp would have all the
+// exponentials (1024 of 32K, 173.9 / 176.9).
 constexpr int kFastPer = 8;
-constexpr int kFastTies = 512;
-struct FastShared {
-  float lo[kRowThreads / 32], hi[kRowThreads / 32];
-  int hist[256];
-  int n_valid, n_cand, odd;
-  uint32_t kth_key;
-  int kth_j;
-  uint32_t cand_key[kFastTies];
-  int cand_j[kFastTies];
+constexpr int kFastRank = 32;  // one warp's; 64: the loop over them costs as much as another level
+constexpr uint32_t kKeyNegInf = 0x007fffffu, kKeyPosInf = 0xff800000u;  // order_key(-inf), order_key(inf)
+struct __align__(16) FastShared {
+  uint32_t lo[kRowThreads / 32], hi[kRowThreads / 32], hi2[kRowThreads / 32];
+  int count[kRowThreads / 32];
+  int hist[2][256];
+  int n_cand;
+  uint32_t found;
+  unsigned long long kth;
+  unsigned long long cand[kFastRank];
 };
 
 inline bool fast_applies(const RowArgs& a) {
@@ -553,145 +564,196 @@ __device__ __forceinline__ void load8(const float* p, int j0, int n, float (&x)[
   }
 }
 
-__device__ bool select_row_fast(const RowArgs& a, FastShared* fs, TeamShared* ts, int b, int h, int i) {
-  const Team tm{static_cast<int>(threadIdx.x), kRowThreads, 0};
-  const int tid = tm.tid, lane = tid & 31;
-  const int j0 = tid * kFastPer;
-  const int diag = a.Pb + i;
-  const long long s_off = b * a.s_b + h * a.s_h + i * a.s_q + j0;
-  float x[kFastPer];
-  load8(reinterpret_cast<const float*>(a.score) + s_off, j0, a.Kb, x);
-  uint32_t ok = 0;  // visible entries
-  if (a.valid) {
-    const uint8_t* v = a.valid + b * a.v_b + h * a.v_h + i * a.v_q;
-    if (a.v_k == 1 && j0 + kFastPer <= a.Kb && (reinterpret_cast<uintptr_t>(v + j0) & 7) == 0) {
-      const uint2 w = *reinterpret_cast<const uint2*>(v + j0);
+// Ranks an entry of a row: higher score first, then lower index.
+__device__ __forceinline__ unsigned long long fast_rank_key(float x, int j) {
+  return (static_cast<unsigned long long>(order_key(x)) << 11) | static_cast<unsigned>(kRowThreads * kFastPer - 1 - j);
+}
+
+__device__ __forceinline__ float key_value(uint32_t key) { return __uint_as_float((key & 0x80000000u) ? key ^ 0x80000000u : ~key); }
+
+// Lowest and highest key of the entries in `cand`, over the CTA.  One barrier.  khi2: the highest but for a warp's highest thread.
+__device__ __forceinline__ void key_range(const float (&x)[kFastPer], uint32_t cand, FastShared* fs, uint32_t* klo, uint32_t* khi, uint32_t* khi2) {
+  uint32_t lo = 0xffffffffu, hi = 0u;
 #pragma unroll
-      for (int u = 0; u < kFastPer; ++u) ok |= (((u < 4 ? w.x : w.y) >> (8 * (u & 3))) & 0xffu) != 0 ? 1u << u : 0u;
-    } else {
-#pragma unroll
-      for (int u = 0; u < kFastPer; ++u)
-        if (j0 + u < a.Kb && v[(j0 + u) * a.v_k] != 0) ok |= 1u << u;
-    }
-  } else {
-    const int last = diag < a.Kb - 1 ? diag : a.Kb - 1;
-    const int c = last - j0 + 1;
-    ok = c <= 0 ? 0u : c >= kFastPer ? 0xffu : (1u << c) - 1u;
+  for (int u = 0; u < kFastPer; ++u) {
+    if ((cand >> u) & 1u) lo = min(lo, order_key(x[u])), hi = max(hi, order_key(x[u]));
   }
-  uint32_t keep = 0;
-  if (a.rule == CA_RULE_THRESHOLD) {
-    const float thr = a.threshold_ptr ? a.threshold_ptr[b * a.threshold_stride] : a.threshold;
+  const uint32_t own = hi;
+  lo = __reduce_min_sync(0xffffffffu, lo), hi = __reduce_max_sync(0xffffffffu, hi);
+  const uint32_t next = __reduce_max_sync(0xffffffffu, own == hi ? 0u : own);
+  if ((threadIdx.x & 31) == 0) fs->lo[threadIdx.x >> 5] = lo, fs->hi[threadIdx.x >> 5] = hi, fs->hi2[threadIdx.x >> 5] = next;
+  __syncthreads();
+  const uint4 l0 = *reinterpret_cast<const uint4*>(fs->lo), l1 = *reinterpret_cast<const uint4*>(fs->lo + 4);
+  const uint4 h0 = *reinterpret_cast<const uint4*>(fs->hi), h1 = *reinterpret_cast<const uint4*>(fs->hi + 4);
+  *klo = min(min(min(l0.x, l0.y), min(l0.z, l0.w)), min(min(l1.x, l1.y), min(l1.z, l1.w)));
+  *khi = max(max(max(h0.x, h0.y), max(h0.z, h0.w)), max(max(h1.x, h1.y), max(h1.z, h1.w)));
+  const uint4 n0 = *reinterpret_cast<const uint4*>(fs->hi2), n1 = *reinterpret_cast<const uint4*>(fs->hi2 + 4);
+  *khi2 = max(max(max(n0.x, n0.y), max(n0.z, n0.w)), max(max(n1.x, n1.y), max(n1.z, n1.w)));
+}
+
+// The bits of the thread's eight entries that the top-k rule keeps.  `ok`: its visible entries.
+__device__ __forceinline__ uint32_t topk_fast(const RowArgs& a, FastShared* fs, float (&x)[kFastPer], uint32_t ok) {
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int j0 = tid * kFastPer;
+  uint32_t klo, khi, khi2, cand = ok;  // cand: the competing entries
 #pragma unroll
-    for (int u = 0; u < kFastPer; ++u) keep |= (x[u] > thr ? 1u : 0u) << u;
-  } else {
-    float lo = INFINITY, hi = -INFINITY;
-    bool odd = false;
+  for (int u = 0; u < kFastPer; ++u) cand &= order_key(x[u]) == kKeyNegInf ? ~(1u << u) : ~0u;
+  const int cnt = __reduce_add_sync(0xffffffffu, __popc(cand) + (__popc(ok) << 16));
+  if (lane == 0) fs->count[tid >> 5] = cnt;
+  fs->hist[0][tid] = 0;
+  if (tid < kFastRank) fs->cand[tid] = 0ull;  // below every entry
+  if (tid == 0) fs->n_cand = 0;
+  key_range(x, cand, fs, &klo, &khi, &khi2);
+  const int4 c0 = *reinterpret_cast<const int4*>(fs->count), c1 = *reinterpret_cast<const int4*>(fs->count + 4);
+  const int both = ((c0.x + c0.y) + (c0.z + c0.w)) + ((c1.x + c1.y) + (c1.z + c1.w));
+  const int n_above = both & 0xffff, n_valid = both >> 16;  // visible and above -inf; visible
+  int k = a.topk_k > 0 ? a.topk_k
+                       : static_cast<int>((static_cast<long long>(a.topk_num) * n_valid + a.topk_den / 2) / a.topk_den);
+  if (k < 1) k = 1;
+  if (k > n_valid) k = n_valid;
+  if (k == 0) return 0u;
+  uint32_t keep = 0;
+  int left = k;
+  const bool finite = klo > kKeyNegInf && khi < kKeyPosInf;
+  if (!finite || k > n_above) {
+    const int c = a.Kb - j0;
+    const uint32_t here = c <= 0 ? 0u : c >= kFastPer ? 0xffu : (1u << c) - 1u;
 #pragma unroll
     for (int u = 0; u < kFastPer; ++u) {
-      if ((ok >> u) & 1u) {
-        lo = fminf(lo, x[u]), hi = fmaxf(hi, x[u]);
-        odd |= !(fabsf(x[u]) < INFINITY);
-      }
+      if (!((ok >> u) & 1u)) x[u] = -INFINITY;
     }
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) {
-      lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, d));
-      hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, d));
+    if (!finite) {  // NaN or +inf: everything, by keys
+      if (k >= a.Kb) return here;
+      cand = here, klo = 0u, khi = 0xffffffffu;
+    } else {  // what is above -inf, and some that are
+      keep = cand, left = k - n_above;
+      cand = here & ~cand, klo = khi = kKeyNegInf;
     }
-    const int cnt = __reduce_add_sync(0xffffffffu, __popc(ok));
-    fs->hist[tid] = 0;
-    if (tid == 0) fs->n_cand = 0;
-    if (lane == 0) fs->lo[tid >> 5] = lo, fs->hi[tid >> 5] = hi, ts->warp_sums[tid >> 5] = cnt;
-    if (__syncthreads_or(odd ? 1 : 0)) return false;
-    int n_valid = 0;
-#pragma unroll
-    for (int w = 0; w < kRowThreads / 32; ++w) {
-      lo = fminf(lo, fs->lo[w]), hi = fmaxf(hi, fs->hi[w]);
-      n_valid += ts->warp_sums[w];
-    }
-    if (!a.valid) n_valid = diag + 1 < a.Kb ? diag + 1 : a.Kb;
-    int k = a.topk_k > 0 ? a.topk_k
-                         : static_cast<int>((static_cast<long long>(a.topk_num) * n_valid + a.topk_den / 2) / a.topk_den);
-    if (k < 1) k = 1;
-    if (k > n_valid) k = n_valid;
-    if (k >= n_valid) {
-      keep = ok;  // all of them (none, if none is visible)
-    } else {
+  } else if (k == n_above) {
+    return cand;
+  }
+  for (int level = 0;; ++level) {
+    int* hist = fs->hist[level & 1];
+    int bin[kFastPer];
+    const float lo = key_value(klo), hi = key_value(khi2 > 0x80000000u ? khi2 : khi);
+    if (level < 2 && finite && lo < 0.f && hi > 0.f) {
       const float scale = 255.9f / (hi - lo);
-      int bin[kFastPer];
 #pragma unroll
-      for (int u = 0; u < kFastPer; ++u) {
-        // 0 .. 255; a NaN (equal scores and an infinite scale) is 0
-        bin[u] = ((ok >> u) & 1u) ? min(255, max(0, __float2int_rz((x[u] - lo) * scale))) : -1;
-        if (bin[u] >= 0) atomicAdd(&fs->hist[bin[u]], 1);
-      }
-      __syncthreads();
-      // every warp finds the bin that holds the k-th largest: lane l owns bins 255-8l .. 248-8l
-      int mine = 0, c[8];
+      for (int u = 0; u < kFastPer; ++u) bin[u] = min(255, max(0, __float2int_rz((x[u] - lo) * scale)));  // NaN (infinite range): 0
+    } else if (klo < khi) {
+      const float scale = 255.9f / __uint2float_ru(khi - klo);  // up to 255 keys: each a bin of its own
 #pragma unroll
-      for (int u = 0; u < 8; ++u) c[u] = fs->hist[255 - 8 * lane - u], mine += c[u];
+      for (int u = 0; u < kFastPer; ++u) bin[u] = __float2int_rz(__uint2float_rz(order_key(x[u]) - klo) * scale);
+    } else {
+#pragma unroll
+      for (int u = 0; u < kFastPer; ++u) bin[u] = kRowThreads - 1 - tid;
+    }
+#pragma unroll
+    for (int u = 0; u < kFastPer; ++u) {
+      if ((cand >> u) & 1u) atomicAdd(&hist[bin[u]], 1);
+    }
+    __syncthreads();
+    if (tid < 32) {
+      // the bin that holds the left-th largest: lane l owns bins 255-8l .. 248-8l
+      const int4 c_lo = *reinterpret_cast<const int4*>(hist + 248 - 8 * lane), c_hi = *reinterpret_cast<const int4*>(hist + 252 - 8 * lane);
+      const int c[8] = {c_hi.w, c_hi.z, c_hi.y, c_hi.x, c_lo.w, c_lo.z, c_lo.y, c_lo.x};
+      const int mine = ((c[0] + c[1]) + (c[2] + c[3])) + ((c[4] + c[5]) + (c[6] + c[7]));
       int inc = mine;
 #pragma unroll
       for (int d = 1; d < 32; d <<= 1) {
         const int nb = __shfl_up_sync(0xffffffffu, inc, d);
         if (lane >= d) inc += nb;
       }
-      const int owner = __ffs(__ballot_sync(0xffffffffu, inc >= k)) - 1;
-      int left = k - (inc - mine), cut = 0, at = 0;
-      bool found = false;
+      int wanted = left - (inc - mine);
+      if (wanted > 0 && wanted <= mine) {  // one lane's
+        int u = 0;
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        if (!found) {
-          if (c[u] >= left) found = true, cut = 255 - 8 * lane - u, at = c[u];
-          else left -= c[u];
+        for (int q = 0; q < 7; ++q) {
+          if (u == q && c[q] < wanted) wanted -= c[q], ++u;
         }
-      }
-      cut = __shfl_sync(0xffffffffu, cut, owner);   // the bin
-      left = __shfl_sync(0xffffffffu, left, owner);  // entries wanted of it
-      at = __shfl_sync(0xffffffffu, at, owner);      // entries in it
-      if (at > kFastTies) return false;
-      uint32_t in_cut = 0;
+        int in_bin = c[0];
 #pragma unroll
-      for (int u = 0; u < kFastPer; ++u) {
-        if (bin[u] > cut) keep |= 1u << u;
-        if (bin[u] == cut) in_cut |= 1u << u;
-      }
-      if (left == at) {
-        keep |= in_cut;
-      } else {
-#pragma unroll
-        for (int u = 0; u < kFastPer; ++u) {
-          if ((in_cut >> u) & 1u) {
-            const int o = atomicAdd(&fs->n_cand, 1);
-            fs->cand_key[o] = order_key(x[u]), fs->cand_j[o] = j0 + u;
-          }
-        }
-        __syncthreads();
-        for (int q = tid; q < at; q += kRowThreads) {
-          const uint32_t key = fs->cand_key[q];
-          const int j = fs->cand_j[q];
-          int before = 0;
-          for (int o = 0; o < at; ++o) {
-            const uint32_t other = fs->cand_key[o];
-            before += other > key || (other == key && fs->cand_j[o] < j);
-          }
-          if (before == left - 1) fs->kth_key = key, fs->kth_j = j;  // just one entry has this place
-        }
-        __syncthreads();
-        const uint32_t kth_key = fs->kth_key;
-        const int kth_j = fs->kth_j;
-#pragma unroll
-        for (int u = 0; u < kFastPer; ++u) {
-          const uint32_t key = order_key(x[u]);
-          if (((in_cut >> u) & 1u) && (key > kth_key || (key == kth_key && j0 + u <= kth_j))) keep |= 1u << u;
-        }
+        for (int q = 1; q < 8; ++q) in_bin = u == q ? c[q] : in_bin;
+        fs->found = static_cast<uint32_t>(255 - 8 * lane - u) | (static_cast<uint32_t>(wanted) << 8) | (static_cast<uint32_t>(in_bin) << 20);
       }
     }
+    __syncthreads();
+    const uint32_t found = fs->found;  // the bin, the entries wanted of it, the entries in it
+    const int cut = static_cast<int>(found & 255u), at = static_cast<int>(found >> 20);
+    left = static_cast<int>((found >> 8) & 0xfffu);
+    uint32_t in_cut = 0;
+#pragma unroll
+    for (int u = 0; u < kFastPer; ++u) {
+      if (bin[u] > cut) keep |= cand & (1u << u);
+      if (bin[u] == cut) in_cut |= 1u << u;
+    }
+    cand &= in_cut;
+    if (left == at) return keep | cand;
+    if (at <= kFastRank) break;
+    fs->hist[(level + 1) & 1][tid] = 0;  // last read in the level before
+    key_range(x, cand, fs, &klo, &khi, &khi2);
   }
 #pragma unroll
   for (int u = 0; u < kFastPer; ++u) {
-    const int d = diag - (j0 + u);
-    if (d >= 0 && (j0 + u < a.sink || d < a.local)) keep |= 1u << u;
+    if ((cand >> u) & 1u) fs->cand[atomicAdd(&fs->n_cand, 1)] = fast_rank_key(x[u], j0 + u);
+  }
+  __syncthreads();
+  const int at = fs->n_cand;
+  if (tid < at) {
+    const unsigned long long me = fs->cand[tid];
+    int before = 0;
+    for (int o = 0; o < at; o += 8) {
+#pragma unroll
+      for (int q = 0; q < 8; ++q) before += fs->cand[o + q] > me;
+    }
+    if (before == left - 1) fs->kth = me;  // just one entry has this place
+  }
+  __syncthreads();
+  const unsigned long long kth = fs->kth;
+#pragma unroll
+  for (int u = 0; u < kFastPer; ++u) {
+    if (((cand >> u) & 1u) && fast_rank_key(x[u], j0 + u) >= kth) keep |= 1u << u;
+  }
+  return keep;
+}
+
+__device__ __forceinline__ void select_row_fast(const RowArgs& a, FastShared* fs, int b, int h, int i) {
+  const int tid = threadIdx.x;
+  const int j0 = tid * kFastPer;
+  const int diag = a.Pb + i;
+  const long long s_off = b * a.s_b + h * a.s_h + i * a.s_q + j0;
+  uint32_t keep = 0, ok = 0;  // ok: visible entries
+  if (i < a.rows_voting) {
+    float x[kFastPer];
+    load8(reinterpret_cast<const float*>(a.score) + s_off, j0, a.Kb, x);
+    if (a.valid) {
+      const uint8_t* v = a.valid + b * a.v_b + h * a.v_h + i * a.v_q;
+      if (a.v_k == 1 && j0 + kFastPer <= a.Kb && (reinterpret_cast<uintptr_t>(v + j0) & 7) == 0) {
+        const uint2 w = *reinterpret_cast<const uint2*>(v + j0);
+#pragma unroll
+        for (int u = 0; u < kFastPer; ++u) ok |= (((u < 4 ? w.x : w.y) >> (8 * (u & 3))) & 0xffu) != 0 ? 1u << u : 0u;
+      } else {
+#pragma unroll
+        for (int u = 0; u < kFastPer; ++u)
+          if (j0 + u < a.Kb && v[(j0 + u) * a.v_k] != 0) ok |= 1u << u;
+      }
+    } else {
+      const int last = diag < a.Kb - 1 ? diag : a.Kb - 1;
+      const int c = last - j0 + 1;
+      ok = c <= 0 ? 0u : c >= kFastPer ? 0xffu : (1u << c) - 1u;
+    }
+    if (a.rule == CA_RULE_THRESHOLD) {
+      const float thr = a.threshold_ptr ? a.threshold_ptr[b * a.threshold_stride] : a.threshold;
+#pragma unroll
+      for (int u = 0; u < kFastPer; ++u) keep |= (x[u] > thr ? 1u : 0u) << u;
+    } else {
+      keep = topk_fast(a, fs, x, ok);
+    }
+#pragma unroll
+    for (int u = 0; u < kFastPer; ++u) {
+      const int d = diag - (j0 + u);
+      if (d >= 0 && (j0 + u < a.sink || d < a.local)) keep |= 1u << u;
+    }
   }
   uint32_t word = (keep & ok) << (8 * (tid & 3));
   word |= __shfl_xor_sync(0xffffffffu, word, 1);
@@ -699,10 +761,9 @@ __device__ bool select_row_fast(const RowArgs& a, FastShared* fs, TeamShared* ts
   if ((tid & 3) == 0 && (j0 >> 5) < a.W && a.bits) {
     a.bits[((static_cast<long long>(b) * a.H + h) * a.Qb + i) * a.W + (j0 >> 5)] = word;
   }
-  return true;
 }
 
-// kFast: launched where fast_applies; a kernel of its own, since beside it the general form is slower (1024 of 32K 171.1 / 172.5 us).
+// kFast: launched where fast_applies.
 template <bool kFast>
 __global__ void __launch_bounds__(kRowThreads, 4) select_rows_kernel(const RowArgs a) {
   ptx::grid_launch_dependents();
@@ -715,12 +776,12 @@ __global__ void __launch_bounds__(kRowThreads, 4) select_rows_kernel(const RowAr
   const int h = (blockIdx.x / a.Qb) % a.H;
   const int b = blockIdx.x / (a.Qb * a.H);
   SEL_MARK(true, tm.tid, 0);
-  bool done = false;
   if constexpr (kFast) {
     __shared__ FastShared fs;
-    if (i < a.rows_voting) done = select_row_fast(a, &fs, &ts, b, h, i);
+    select_row_fast(a, &fs, b, h, i);
+  } else {
+    select_row(a, tm, &ts, dyn_smem, b, h, i, false);
   }
-  if (!done) select_row(a, tm, &ts, dyn_smem, b, h, i, false);
   SEL_MARK(true, tm.tid, 7);
   if (!a.fuse) return;
   const int kv_row = b * (a.H / a.G) + h / a.G;
