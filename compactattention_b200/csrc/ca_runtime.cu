@@ -60,6 +60,7 @@ int get_device_info(DeviceInfo* out) {
 // One CTA waits, with each of the two wait routines behind every mbarrier wait of the tcgen05 / TMA kernels in turn, on a barrier
 // nothing ever arrives on: the wait must end after `limit_ns` with the abort flag set, and the kernel must return.
 // *waited_ns: the longer of the two waits; CA_STATUS_TIMEOUT is raised only if both ended as they should, not before the limit.
+// The second routine counts units of 1.024 us and may end two of them early, so it gets two more here.
 __global__ void selftest_bounded_wait_kernel(unsigned long long limit_ns, int32_t* status, unsigned long long* waited_ns) {
   __shared__ uint64_t bar;
   __shared__ int abort_flag;
@@ -75,7 +76,7 @@ __global__ void selftest_bounded_wait_kernel(unsigned long long limit_ns, int32_
     const uint64_t t0 = ptx::globaltimer_ns();
     // every thread waits like the roles of a kernel do; the first to pass the limit raises the flag, the others see it
     const bool ok = routine == 0 ? ptx::mbar_wait_bounded(ptx::smem_u32(&bar), 0, &abort_flag, limit_ns)
-                                 : ptx::mbar_wait_lean(ptx::smem_u32(&bar), 0, ptx::smem_u32(&abort_flag), static_cast<uint32_t>((limit_ns + 999) / 1000));
+                                 : ptx::mbar_wait_lean(ptx::smem_u32(&bar), 0, ptx::smem_u32(&abort_flag), static_cast<uint32_t>((limit_ns + 999) / 1000) + 2);
     const bool none = __syncthreads_or(ok ? 1 : 0) == 0;
     const uint64_t waited = ptx::globaltimer_ns() - t0;
     ended = ended && none && *const_cast<volatile int*>(&abort_flag) != 0 && waited >= limit_ns;

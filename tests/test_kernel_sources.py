@@ -38,3 +38,16 @@ def test_dependent_launches_load_coherently():
         text = _without_comments(path)
         found = re.findall(r"__ldg|ld\.global\.nc|const\s[^,;(){}]*\*\s*__restrict__", text)
         assert not found, f"{path.name}: {found}"
+
+
+def test_the_self_tests_limit_covers_the_coarse_clock():
+    """``mbar_wait_lean`` keeps time in units of 1024 ns with the lowest bit set.  For every start within a pair of units and short limit,
+    the limit that the self-test passes may not let the wait end before ``limit_ns``."""
+    kernel = _without_comments(CSRC / "ca_runtime.cu").split("selftest_bounded_wait_kernel(", 1)[1].split("extern \"C\"")[0]
+    extra = int(re.search(r"\(limit_ns \+ 999\) / 1000\)(?: \+ (\d+))?\);", kernel).group(1) or 0)
+    for limit_ns in (1, 500, 1000, 1024, 3000, 10_000, 40_000):
+        limit = (limit_ns + 999) // 1000 + extra
+        for start in range(0, 2048, 64):
+            t0 = (start >> 10) | 1
+            end = next(t for t in range(start, start + 10**6, 64) if ((t >> 10) | 1) - t0 > limit)
+            assert end - start >= limit_ns, (limit_ns, start)
