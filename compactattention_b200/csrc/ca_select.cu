@@ -766,7 +766,6 @@ __device__ __forceinline__ void select_row_fast(const RowArgs& a, FastShared* fs
 // kFast: launched where fast_applies.
 template <bool kFast>
 __global__ void __launch_bounds__(kRowThreads, 4) select_rows_kernel(const RowArgs a) {
-  ptx::grid_launch_dependents();
   ptx::grid_dependency_wait();  // nothing in global memory is touched before this
   extern __shared__ __align__(16) unsigned char dyn_smem[];
   __shared__ TeamShared ts;
@@ -783,6 +782,9 @@ __global__ void __launch_bounds__(kRowThreads, 4) select_rows_kernel(const RowAr
     select_row(a, tm, &ts, dyn_smem, b, h, i, false);
   }
   SEL_MARK(true, tm.tid, 7);
+  // Not at the start: the attention kernel's CTAs (one to an SM, which they fill) then come while rows are under way, and the faster the
+  // rows the more that cost.  us a pass at the start / here / behind the ticket: one KV head of 128K 89.6 / 83.6 / 83.9.
+  ptx::grid_launch_dependents();
   if (!a.fuse) return;
   const int kv_row = b * (a.H / a.G) + h / a.G;
   // ---- fused Block-Union: the last row CTA of this KV-head row builds the table.  Nobody waits: a CTA
