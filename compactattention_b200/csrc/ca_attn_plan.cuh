@@ -1,7 +1,8 @@
 // How the attention kernels share their work out: the lengths of the 256-row kernel's units and whether they are cut
 // across CTAs, and (last) the decode kernel's clusters.  Lengths are in KV steps of 128
-// tokens (about 2.2 us).  Plain arithmetic on both sides: the kernel decides from the rows' counts; the host, where it
-// knows them, by the same rule.
+// tokens.  Plain arithmetic on both sides: the kernel decides from the rows' counts; the host, where it knows them, by the
+// same rule.  The prices and the times beside them were measured with an earlier form of the kernel and of the merge, a KV step
+// of about 2.2 us; a step now takes about 2560 cycles (1.3 to 1.7 us) and the merge less too, and the prices were not taken anew.
 #pragma once
 
 #include <math.h>
@@ -18,7 +19,7 @@ namespace attn {
 constexpr int kSub = 64;  // tokens per TMA box / sub-block
 
 constexpr int kMinSpanSteps = 4;           // shortest span worth a CTA of its own when units are cut
-// What cutting units costs a CTA (partials, the merge), in KV steps of about 2.2 us, with up to ~8 pieces a unit; every
+// What cutting units costs a CTA (partials, the merge), in KV steps, with up to ~8 pieces a unit; every
 // further piece costs the merge about kPieceSteps more (4 units of 105 steps in 13 / 21 / 27 / 36 pieces each: 46 / 49 /
 // 53 / 60 us).  Whole against cut, us: 64 units of 1-16 steps 44 / 31, 256 of them 73 / 61, 32 of ~20 37 / 32, 16 units of
 // one KV head at 128K 442 / 77; units of at most 8 steps, one per SM, stay whole (27).

@@ -50,11 +50,10 @@ constexpr int kTmemCols = 512;
 constexpr int kMaxRows = 1024;  // (batch x kv heads) rows per launch
 constexpr int kMaxSegs = 64;    // segments planned per batch
 constexpr float kRescaleThreshold = 8.0f;  // log2 units; lazy accumulator rescale
-// Measured on B200 (sustained 300-launch loop, 128K context, 20 % density): handing P to the MMA warp
-// in two halves 434 us, in one piece 450 us; packed fp32 pairs for the scale and the row sum 421 us.
-// A polynomial exp2 on the FMA pipe for part of the exponentials (2 / 4 / 6 of every 16 pairs) took
-// 486 / 499 / 518 us against 485 us without: with the softmax warps of both tiles on every scheduler
-// the added instructions cost more than the MUFU operations they replace, so there is none.
+// Measured with the earlier form (one issuing lane in a branch, P over S; 300 launches, 128K context, 20 % density): handing P
+// to the MMA warp in two halves 434 us, in one piece 450 us; packed fp32 pairs for the scale and the row sum 421 us; a polynomial
+// exp2 on the FMA pipe for 2 / 4 / 6 of every 16 pairs 486 / 499 / 518 us, without it 485.  The issuing lane was the pace then, so the
+// last says nothing of this form, where MUFU is about as busy as the tensor pipe; it has not been measured here.
 #ifndef CA_ATTN_PROFILE
 #define CA_ATTN_PROFILE 0
 #endif
@@ -244,9 +243,9 @@ __device__ void plan_segments(const KernelArgs& a, Shared* sh, long long span_be
   sh->more = (acc < span_end && row < R) ? 1 : 0;
 }
 
-// P = exp2(S*sc + neg_m) for one 128-column row held in registers: packs to 16 bit, stores the four
-// 32-column chunks over S in TMEM, signals the MMA warp after each of the kPParts pieces.  The scale
-// and the row sum use packed fp32 pairs.  Returns the row sum of P.
+// P = exp2(S*sc + neg_m) for one 128-column row held in registers: packs to 16 bit, calls p_free, which blocks until P's own TMEM
+// columns may be overwritten (before the first store), stores the four 32-column chunks there, signals the MMA warp after each of
+// the kPParts pieces.  The scale and the row sum use packed fp32 pairs.  Returns the row sum of P.
 template <typename T, typename Free>
 __device__ __forceinline__ float exp_pack_store(const uint32_t (&sv)[128], float sc, float neg_m, uint32_t tP,
                                                 uint32_t p_part_bar, Free p_free) {
@@ -423,8 +422,8 @@ __global__ void __launch_bounds__(kThreads, 1)
 #endif
   // role state that lives across segments
   int ring_n = 0;        // ring entries issued (loader) / consumed (MMA)
-  uint32_t it = 0;       // KV steps processed so far: parity of s_full / p_part
-  uint32_t seg_seq = 0;  // segments processed so far: parity of q_full / q_free / o_done / o_free
+  uint32_t it = 0;       // KV steps processed so far: parity of s_full / p_part / pv_done, and, two to a step, of s_free
+  uint32_t seg_seq = 0;  // segments processed so far: parity of q_full / q_free / o_free
   uint32_t q_issued = 0; // Q loads issued (loader)
   bool ok = true;
 
@@ -536,16 +535,15 @@ __global__ void __launch_bounds__(kThreads, 1)
         // =============================== MMA issuer ===============================
         {
           // The warp stays converged and one elected lane issues.  From a branch that one lane takes, the MMAs and commits of a
-          // KV step took that lane 2850 cycles, 83 % of the step (1024 x 106K keys, 32/8 heads); from the converged warp 1790.
+          // KV step took that lane 2850 cycles, 78 % of the step (1024 x 106K keys, 32/8 heads); from the converged warp 1790.
           // us before / after, single launches and at the power cap: that shape 472 / 458, 535 / 528; 8192 x 8192, f16 538 / 512,
           // 580 / 562; 8192 x 40K, 28/4 heads 3379 / 3305, 3914 / 3823.
           const uint32_t lead = ptx::elect_one();
           const uint32_t tS = tmem;
           const uint32_t tP[2] = {tmem + 128u, tmem + 192u};
           const uint32_t tO[2] = {tmem + 256u, tmem + 384u};
-          // Descriptors: one base per operand buffer, then a constant added per MMA (the start address
-          // sits in the low 14 bits in 16-byte units and never carries), so the single issuing thread
-          // spends two adds per instruction instead of rebuilding descriptors.
+          // Descriptors: one base per operand buffer; within a product's block of instructions a constant is added per MMA (the
+          // start address sits in the low 14 bits in 16-byte units and never carries).
           const uint64_t q_desc[2] = {ptx::make_smem_desc_sw128(q_smem, 0, 1024),
                                       ptx::make_smem_desc_sw128(q_smem + kTileBytes, 0, 1024)};
           const uint64_t k_desc0 = ptx::make_smem_desc_sw128(ring_smem, 0, 1024);
@@ -725,7 +723,9 @@ __global__ void __launch_bounds__(kThreads, 1)
                 // Two rounds of 16 columns are in flight.  us where the maximum rises by 9 in every step, and normal scores, for rounds
                 // one at a time with a wait for each store / this: 16 units of 256 steps 561 / 543, 418 / 420; 2048 x 4096, 32/8 heads
                 // 126.2 / 122.5, 103.2 / 103.1.  32 columns at a time: 538, 430; after P, in the registers of S, told to the MMA warp
-                // only then: 490, 421 and 116, 106: what rescales in every step is rarer than what hardly ever does.
+                // only then: 490, 421 and 116, 106: what rescales in every step is rarer than what hardly ever does.  The pair makes the
+                // kernel spill 92 bytes; one round at a time, still with one wait at the end, spills none and is no faster: 564 / 549 where
+                // the maximum rises, 425.7 / 426.1 for normal scores.
   #pragma unroll 2
                 for (int c = 0; c < 8; ++c) {
                   uint32_t w[16];

@@ -264,7 +264,7 @@ __device__ __forceinline__ void mma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_
       "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// D[tmem] (+)= A[tmem] * B[smem].
+// D[tmem] (+)= A[tmem] * B[smem] (the probes under microbench/ use it; the kernels issue whole products, below).
 __device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
                                        uint32_t accumulate) {
   asm volatile(
@@ -289,9 +289,9 @@ __device__ __forceinline__ void tc_commit_if(uint32_t lead, uint32_t bar) {
 // K-major in two 128-byte-swizzled halves of 16 KB.  One block, so that nothing comes between the instructions.
 __device__ __forceinline__ void mma_ss_128x128x128(uint32_t lead, uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc) {
   asm volatile(
-      "{\n\t.reg .pred p, t, e;\n\t.reg .b64 da, db;\n\t.reg .b32 a;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\tsetp.eq.b32 t, 0, 0;\n\t"
-      "setp.ne.b32 e, %5, 0;\n\t"
+      "{\n\t.reg .pred p, t, e;\n\t.reg .b64 da, db;\n\t"
+      "setp.ne.b32 p, 0, 0;\n\tsetp.eq.b32 t, 0, 0;\n\t"
+      "setp.ne.b32 e, %4, 0;\n\t"
       "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
       "add.s64 da, %1, 2;\n\tadd.s64 db, %2, 2;\n\t@e tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, t;\n\t"
       "add.s64 da, %1, 4;\n\tadd.s64 db, %2, 4;\n\t@e tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, t;\n\t"
@@ -301,7 +301,7 @@ __device__ __forceinline__ void mma_ss_128x128x128(uint32_t lead, uint32_t d_tme
       "add.s64 da, %1, 1028;\n\tadd.s64 db, %2, 1028;\n\t@e tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, t;\n\t"
       "add.s64 da, %1, 1030;\n\tadd.s64 db, %2, 1030;\n\t@e tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, t;\n\t"
       "}" ::"r"(d_tmem),
-      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(0), "r"(lead)
+      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(lead)
       : "memory");
 }
 // The same for D[tmem] (+)= A[tmem] * B[smem], 128 x 128 x 64, B MN-major: `accumulate` is the first instruction's.
@@ -358,17 +358,6 @@ __device__ __forceinline__ void tmem_ld32_row(uint32_t taddr, uint32_t (&r)[128]
         "=r"(r[OFF + 24]), "=r"(r[OFF + 25]), "=r"(r[OFF + 26]), "=r"(r[OFF + 27]), "=r"(r[OFF + 28]), "=r"(r[OFF + 29]),
         "=r"(r[OFF + 30]), "=r"(r[OFF + 31])
       : "r"(taddr)
-      : "memory");
-}
-__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
-      "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};" ::"r"(taddr),
-      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
-      "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]),
-      "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]),
-      "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
       : "memory");
 }
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
