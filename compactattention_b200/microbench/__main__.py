@@ -6,13 +6,13 @@
     python -m compactattention_b200.microbench chain       # S -> softmax -> P -> P.V dependency chain of one tile
 
 * ``mma_rate.cu``: one thread of one CTA per SM issues 8192 MMAs back to back (operands are zeros):
-  128x128x16 with both operands in shared memory, with A in tensor memory, alternating groups as the
-  attention loop issues them, 128x256x16, and 128x64x16 / 128x32x16 (``MMA_N``).
+  128x128x16 with both operands in shared memory, with A in tensor memory, alternating groups as an
+  earlier form of the attention loop issued them, 128x256x16, and 128x64x16 / 128x32x16 (``MMA_N``).
 * ``handoff.cu``: an issuer thread issues n MMAs and commits to an mbarrier, 128 worker threads wait
   on it and arrive on a second mbarrier the issuer waits on: the fixed latency of one S -> P hand-off.
-* ``chain.cu``: the attention kernel's per-tile loop in isolation (S = Q.K^T, softmax of a 128-column
-  row per thread, P back to tensor memory in two pieces, O += P.V, next S): cycles per KV step for the
-  kernel's softmax and for variants (chunked load, two warpgroups per tile, polynomial exp2).
+* ``chain.cu``: the per-tile loop of an earlier form of the attention kernel, whose P lay over its S, in isolation (S = Q.K^T, softmax of a 128-column
+  row per thread, P back to tensor memory in two pieces, O += P.V, next S): cycles per KV step for its
+  softmax and for variants (chunked load, two warpgroups per tile, polynomial exp2).
 """
 from __future__ import annotations
 

@@ -1,7 +1,7 @@
-// Harness for the per-tile dependency chain of the attention kernel: S = Q.K^T (8 MMAs) -> softmax -> P -> O += P.V (8 MMAs)
+// Harness for the per-tile dependency chain of an earlier form of the attention kernel, whose P lay over its S: S = Q.K^T (8 MMAs) -> softmax -> P -> O += P.V (8 MMAs)
 // -> next S ...  One tile, so the period is exactly 1024 cycles of MMA work + hand-off latencies + softmax time.
 // Timing only (operands are zeros).  argv: variant iters
-//   0: softmax as in the kernel (one thread per row, 128 columns, P in two pieces)
+//   0: softmax as in that kernel (one thread per row, 128 columns, P in two pieces)
 //   1: S loaded in chunks, row max of a chunk computed while the next chunks are in flight
 //   2: two warpgroups per tile, each thread owns 64 columns of a row (row max exchanged through shared memory)
 //   3: variant 2 + polynomial exp2 for POLY of every 16 pairs (env POLY)
